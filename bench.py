@@ -185,7 +185,8 @@ def wl_config1(small: bool = False):
     mesh = Mesh(trees, uniform_leaves(trees, level))
     S0 = sod_state(mesh.centroids())
     cfg = workload_config("config1", int(mesh.n), [level])
-    alg = {"m0_recon": 40 + 28 + 240, "m0_flux_rk<2>": 240 + 40 + 40 + 28 + 40}
+    alg = {"m0_recon": 40 + 28 + 240, "m0_face_flux<2>": 240 + 28 + 120,
+           "m0_update<2>": 120 + 40 + 40 + 28 + 40}
     return mesh, S0, cfg["dt"], cfg, dict(model=0), alg, True
 
 

@@ -236,6 +236,9 @@ void ffv_fill_geom(const ffv_mesh *m, ffv_geom *g) {
     g->dcc[l][2] = 0.5 * h + 0.25 * h;
     g->dcf[l][3] = 0.0;
     g->dcc[l][3] = 0.0;
+    for (int q = 0; q < 4; q++) g->rdcc[l][q] = 1.0 / g->dcc[l][q];
+    int ex;
+    if (frexp(h, &ex) == 0.5 && g->dcc[l][0] == h && g->dcf[l][0] == 0.5 * h) g->pow2 |= 1u << l;
     for (int q = 0; q < 4; q++) {
       g->dcf_f[l][q] = (float)g->dcf[l][q];
       g->idcc_f[l][q] = (float)(1.0 / g->dcc[l][q]);

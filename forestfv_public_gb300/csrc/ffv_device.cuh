@@ -31,6 +31,10 @@ struct ffv_geom {
   double h[FFV_MAX_LEVEL + 2];
   double dcf[FFV_MAX_LEVEL + 2][4];    // by face class: same, coarser, finer, boundary
   double dcc[FFV_MAX_LEVEL + 2][4];
+  // 1 / dcc rounded to nearest (infinite at a boundary), and the levels whose cell edge and
+  // volume are powers of two (bit l): scaling by those is exact
+  double rdcc[FFV_MAX_LEVEL + 2][4];
+  uint32_t pow2;
   // FP32 forms for the FP32-flux reconstruction: dcf and 1 / dcc (inf at a boundary)
   float dcf_f[FFV_MAX_LEVEL + 2][4];
   float idcc_f[FFV_MAX_LEVEL + 2][4];
