@@ -232,7 +232,8 @@ def m5_alg_bytes(neq: int, nmat: int) -> dict:
     FP64, face records of neq + N + 1 FP32 values."""
     d = 8 * neq
     rec = 4 * (neq + nmat + 1)
-    return {"m5_recon_face": d + 28 + 6 * d,
+    return {"m5_recon_slopes": d + 28 + 6 * d,
+            "m5_relax_faces": 6 * d + 6 * 8 * (2 * nmat + 8),
             "m5_face_flux": 6 * d + d + 28 + 6 * d + 6 * 3 * 8 + 6 * 8,
             "m5_cell_update": d + 6 * d + 6 * 3 * 8 + d + 28 + d + d + 1,
             "m5_relax_cell": d + d + 1,

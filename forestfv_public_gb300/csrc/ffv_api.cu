@@ -377,6 +377,15 @@ int ffv_create(ffv_ctx **out, const ffv_params *p, int device) {
       k.ig1[i] = gm1 != 0.0 ? 1.0 / gm1 : 0.0;
       k.gpg[i] = k.gpi[i] * k.ig1[i];
       k.igam[i] = p->gamma[i] != 0.0 ? 1.0 / p->gamma[i] : 0.0;
+      k.gm1[i] = gm1;
+      // volatile: the product and the sum round separately (no contraction by the host compiler)
+      const volatile double deepest = -(1.0 - 1.0e-8) * p->pinf[i];
+      k.pfloor[i] = deepest + 1.0e-8;
+      k.preset[i] = deepest + 1.0;
+      if (i < 3) {
+        double cf = 1.0;
+        for (int j = 1; j <= 10; j++) k.binom[i][j - 1] = cf *= (k.igam[i] - (j - 1)) / j;
+      }
       k.pinf_f[i] = (float)p->pinf[i];
       k.igam_f[i] = (float)k.igam[i];
       k.mu_f[i] = (float)p->mu[i];
@@ -393,6 +402,8 @@ int ffv_create(ffv_ctx **out, const ffv_params *p, int device) {
       k.pinf_d[i] = df_from_double(p->pinf[i]);
       k.floor_d[i] = df_from_double(-(1.0 - 1.0e-8) * p->pinf[i] + 1.0e-8);
     }
+    k.lo = p->amin / 100.0;
+    k.hi = 1.0 - (p->amin / 100.0);
     k.alo_f = (float)(p->amin / 100.0);
     k.ahi_f = (float)(1.0 - (p->amin / 100.0));
     k.avf_lim_f = (float)k.avf_lim;

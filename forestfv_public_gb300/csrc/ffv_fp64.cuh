@@ -72,9 +72,11 @@ FFV_F64_FN int64_t order_key(double x) {
   const int64_t s = (int64_t)bits(x);
   return s ^ ((s >> 63) & 0x7fffffffffffffffll);
 }
-// x < y, x <= y for a y that is neither NaN nor zero (false where x is NaN)
+// x < y, x <= y, x > y, x >= y for a y that is neither NaN nor zero (false where x is NaN)
 FFV_F64_FN bool lt(double x, double y) { return order_key(x) < order_key(y) && !is_nan(x); }
 FFV_F64_FN bool le(double x, double y) { return order_key(x) <= order_key(y) && !is_nan(x); }
+FFV_F64_FN bool gt(double x, double y) { return order_key(x) > order_key(y) && !is_nan(x); }
+FFV_F64_FN bool ge(double x, double y) { return order_key(x) >= order_key(y) && !is_nan(x); }
 
 // A divisor and its reciprocal, rounded to nearest.
 struct Rcp {

@@ -19,6 +19,11 @@ struct M5Consts {
   // gamma p_inf / (gamma - 1), 1 / gamma
   double gpi[FFV_MAX_MATERIALS], ig1[FFV_MAX_MATERIALS], gpg[FFV_MAX_MATERIALS],
       igam[FFV_MAX_MATERIALS];
+  // FP64 form: gamma - 1, the relaxation's pressure floor -(1 - 1e-8) p_inf + 1e-8 and reset value,
+  // AMIN / 100 and 1 - AMIN / 100, and the binomial coefficients of (1 + t)^(1 / gamma), t^1..t^10
+  double gm1[FFV_MAX_MATERIALS], pfloor[FFV_MAX_MATERIALS], preset[FFV_MAX_MATERIALS];
+  double lo, hi;
+  double binom[3][10];
   // the same in FP32: p_inf, 1 / gamma, mu, gamma, the relaxation's pressure floor and reset
   // value, AMIN / 100 and 1 - AMIN / 100
   float pinf_f[FFV_MAX_MATERIALS], igam_f[FFV_MAX_MATERIALS], mu_f[FFV_MAX_MATERIALS],

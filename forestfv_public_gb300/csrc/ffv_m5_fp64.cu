@@ -6,9 +6,17 @@
 // rounding differences from the reference come from pow(): CUDA's and glibc's pow differ
 // in the last bit for some arguments.
 //
+// The kernels are bound by the FP64 pipe: comparisons, clamps, halvings and sign tests work on
+// the bit patterns, quotients by one divisor share its reciprocal (ffv_fp64.cuh), and terms that
+// are exactly zero -- the deformation of a fluid cell (A = 0), the components of a face's unit
+// normal -- are left out.  None of this changes a bit of the result.  The consistent flux form,
+// which has no reference to equal bit for bit, also takes its own Newton iteration
+// (relaxationvec).
+//
 // One stage:
-//   m5_recon_face   (cell, face)  MUSCL face state + face-state pressure relaxation
-//                                  (m5_faceinterp_V1 / m5_reconctruct_V1 / m5_relaxationvec)
+//   m5_recon_slopes (cell, axis)  MUSCL states of the two faces (m5_faceinterp_V1 /
+//                                  m5_reconctruct_V1)
+//   m5_relax_faces  (cell, face)  their pressure relaxation, in place (m5_relaxationvec)
 //   m5_face_flux    (cell, face)  HLLC or ghost-fluid HLLC per face or subface; a 1:1 face
 //                                  is evaluated once, by the cell first in leaf order, and
 //                                  the other takes its negative (the reference's flux
@@ -22,6 +30,7 @@
 #include <math.h>
 
 #include "ffv_device.cuh"
+#include "ffv_fp64.cuh"
 #include "ffv_m5.cuh"
 #include "ffv_m5_frame.cuh"
 #include "ffv_plastic.cuh"
@@ -29,69 +38,104 @@
 namespace {
 
 // ------------------------------------------------------------------ EOS (state_equation.c)
-__device__ __forceinline__ void gmat_of(const double A[9], double G[9], double &Gmag) {
-  G[0] = A[0] * A[0] + A[1] * A[1] + A[2] * A[2];
-  G[1] = A[0] * A[3] + A[1] * A[4] + A[2] * A[5];
-  G[2] = A[0] * A[6] + A[1] * A[7] + A[2] * A[8];
-  G[3] = A[3] * A[0] + A[4] * A[1] + A[5] * A[2];
-  G[4] = A[3] * A[3] + A[4] * A[4] + A[5] * A[5];
-  G[5] = A[3] * A[6] + A[4] * A[7] + A[5] * A[8];
-  G[6] = A[6] * A[0] + A[7] * A[1] + A[8] * A[2];
-  G[7] = A[6] * A[3] + A[7] * A[4] + A[8] * A[5];
-  G[8] = A[6] * A[6] + A[7] * A[7] + A[8] * A[8];
-  Gmag = G[0] * (G[4] * G[8] - G[5] * G[7]) - G[1] * (G[3] * G[8] - G[5] * G[6]) +
-         G[2] * (G[3] * G[7] - G[4] * G[6]);
+// every entry of a deformation tensor is a zero: a fluid cell
+__device__ __forceinline__ bool no_deformation(const double A[9]) {
+  uint64_t any = 0;
+#pragma unroll
+  for (int q = 0; q < 9; q++) any |= f64::abs_bits(A[q]);
+  return any == 0;
 }
 
-// state_equation.c:269-317 and :217-267 (need_mu: the G_det form's extra mu != 0 test)
-__device__ double elastic_energy(const double G[9], double Gmag, double mu, bool need_mu) {
-  if (!(fabs(Gmag) != 0.0) || (need_mu && !(mu != 0.0))) return 0.0;
-  double g13 = pow(fabs(Gmag), 1.0 / 3.0);
-  if (isnan(g13)) g13 = 0.0;
-  const double M1[9] = {G[0] - g13, G[1], G[2], G[3], G[4] - g13, G[5], G[6], G[7], G[8] - g13};
-  double M2[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) M2[i * 3 + j] += M1[i * 3 + k] * M1[k * 3 + j];
-  const double tr1 = M2[0] + M2[4] + M2[8];
-  return mu / (4.0 * pow(fabs(Gmag), 1.0 / 6.0)) * tr1;
+// G = A A^T (symmetric to the bit: the reference's two expressions of an off-diagonal entry have
+// the same products in the same order) and the powers of its determinant that the elastic energy
+// and stress of every solid take; solid: the determinant is not zero
+struct Elastic {
+  double G[6];  // G00, G11, G22, G01, G02, G12
+  double p13, p16;
+  bool solid;
+};
+
+__device__ __forceinline__ void elastic_of(const M5Consts &k, const double A[9], Elastic &e) {
+  e.solid = false;
+  if (k.nsolids == 0 || no_deformation(A)) return;
+  const double G0 = A[0] * A[0] + A[1] * A[1] + A[2] * A[2];
+  const double G1 = A[0] * A[3] + A[1] * A[4] + A[2] * A[5];
+  const double G2 = A[0] * A[6] + A[1] * A[7] + A[2] * A[8];
+  const double G4 = A[3] * A[3] + A[4] * A[4] + A[5] * A[5];
+  const double G5 = A[3] * A[6] + A[4] * A[7] + A[5] * A[8];
+  const double G8 = A[6] * A[6] + A[7] * A[7] + A[8] * A[8];
+  const double Gmag = G0 * (G4 * G8 - G5 * G5) - G1 * (G1 * G8 - G5 * G2) + G2 * (G1 * G5 - G4 * G2);
+  e.G[0] = G0;
+  e.G[1] = G4;
+  e.G[2] = G8;
+  e.G[3] = G1;
+  e.G[4] = G2;
+  e.G[5] = G5;
+  if (f64::abs_bits(Gmag) == 0) return;
+  e.solid = true;
+  e.p13 = pow(fabs(Gmag), 1.0 / 3.0);
+  e.p16 = pow(fabs(Gmag), 1.0 / 6.0);
+}
+
+// state_equation.c:269-317 and :217-267
+__device__ __forceinline__ double elastic_energy(const Elastic &e, double mu) {
+  if (!e.solid || mu == 0.0) return 0.0;
+  const double g13 = f64::is_nan(e.p13) ? 0.0 : e.p13;
+  const double d0 = e.G[0] - g13, d1 = e.G[1] - g13, d2 = e.G[2] - g13;
+  const double a = e.G[3], b = e.G[4], c = e.G[5];
+  const double tr1 = (d0 * d0 + a * a + b * b) + (a * a + d1 * d1 + c * c) + (b * b + c * c + d2 * d2);
+  return mu / (4.0 * e.p16) * tr1;
 }
 
 // state_equation.c:143-204, accumulated into st (and stored in ast when given)
-__device__ void eos_stress_acc(double st[3][3], double avf, double pr, const double G[9],
-                               double Gmag, double mu, double (*ast)[3]) {
-  double s[3][3];
-  if ((fabs(Gmag) != 0.0) && (mu != 0.0)) {
-    double G2[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+__device__ __forceinline__ void eos_stress_acc(double st[3][3], double avf, double pr,
+                                               const Elastic &e, double mu, double (*ast)[3]) {
+  const double press = -avf * pr;
+  if (e.solid && mu != 0.0) {
+    const double G0 = e.G[0], G4 = e.G[1], G8 = e.G[2], G1 = e.G[3], G2 = e.G[4], G5 = e.G[5];
+    const double q0 = G0 * G0 + G1 * G1 + G2 * G2, q4 = G1 * G1 + G4 * G4 + G5 * G5,
+                 q8 = G2 * G2 + G5 * G5 + G8 * G8, q1 = G0 * G1 + G1 * G4 + G2 * G5,
+                 q2 = G0 * G2 + G1 * G5 + G2 * G8, q5 = G1 * G2 + G4 * G5 + G5 * G8;
+    const f64::Rcp three{3.0, 1.0 / 3.0};
+    const double J1 = f64::div(G0 + G4 + G8, three), J2 = f64::div(q0 + q4 + q8, three);
+    const double f = mu / e.p16;
+    const double s0 = press - f * (q0 - J2 - e.p13 * (G0 - J1)),
+                 s4 = press - f * (q4 - J2 - e.p13 * (G4 - J1)),
+                 s8 = press - f * (q8 - J2 - e.p13 * (G8 - J1));
+    const double s1 = -f * (q1 - e.p13 * G1), s2 = -f * (q2 - e.p13 * G2), s5 = -f * (q5 - e.p13 * G5);
+    const double s[3][3] = {{s0, s1, s2}, {s1, s4, s5}, {s2, s5, s8}};
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
+    for (int i = 0; i < 3; i++)
 #pragma unroll
-      for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) G2[i * 3 + j] += G[i * 3 + k] * G[k * 3 + j];
-    const double J1 = G[0] + G[4] + G[8], J2 = G2[0] + G2[4] + G2[8];
-    const double p13 = pow(fabs(Gmag), 1.0 / 3.0);
-    const double f = mu / pow(fabs(Gmag), 1.0 / 6.0);
-#pragma unroll
-    for (int q = 0; q < 9; q++) {
-      const double ss = (q == 0 || q == 4 || q == 8) ? G2[q] - J2 / 3.0 - p13 * (G[q] - J1 / 3.0)
-                                                     : G2[q] - p13 * (G[q]);
-      s[q / 3][q % 3] = (q == 0 || q == 4 || q == 8) ? -avf * pr - f * (ss) : -f * (ss);
-    }
+      for (int j = 0; j < 3; j++) {
+        if (j >= i) st[i][j] += s[i][j];
+        else st[i][j] = st[j][i];
+        if (ast) ast[i][j] = s[i][j];
+      }
   } else {
 #pragma unroll
-    for (int q = 0; q < 9; q++) s[q / 3][q % 3] = (q == 0 || q == 4 || q == 8) ? -avf * pr : 0.0;
-  }
-#pragma unroll
-  for (int i = 0; i < 3; i++)
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-      st[i][j] += s[i][j];
-      if (ast) ast[i][j] = s[i][j];
+    for (int i = 0; i < 3; i++) {
+      st[i][i] += press;
+      if (ast)
+        for (int j = 0; j < 3; j++) ast[i][j] = i == j ? press : 0.0;
     }
+  }
+}
+
+// a volume fraction between amin / 100 and 1 - amin / 100
+__device__ __forceinline__ double clamp_vf(const M5Consts &k, double a) {
+  return f64::le(a, k.lo) ? k.lo : (f64::ge(a, k.hi) ? k.hi : a);
+}
+
+// phi[0] (m5_facevalues.c:83-99): the solid fraction(s) against AVF_LIM; ac the cell's fractions
+template <int N>
+__device__ __forceinline__ double phi0_of(const M5Consts &k, double a0, double a1) {
+  const double c0 = clamp_vf(k, a0);
+  if (N > 2 && k.nsolids == 2 && k.mu[0] != 0.0) {
+    const double c1 = clamp_vf(k, a1);
+    return (f64::gt(c0, c1) ? c0 : c1) - k.avf_lim;
+  }
+  return c0 - k.avf_lim;
 }
 
 template <int N>
@@ -100,75 +144,63 @@ struct Sol {
   double ra[N], avf[N], are[N], p[N];
   double A[9], st[3][3];
   double vec[K5<N>::NC];  // conservative part of the state vector (HLLC corrections)
+  bool flat;              // A = 0
 };
 
 // m5_facevalues.c:3-192 (from_face false: U is a cell state) and m5_facercnstr.c:3-191
-// (from_face true: U is a face state); Sc is the cell-centre state whose volume fractions
-// give phi.  ast (optional) receives each material's stress.
+// (from_face true: U is a face state); phi0 from the cell-centre state's volume fractions.
+// ast (optional) receives each material's stress.
 template <int N>
-__device__ void make_sol(const M5Consts &k, const double *U, const double *Sc, bool from_face,
+__device__ void make_sol(const M5Consts &k, const double *U, double phi0, bool from_face,
                          Sol<N> &s, double (*ast)[3][3] = nullptr) {
   using C = K5<N>;
-  const double lo = k.amin / 100.0, hi = 1.0 - (k.amin / 100.0);
-  s.r = 0.0;
+  s.r = U[0];
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    s.r += U[i];
+    if (i) s.r += U[i];
     s.ra[i] = U[i];
     s.vec[i] = U[i];
   }
-  s.u = U[C::i1 + 0] / s.r;
-  s.v = U[C::i1 + 1] / s.r;
-  s.w = U[C::i1 + 2] / s.r;
+  const f64::Rcp r = f64::rcp(s.r);
+  s.u = f64::div(U[C::i1 + 0], r);
+  s.v = f64::div(U[C::i1 + 1], r);
+  s.w = f64::div(U[C::i1 + 2], r);
   s.vec[C::i1 + 0] = U[C::i1 + 0];
   s.vec[C::i1 + 1] = U[C::i1 + 1];
   s.vec[C::i1 + 2] = U[C::i1 + 2];
-  s.e = U[C::i2] / s.r;
+  s.e = f64::div(U[C::i2], r);
   s.vec[C::i2] = U[C::i2];
-  double at[N], ac[N], sum = 0.0;
+  double at[N], sum = 0.0;
 #pragma unroll
   for (int i = 0; i < N - 1; ++i) {
-    at[i] = U[C::i3 + i];
-    ac[i] = Sc[C::i3 + i];
-    if (at[i] <= lo) at[i] = lo;
-    else if (at[i] >= hi) at[i] = hi;
-    if (from_face) {
-      if (ac[i] >= hi) ac[i] = hi;
-      else if (ac[i] <= lo) ac[i] = lo;
-    } else {
-      if (ac[i] <= lo) ac[i] = lo;
-      else if (ac[i] >= hi) ac[i] = hi;
-    }
-    sum += at[i];
+    at[i] = clamp_vf(k, U[C::i3 + i]);
+    sum = i ? sum + at[i] : at[i];
   }
-  if (sum > hi) {
-    const double dif = sum - hi;
+  double last = 1.0 - sum;  // the last fraction; avf[N - 1] sums the scaled ones once more
+  at[N - 1] = last;
+  if (f64::gt(sum, k.hi)) {
+    const double dif = sum - k.hi;
+    const f64::Rcp rs = f64::rcp(sum);
+    sum = 0.0;
 #pragma unroll
     for (int j = 0; j < N - 1; ++j) {
-      const double per = at[j] / sum;
-      at[j] = at[j] - per * dif;
+      at[j] = at[j] - f64::div(at[j], rs) * dif;
+      sum = j ? sum + at[j] : at[j];
     }
-    sum = hi;
+    at[N - 1] = 1.0 - k.hi;
+    last = 1.0 - sum;
   }
-  at[N - 1] = 1.0 - sum;
-  sum = 0.0;
 #pragma unroll
-  for (int i = 0; i < N - 1; ++i) {
-    s.avf[i] = at[i];
-    sum += at[i];
-  }
-  s.avf[N - 1] = 1.0 - sum;
-  // phi[0] (m5_facevalues.c:83-99): the solid fraction(s) against AVF_LIM
-  if (k.nsolids == 2 && k.mu[0] != 0.0)
-    s.phi0 = ((ac[0] > ac[N > 2 ? 1 : 0]) ? ac[0] : ac[N > 2 ? 1 : 0]) - k.avf_lim;
-  else
-    s.phi0 = ac[0] - k.avf_lim;
+  for (int i = 0; i < N - 1; ++i) s.avf[i] = at[i];
+  s.avf[N - 1] = last;
+  s.phi0 = phi0;
 #pragma unroll
   for (int i = 0; i < N; ++i) s.are[i] = U[C::i4 + i];
 #pragma unroll
   for (int q = 0; q < 9; q++) s.A[q] = U[C::i5 + q];
-  double G[9], Gmag;
-  gmat_of(s.A, G, Gmag);
+  s.flat = no_deformation(s.A);
+  Elastic el;
+  elastic_of(k, s.A, el);
 #pragma unroll
   for (int i = 0; i < 3; i++)
 #pragma unroll
@@ -176,14 +208,20 @@ __device__ void make_sol(const M5Consts &k, const double *U, const double *Sc, b
   double c2 = 0.0;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    const double ael = (k.mu[i] != 0.0) ? elastic_energy(G, Gmag, k.mu[i], false) : 0.0;
+    const double ael = elastic_energy(el, k.mu[i]);
     const double a = from_face ? s.avf[i] : at[i];
-    const double press = ((k.gamma[i] - 1.0) * (s.are[i] - ael) / a) - k.gamma[i] * k.pinf[i];
-    c2 += (a / s.r) * k.gamma[i] * (press + k.pinf[i]);
+    const double press = (k.gm1[i] * (s.are[i] - ael) / a) - k.gpi[i];
+    c2 += f64::div(a, r) * k.gamma[i] * (press + k.pinf[i]);
     s.p[i] = press;
-    eos_stress_acc(s.st, s.avf[i], press, G, Gmag, k.mu[i], ast ? ast[i] : nullptr);
+    eos_stress_acc(s.st, s.avf[i], press, el, k.mu[i], ast ? ast[i] : nullptr);
   }
   s.c2 = c2;
+}
+
+// the same with phi0 from the cell state Sc
+template <int N>
+__device__ __forceinline__ double phi0_state(const M5Consts &k, const double *Sc) {
+  return phi0_of<N>(k, Sc[K5<N>::i3], N > 2 ? Sc[K5<N>::i3 + 1] : 0.0);
 }
 
 // m5_bc.c (m5_bc_symmetry) / bc_reflective.c / bc_wall.c: ghost velocity
@@ -207,83 +245,84 @@ struct NC {
 
 // m5_star_region.c:3-158
 template <int F, int N>
-__device__ unsigned star_region(const M5Consts &k, const Sol<N> &s, const Sol<N> &L,
-                                const Sol<N> &R, bool leftside, double u_S, double SL, double SR,
+__device__ unsigned star_region(const M5Consts &k, const Sol<N> &s, double rL, double rR,
+                                bool both_solid, bool leftside, double u_S, double SL, double SR,
                                 double uL, double vL, double wL, double uR, double vR, double wR,
                                 const double sL[3], const double sR[3], double *Us, NC<N> &nc) {
   using C = K5<N>;
-  double SK, uK, vK, wK, s11K, s12K, s13K;
-  if (leftside) {
-    SK = SL; uK = uL; vK = vL; wK = wL; s11K = sL[0]; s12K = sL[1]; s13K = sL[2];
-  } else {
-    SK = SR; uK = uR; vK = vR; wK = wR; s11K = sR[0]; s12K = sR[1]; s13K = sR[2];
-  }
+  const double SK = leftside ? SL : SR, uK = leftside ? uL : uR, vK = leftside ? vL : vR,
+               wK = leftside ? wL : wR, s11K = leftside ? sL[0] : sR[0],
+               s12K = leftside ? sL[1] : sR[1], s13K = leftside ? sL[2] : sR[2];
+  // SK - u* and u* - SK are each other's negation to the bit, and so are quotients by them
+  const f64::Rcp dS = f64::rcp(SK - u_S);
+  const double dK = SK - uK;
   double ar_S[N], r_S = 0.0;
 #pragma unroll
   for (int v = 0; v < N; ++v) {
-    ar_S[v] = s.ra[v] * (SK - uK) / (SK - u_S);
-    r_S += ar_S[v];
+    ar_S[v] = f64::div(s.ra[v] * dK, dS);
+    r_S = v ? r_S + ar_S[v] : ar_S[v];
   }
-  const double s11_S = ((uR - SR) * R.r * (sL[0]) - (uL - SL) * L.r * (sR[0]) +
-                        (uL - SL) * L.r * (uR - SR) * R.r * (uR - uL)) /
-                       ((uR - SR) * R.r - (uL - SL) * L.r);
-  double s12_S, s13_S;
-  if ((L.phi0 > 0.0) && (R.phi0 > 0.0)) {
-    s12_S = ((uR - SR) * R.r * (sL[1]) - (uL - SL) * L.r * (sR[1]) +
-             (uL - SL) * L.r * (uR - SR) * R.r * (vR - vL)) /
-            ((uR - SR) * R.r - (uL - SL) * L.r);
-    s13_S = ((uR - SR) * R.r * (sL[2]) - (uL - SL) * L.r * (sR[2]) +
-             (uL - SL) * L.r * (uR - SR) * R.r * (wR - wL)) /
-            ((uR - SR) * R.r - (uL - SL) * L.r);
-  } else {
-    s12_S = 0.0;
-    s13_S = 0.0;
+  const double mR = (uR - SR) * rR, mL = (uL - SL) * rL, mLR = mL * (uR - SR) * rR;
+  const f64::Rcp den = f64::rcp(mR - mL);
+  const double s11_S = f64::div(mR * (sL[0]) - mL * (sR[0]) + mLR * (uR - uL), den);
+  double s12_S = 0.0, s13_S = 0.0;
+  if (both_solid) {
+    s12_S = f64::div(mR * (sL[1]) - mL * (sR[1]) + mLR * (vR - vL), den);
+    s13_S = f64::div(mR * (sL[2]) - mL * (sR[2]) + mLR * (wR - wL), den);
   }
-  const double v_S = vK + (s12_S - s12K) / ((uK - SK) * s.r);
-  const double w_S = wK + (s13_S - s13K) / ((uK - SK) * s.r);
+  const double j12 = s12_S - s12K, j13 = s13_S - s13K;
+  double v_S = vK + 0.0, w_S = wK + 0.0;
+  if (f64::abs_bits(j12) | f64::abs_bits(j13)) {
+    const f64::Rcp dv = f64::rcp((uK - SK) * s.r);
+    v_S = vK + f64::div(j12, dv);
+    w_S = wK + f64::div(j13, dv);
+  }
   const double vel[3] = {glob<F, 0>(u_S, v_S, w_S), glob<F, 1>(u_S, v_S, w_S),
                          glob<F, 2>(u_S, v_S, w_S)};
   const double re = s.r * s.e;
   // the reference's expression, or the Rankine-Hugoniot energy jump across the S_K wave
   // (FFV_FLUX_CONSISTENT, include/ffv.h)
-  const double Em_S =
-      k.flux_form == FFV_FLUX_CONSISTENT
-          ? (re * (uK - SK) - s11K * uK - s12K * vK - s13K * wK + s11_S * u_S + s12_S * v_S +
-             s13_S * w_S) / (r_S * (u_S - SK))
-          : (re * (uK - SK) + s11K * uK - s12K * vK - s13K * wK + s11_S * u_S + s12_S * v_S +
-             s13_S * w_S) / (r_S * (u_S + SK));
-  double Am[3][3], Al[3][3], AS[3][3], Ag[3][3];
+  const double sg11 = k.flux_form == FFV_FLUX_CONSISTENT ? f64::neg(s11K) : s11K;
+  const double Em_S = (re * (uK - SK) + sg11 * uK - s12K * vK - s13K * wK + s11_S * u_S + s12_S * v_S +
+                       s13_S * w_S) /
+                      (r_S * (k.flux_form == FFV_FLUX_CONSISTENT ? u_S - SK : u_S + SK));
+  Elastic el;
+  el.solid = false;
+  double Ag[3][3];
+  if (!s.flat) {
+    double Am[3][3], Al[3][3], AS[3][3];
 #pragma unroll
-  for (int i = 0; i < 3; i++)
+    for (int i = 0; i < 3; i++)
 #pragma unroll
-    for (int j = 0; j < 3; j++) Am[i][j] = s.A[3 * i + j];
-  tens_to_local<F>(Am, Al);
+      for (int j = 0; j < 3; j++) Am[i][j] = s.A[3 * i + j];
+    tens_to_local<F>(Am, Al);
+    const double ju = uK - SK, jv = vK - v_S, jw = wK - w_S;
 #pragma unroll
-  for (int j = 0; j < 3; j++) {
-    AS[0][j] = (Al[0][j] * (uK - SK) - Al[1][j] * (vK - v_S) + Al[2][j] * (wK - w_S)) / (u_S - SK);
-    AS[1][j] = Al[1][j];
-    AS[2][j] = Al[2][j];
+    for (int j = 0; j < 3; j++) {
+      AS[0][j] = f64::neg(f64::div(Al[0][j] * ju - Al[1][j] * jv + Al[2][j] * jw, dS));
+      AS[1][j] = Al[1][j];
+      AS[2][j] = Al[2][j];
+    }
+    tens_to_global<F>(AS, Ag);
+    elastic_of(k, &Ag[0][0], el);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+      for (int j = 0; j < 3; j++) Ag[i][j] = 0.0;
   }
-  tens_to_global<F>(AS, Ag);
-  double G[9];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-      G[3 * i + j] = Ag[i][0] * Ag[j][0] + Ag[i][1] * Ag[j][1] + Ag[i][2] * Ag[j][2];
-  const double Gmag = G[0] * (G[4] * G[8] - G[5] * G[7]) - G[1] * (G[3] * G[8] - G[5] * G[6]) +
-                      G[2] * (G[3] * G[7] - G[4] * G[6]);
 #pragma unroll
   for (int v = 0; v < N; ++v) {
     const double rm = (s.ra[v] / s.avf[v]);
-    const double rm_S = (s.ra[v] / s.avf[v]) * (uK - SK) / (u_S - SK);
+    const double rm_S = f64::neg(f64::div(rm * (uK - SK), dS));
     const double p_k = -s.p[v];
-    const double ga = k.gamma[v], pi = k.pinf[v];
-    const double p_S = (p_k + pi) * (((ga - 1.0) * rm + (ga + 1.0) * rm_S) /
-                                     ((ga - 1.0) * rm_S + (ga + 1.0) * rm)) - pi;
-    const double ael = elastic_energy(G, Gmag, k.mu[v], true);
-    const double eel = ael / (s.avf[v] * rm_S);
-    const double e_S = (p_S + ga * pi) / (rm_S * (ga + 1.0)) + eel;
+    const double ga = k.gamma[v], pi = k.pinf[v], gp1 = ga + 1.0, gm1 = k.gm1[v];
+    const double p_S = (p_k + pi) * ((gm1 * rm + gp1 * rm_S) / (gm1 * rm_S + gp1 * rm)) - pi;
+    const double ael = elastic_energy(el, k.mu[v]);
+    double e_S = (p_S + k.gpi[v]) / (rm_S * gp1);
+    // (a zero elastic energy adds a zero; rm_S or a fraction of zero makes it 0 / 0)
+    const double den_e = s.avf[v] * rm_S;
+    if (f64::abs_bits(ael) || !f64::moderate(den_e)) e_S += ael / den_e;
     nc.are[v] = ar_S[v] * e_S;
   }
 #pragma unroll
@@ -302,7 +341,7 @@ __device__ unsigned star_region(const M5Consts &k, const Sol<N> &s, const Sol<N>
   unsigned st = 0;
 #pragma unroll
   for (int iv = 0; iv < C::NC; ++iv)
-    if (isnan(Us[iv])) st |= FFV_ST_NAN;
+    if (f64::is_nan(Us[iv])) st |= FFV_ST_NAN;
   return st;
 }
 
@@ -344,12 +383,48 @@ __device__ void flux_n(const Sol<N> &s, int flag, bool gfm, bool cons, NC<N> &nc
   for (int v = 0; v < N - 1; ++v) Fn[C::i3 + v] = sgn<sg>(ua * nc.avf[v]);
 #pragma unroll
   for (int v = 0; v < N; ++v) Fn[C::i4 + v] = sgn<sg>(ua * nc.are[v]);
+  if (s.flat) {  // a fluid state: the star state's deformation is zero too
 #pragma unroll
-  for (int q = 0; q < 9; q++) Fn[C::i5 + q] = sgn<sg>(ua * nc.A[q]);
+    for (int q = 0; q < 9; q++) Fn[C::i5 + q] = 0.0;
+  } else {
+#pragma unroll
+    for (int q = 0; q < 9; q++) Fn[C::i5 + q] = sgn<sg>(ua * nc.A[q]);
+  }
+}
+
+// K = a ? A : B, field by field (selects: the states stay in registers)
+template <int N>
+__device__ __forceinline__ void select_sol(bool a, const Sol<N> &A, const Sol<N> &B, Sol<N> &K) {
+  K.r = a ? A.r : B.r;
+  K.u = a ? A.u : B.u;
+  K.v = a ? A.v : B.v;
+  K.w = a ? A.w : B.w;
+  K.e = a ? A.e : B.e;
+  K.ut = a ? A.ut : B.ut;
+  K.vt = a ? A.vt : B.vt;
+  K.wt = a ? A.wt : B.wt;
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    K.ra[i] = a ? A.ra[i] : B.ra[i];
+    K.avf[i] = a ? A.avf[i] : B.avf[i];
+    K.are[i] = a ? A.are[i] : B.are[i];
+    K.p[i] = a ? A.p[i] : B.p[i];
+  }
+  K.flat = a ? A.flat : B.flat;
+#pragma unroll
+  for (int q = 0; q < 9; q++) K.A[q] = a ? A.A[q] : B.A[q];
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) K.st[i][j] = a ? A.st[i][j] : B.st[i][j];
+#pragma unroll
+  for (int q = 0; q < K5<N>::NC; q++) K.vec[q] = a ? A.vec[q] : B.vec[q];
 }
 
 // m5_hllc.c:3-95 / m5_hllc_gfm.c:3-100 with the wave speeds, accumulated as
-// m5_residual.c:155-165: ff += A (F.n + corr); unc receives the face velocity.
+// m5_residual.c:155-165: ff += A (F.n + corr); unc receives the face velocity.  The solver's four
+// branches share one star-region and one physical-flux evaluation, on the state of the contact's
+// upwind side: lanes of a warp on different sides of the contact do not run one after the other.
 template <int F, int N>
 __device__ unsigned hllc_acc(const M5Consts &k, Sol<N> L, Sol<N> R, int bc, bool gfm,
                              double Area, double *ff, double unc[3]) {
@@ -384,38 +459,40 @@ __device__ unsigned hllc_acc(const M5Consts &k, Sol<N> L, Sol<N> R, int bc, bool
   const double sL[3] = {TL[0][0], TL[0][1], TL[0][2]}, sR[3] = {TR[0][0], TR[0][1], TR[0][2]};
   double u_S = ((L.r * (uL * uL) - (sL[0])) - (R.r * (uR * uR) - (sR[0])) - (SL * ruL) +
                 (SR * ruR)) / (ruL - ruR - (SL * L.r) + (SR * R.r));
-  unsigned st = (isnan(u_S) || isnan(SR) || isnan(SL)) ? FFV_ST_NAN_SPEED : 0u;
+  unsigned st = (f64::is_nan(u_S) || f64::is_nan(SR) || f64::is_nan(SL)) ? FFV_ST_NAN_SPEED : 0u;
   if (!gfm && bc == 4) u_S = 0.0;
   NC<N> nc;
-  double Fn[C::NEQ], Us[C::NC], corr[C::NC];
-#pragma unroll
-  for (int iv = 0; iv < C::NC; ++iv) corr[iv] = 0.0;
-  const bool left_star = gfm ? (SL < 0.0 && 0.0 <= u_S) : (SL <= 0.0 && 0.0 <= u_S);
-  const bool right_star = gfm ? (u_S < 0.0 && 0.0 < SR) : (u_S <= 0.0 && 0.0 <= SR);
-  if (0.0 <= SL) {
-    flux_n<F>(L, 0, gfm, k.flux_form == FFV_FLUX_CONSISTENT, nc, Fn);
-  } else if (left_star) {
-    st |= star_region<F>(k, L, L, R, true, u_S, SL, SR, uL, vL, wL, uR, vR, wR, sL, sR, Us, nc);
-    flux_n<F>(L, 1, gfm, k.flux_form == FFV_FLUX_CONSISTENT, nc, Fn);
-#pragma unroll
-    for (int iv = 0; iv < C::NC; ++iv) corr[iv] = SL * (Us[iv] - L.vec[iv]);
-  } else if (right_star) {
-    st |= star_region<F>(k, R, L, R, false, u_S, SL, SR, uL, vL, wL, uR, vR, wR, sL, sR, Us, nc);
-    flux_n<F>(R, 2, gfm, k.flux_form == FFV_FLUX_CONSISTENT, nc, Fn);
-#pragma unroll
-    for (int iv = 0; iv < C::NC; ++iv) corr[iv] = SR * (Us[iv] - R.vec[iv]);
-  } else if (SR <= 0.0) {
-    flux_n<F>(R, 3, gfm, k.flux_form == FFV_FLUX_CONSISTENT, nc, Fn);
-  } else {
+  double Fn[C::NEQ], Us[C::NC];
+  // 0: supersonic from the left, 1: left star state, 2: right star state, 3: supersonic from
+  // the right
+  const bool left_star = (gfm ? f64::lt0(SL) : f64::le0(SL)) && f64::ge0(u_S);
+  const bool right_star = gfm ? (f64::lt0(u_S) && f64::gt0(SR)) : (f64::le0(u_S) && f64::ge0(SR));
+  const int branch = f64::ge0(SL) ? 0 : left_star ? 1 : right_star ? 2 : f64::le0(SR) ? 3 : -1;
+  if (branch < 0) {
     st |= FFV_ST_NO_BRANCH;
 #pragma unroll
-    for (int iv = 0; iv < C::NEQ; ++iv) Fn[iv] = 0.0;
+    for (int d = 0; d < 3; d++) unc[d] = 0.0;
+    return st;  // adds nothing
+  }
+  const bool left = branch <= 1, starred = branch == 1 || branch == 2;
+  Sol<N> K;
+  select_sol<N>(left, L, R, K);
+  const double SK = left ? SL : SR;
+  if (starred)
+    st |= star_region<F>(k, K, L.r, R.r, f64::gt0(L.phi0) && f64::gt0(R.phi0), left, u_S, SL, SR,
+                         uL, vL, wL, uR, vR, wR, sL, sR, Us, nc);
+  flux_n<F>(K, branch, gfm, k.flux_form == FFV_FLUX_CONSISTENT, nc, Fn);
 #pragma unroll
-    for (int d = 0; d < 3; d++) nc.unc[d] = 0.0;
+  for (int iv = 0; iv < C::NC; ++iv) {
+    const double corr = starred ? SK * (Us[iv] - K.vec[iv]) : 0.0;
+    ff[iv] += (Area) * (Fn[iv] + corr);
   }
 #pragma unroll
-  for (int iv = 0; iv < C::NEQ; ++iv)
-    ff[iv] += (Area) * (Fn[iv] + (iv < C::NC ? corr[iv] : 0.0));
+  for (int iv = C::NC; iv < C::i5; ++iv) ff[iv] += (Area) * Fn[iv];
+  // (the deformation's flux of a fluid state is a zero)
+  if (!K.flat)
+#pragma unroll
+    for (int iv = C::i5; iv < C::NEQ; ++iv) ff[iv] += (Area) * Fn[iv];
 #pragma unroll
   for (int d = 0; d < 3; d++) unc[d] = nc.unc[d];
   return st;
@@ -444,70 +521,188 @@ __device__ void symmetry_acc(const Sol<N> &Lc, bool cons, double Area, double *f
 }
 
 // ------------------------------------------------------------ relaxation (m5_relaxationvec.c)
+// the N - 1 fractions scaled so that their sum is the upper bound
+template <int N>
+__device__ __forceinline__ void scale_vf(const M5Consts &k, double *avf, double sum) {
+  const double dif = sum - k.hi;
+  const f64::Rcp rs = f64::rcp(sum);
+#pragma unroll
+  for (int j = 0; j < N - 1; ++j) avf[j] = avf[j] - f64::div(avf[j], rs) * dif;
+}
+
 template <int N>
 __device__ __forceinline__ void vf_limit_relax(const M5Consts &k, double *avf, bool elseif) {
-  const double lo = k.amin / 100.0, hi = 1.0 - (k.amin / 100.0);
   double sum = 0.0;
 #pragma unroll
   for (int i = 0; i < N - 1; ++i) {
-    if (elseif) {
-      if (avf[i] <= lo) avf[i] = lo;
-      else if (avf[i] >= hi) avf[i] = hi;
-    } else {
-      if (avf[i] <= lo) avf[i] = lo;
-      if (avf[i] >= hi) avf[i] = hi;
-    }
-    sum += avf[i];
+    if (f64::le(avf[i], k.lo)) avf[i] = k.lo;
+    else if (f64::ge(avf[i], k.hi)) avf[i] = k.hi;
+    if (!elseif && f64::ge(avf[i], k.hi)) avf[i] = k.hi;  // two ifs: a lower bound above the upper
+    sum = i ? sum + avf[i] : avf[i];
   }
-  if (sum >= hi) {
-    const double dif = sum - hi;
-#pragma unroll
-    for (int j = 0; j < N - 1; ++j) {
-      const double per = avf[j] / sum;
-      avf[j] = avf[j] - per * dif;
-    }
-    sum = hi;
+  if (f64::ge(sum, k.hi)) {
+    scale_vf<N>(k, avf, sum);
+    sum = k.hi;
   }
   avf[N - 1] = 1.0 - sum;
 }
 
+// 1 / x to about an ulp, for 1e-37 < |x| < 1e37: the FP32 reciprocal (conversions on the integer
+// pipe) and two Newton-Raphson steps of x r = 1
+__device__ __forceinline__ double rcp_near(double x) {
+  double r = f64_of_f32(1.0f / f32_of_f64(x));
+  r = fma(fma(-x, r, 1.0), r, r);
+  return fma(fma(-x, r, 1.0), r, r);
+}
+
+// Newton on sum_k alpha_k(p) = 1 along each material's isentrope (m5_relaxationvec.c:456-490), to
+// |F| <= 1e-12 or the reference's cap of 500 iterations; alpha[k] receives the last iterate's
+// fractions, the return value is true when an iterate is NaN.  The reference's arithmetic: an
+// iterate that repeats bitwise is a fixed point (F, dF and the densities repeat with it), so
+// leaving there gives exactly the reference's result.  Most non-converging face states of a stiff
+// two-phase interface reach such a point within a few iterations and would otherwise spin to the
+// cap.
 template <int N>
+__device__ __forceinline__ bool newton_reference(const M5Consts &k, const double *avf,
+                                                 const double *ar, const bool *live,
+                                                 const double *pk, double p, double *alpha) {
+  double rk[N];
+  f64::Rcp den[N];
+#pragma unroll
+  for (int iv = 0; iv < N; ++iv) {
+    alpha[iv] = 0.0;
+    if (live[iv]) {
+      rk[iv] = ar[iv] / avf[iv];
+      den[iv] = f64::rcp(pk[iv] + k.pinf[iv]);
+    }
+  }
+  double F = 1.0e-9, dF = 1.0e9, p_prev = NAN;
+#pragma unroll 1
+  for (int iter = 0; f64::abs_gt(F, 1.0e-12) && iter < 500; iter++) {
+    p = p - F / dF;
+#pragma unroll
+    for (int iv = 0; iv < N; ++iv)
+      if (f64::lt(p, k.pfloor[iv])) p = k.preset[iv];
+    F = -1.0;
+    dF = 0.0;
+#pragma unroll
+    for (int iv = 0; iv < N; ++iv) {
+      if (live[iv]) {
+        const double pp = p + k.pinf[iv];
+        const double rho = rk[iv] * pow(f64::div(pp, den[iv]), k.igam[iv]);
+        alpha[iv] = ar[iv] / rho;
+        F = F + alpha[iv];
+        dF = dF - ar[iv] / (k.gamma[iv] * rho * pp);
+      }
+    }
+    if (f64::is_nan(p) || f64::is_nan(F) || f64::is_nan(dF)) return true;
+    if (p == p_prev) break;
+    p_prev = p;
+  }
+  return false;
+}
+
+// The same iteration without a reference to equal bit for bit (the consistent flux form).  The
+// ratio x = (p + p_inf) / (p_k + p_inf) is near 1 in all but the cells of an interface or a strong
+// shock: for |x - 1| <= 1/32 the power is 1 + t P(t), t = x - 1 (exact), P the binomial series to t^9
+// (the first omitted term is below 3e-18), rounded once -- an error of at most 0.53 ulp, below
+// pow's.  Reciprocals of the two other quotients' divisors take Newton-Raphson steps; the
+// fraction itself is corrected by its remainder.  31 FP64 instructions per material and iteration
+// against ~110 with pow and three divisions; the iterates differ from the reference's in the last
+// bit at most, so that the stopping test falls alike (a series in p - p_k, more exact still, moved
+// it in one state of 200,000, and with it a fraction by 1e-12).
+template <int N>
+__device__ __forceinline__ bool newton_series(const M5Consts &k, const double *avf,
+                                              const double *ar, const bool *live,
+                                              const double *pk, double p, double *alpha) {
+  double rk[N];
+  f64::Rcp den[N];
+#pragma unroll
+  for (int iv = 0; iv < N; ++iv) {
+    alpha[iv] = 0.0;
+    if (live[iv]) {
+      rk[iv] = ar[iv] / avf[iv];
+      den[iv] = f64::rcp(pk[iv] + k.pinf[iv]);
+    }
+  }
+  double F = 1.0e-9, dF = 1.0e9, p_prev = NAN;
+#pragma unroll 1
+  for (int iter = 0; f64::abs_gt(F, 1.0e-12) && iter < 500; iter++) {
+    p = p - F / dF;
+#pragma unroll
+    for (int iv = 0; iv < N; ++iv)
+      if (f64::lt(p, k.pfloor[iv])) p = k.preset[iv];
+    F = -1.0;
+    dF = 0.0;
+#pragma unroll
+    for (int iv = 0; iv < N; ++iv) {
+      if (live[iv]) {
+        const double pp = p + k.pinf[iv], x = f64::div(pp, den[iv]), t = x - 1.0;
+        double pw;
+        if (f64::abs_bits(t) <= 0x3fa0000000000000ull) {  // 1/32
+          const double *c = k.binom[iv];
+          pw = c[9];
+#pragma unroll
+          for (int j = 8; j >= 0; j--) pw = fma(pw, t, c[j]);
+          pw = fma(pw, t, 1.0);
+        } else {
+          pw = pow(x, k.igam[iv]);
+        }
+        const double rho = rk[iv] * pw, r = rcp_near(rho), q = ar[iv] * r;
+        alpha[iv] = fma(fma(-q, rho, ar[iv]), r, q);
+        F = F + alpha[iv];
+        dF = fma(-alpha[iv], rcp_near(k.gamma[iv] * pp), dF);
+      }
+    }
+    if (f64::is_nan(p) || f64::is_nan(F) || f64::is_nan(dF)) return true;
+    if (p == p_prev) break;
+    p_prev = p;
+  }
+  return false;
+}
+
+template <int N, bool FAST>
 __device__ unsigned relaxationvec(const M5Consts &k, double *V) {
   using C = K5<N>;
-  double ar[N], are[N], avf[N], avf0[N], A[9], G[9], Gmag;
+  double ar[N], are[N], avf[N], avf0[N], ael[N];
   double rho = 0.0;
 #pragma unroll
   for (int iv = 0; iv < N; ++iv) {
     ar[iv] = V[iv + C::i0];
     are[iv] = V[iv + C::i4];
-    rho += ar[iv];
+    rho = iv ? rho + ar[iv] : ar[iv];
   }
-  const double u = V[C::i1 + 0] / rho, v = V[C::i1 + 1] / rho, w = V[C::i1 + 2] / rho;
+  const f64::Rcp rr = f64::rcp(rho);
+  const double u = f64::div(V[C::i1 + 0], rr), v = f64::div(V[C::i1 + 1], rr),
+               w = f64::div(V[C::i1 + 2], rr);
   const double rE = V[C::i2];
 #pragma unroll
   for (int iv = 0; iv < N - 1; ++iv) avf[iv] = V[iv + C::i3];
   vf_limit_relax<N>(k, avf, true);
 #pragma unroll
   for (int iv = 0; iv < N; ++iv) avf0[iv] = avf[iv];
+  {
+    Elastic el;
+    elastic_of(k, V + C::i5, el);
 #pragma unroll
-  for (int q = 0; q < 9; q++) A[q] = V[q + C::i5];
-  gmat_of(A, G, Gmag);
-  const double eps_sml = 1.0e-12, eps_big = 1.0e-8;
+    for (int iv = 0; iv < N; ++iv) ael[iv] = elastic_energy(el, k.mu[iv]);
+  }
+  const double eps_sml = 1.0e-12;
   unsigned st = 0;
-  if (k.prelax == 1) {
+  int i_as = 0;
+  if (N == 2 && k.prelax == 1) {  // closed form for two materials (only)
     double t0[N], p0[N];
 #pragma unroll
     for (int iv = 0; iv < N; ++iv) {
-      const double ael = (k.mu[iv] != 0.0) ? elastic_energy(G, Gmag, k.mu[iv], false) : 0.0;
       t0[iv] = 1.0 / (ar[iv] / avf[iv]);
-      p0[iv] = ((k.gamma[iv] - 1.0) * (are[iv] - ael) / avf[iv]) - k.gamma[iv] * k.pinf[iv];
+      p0[iv] = (k.gm1[iv] * (are[iv] - ael[iv]) / avf[iv]) - k.gpi[iv];
     }
     const double *ga = k.gamma, *pi = k.pinf;
     const double A_1 = (avf[0] / ga[0]) * (p0[0] + pi[0]) / ((avf[0] / ga[0]) + (avf[1] / ga[1]));
     const double A_2 = (avf[1] / ga[1]) * (p0[1] + pi[1]) / ((avf[0] / ga[0]) + (avf[1] / ga[1]));
     const double d = (A_2 - A_1 - (pi[1] - pi[0]));
     const double pe = 0.5 * (A_1 + A_2 - (pi[0] + pi[1])) + sqrt(0.25 * (d * d) + A_1 * A_2);
-    if (isnan(pe)) st |= FFV_ST_NAN;
+    if (f64::is_nan(pe)) st |= FFV_ST_NAN;
 #pragma unroll
     for (int iv = 0; iv < N; ++iv) {
       const double t1 = t0[iv] * (p0[iv] + ga[iv] * pi[iv] + (ga[iv] - 1.0) * pe) /
@@ -516,112 +711,80 @@ __device__ unsigned relaxationvec(const M5Consts &k, double *V) {
       avf[iv] = ar[iv] / rm;
     }
     vf_limit_relax<N>(k, avf, false);
-#pragma unroll
-    for (int q = 0; q < 9; q++) A[q] = A[q] * (avf[0] / avf0[0]);
   } else {  // PRELAX 3
-    double rhoKs[N], pkinit[N];
+    double pkinit[N];
+    bool live[N], irelax = true;
 #pragma unroll
     for (int iv = 0; iv < N; ++iv) {
-      if (avf[iv] < 0.0 || ar[iv] < 0.0) {
+      if (f64::lt0(avf[iv]) || f64::lt0(ar[iv])) {
         avf[iv] = eps_sml;
         ar[iv] = eps_sml;
         are[iv] = eps_sml;
       }
-      if (avf[iv] >= 1.0) avf[iv] = 1.0 - eps_sml;
+      if (f64::ge(avf[iv], 1.0)) avf[iv] = 1.0 - eps_sml;
     }
-    bool irelax = true;
 #pragma unroll
     for (int iv = 0; iv < N; ++iv)
-      if (avf[iv] > 1.0 - eps_sml) irelax = false;
+      if (f64::gt(avf[iv], 1.0 - eps_sml)) irelax = false;
     if (irelax) {
-      double p_relaxed = 0.0;
+      double p0 = 0.0;
 #pragma unroll
       for (int iv = 0; iv < N; ++iv) {
-        if (avf[iv] > eps_sml) {
-          const double ael = (k.mu[iv] != 0.0) ? elastic_energy(G, Gmag, k.mu[iv], false) : 0.0;
-          pkinit[iv] = ((k.gamma[iv] - 1.0) * (are[iv] - ael) / avf[iv]) - k.gamma[iv] * k.pinf[iv];
-          if (pkinit[iv] <= -(1.0 - eps_big) * k.pinf[iv] + eps_big)
-            pkinit[iv] = -(1.0 - eps_big) * k.pinf[iv] + eps_big;
-        } else {
-          pkinit[iv] = 0.0;
+        live[iv] = f64::gt(avf[iv], eps_sml);
+        pkinit[iv] = 0.0;
+        if (live[iv]) {
+          pkinit[iv] = (k.gm1[iv] * (are[iv] - ael[iv]) / avf[iv]) - k.gpi[iv];
+          if (f64::le(pkinit[iv], k.pfloor[iv])) pkinit[iv] = k.pfloor[iv];
         }
-        p_relaxed += avf[iv] * pkinit[iv];
+        p0 += avf[iv] * pkinit[iv];
       }
-      int iter = 0;
-      double F = 1.0e-9, dF = 1.0e9, p_prev = NAN;
-#pragma unroll
-      for (int iv = 0; iv < N; ++iv) rhoKs[iv] = 0.0;
-      // the reference's own iteration cap (m5_relaxationvec.c:458) bounds this loop.  An
-      // iterate that repeats bitwise is a fixed point: F, dF and rhoKs repeat with it, so
-      // the remaining iterations up to the cap would recompute the same values -- leaving
-      // there gives exactly the reference's result (most non-converging face states of a
-      // stiff two-phase interface reach such a point within a few iterations and would
-      // otherwise spin to the cap).
-      while ((fabs(F) > 1.0e-12) && (iter < 500)) {
-        p_relaxed = p_relaxed - F / dF;
-        iter = iter + 1;
-#pragma unroll
-        for (int iv = 0; iv < N; ++iv)
-          if (p_relaxed < -(1.0 - eps_big) * k.pinf[iv] + eps_big)
-            p_relaxed = -(1.0 - eps_big) * k.pinf[iv] + 1.0;
-        F = -1.0;
-        dF = 0.0;
-#pragma unroll
-        for (int iv = 0; iv < N; ++iv) {
-          if (avf[iv] > eps_sml) {
-            const double am = (avf[iv] > eps_sml) ? avf[iv] : eps_sml;
-            rhoKs[iv] = ar[iv] / am *
-                        pow((p_relaxed + k.pinf[iv]) / (pkinit[iv] + k.pinf[iv]), 1.0 / k.gamma[iv]);
-            F = F + ar[iv] / rhoKs[iv];
-            dF = dF - ar[iv] / (k.gamma[iv] * rhoKs[iv] * (p_relaxed + k.pinf[iv]));
-          }
-        }
-        if (isnan(p_relaxed) || isnan(F) || isnan(dF)) {
-          st |= FFV_ST_NAN;
-          break;
-        }
-        if (p_relaxed == p_prev) break;
-        p_prev = p_relaxed;
-      }
+      double alpha[N];
+      const bool nan = FAST ? newton_series<N>(k, avf, ar, live, pkinit, p0, alpha)
+                            : newton_reference<N>(k, avf, ar, live, pkinit, p0, alpha);
+      if (nan) st |= FFV_ST_NAN;
 #pragma unroll
       for (int iv = 0; iv < N; ++iv)
-        if (avf[iv] > eps_sml) avf[iv] = ar[iv] / rhoKs[iv];
+        if (live[iv]) avf[iv] = alpha[iv];
       vf_limit_relax<N>(k, avf, true);
     }
-    const int i_as = ((avf[0] < avf[1]) && (k.mu[1] != 0.0)) ? 1 : 0;
+    i_as = (k.mu[1] != 0.0 && avf[0] < avf[1]) ? 1 : 0;
+  }
+  // the deformation scales with the solid's fraction; a fluid's is zero
+  if (!no_deformation(V + C::i5)) {
     const double ratio = avf[i_as] / avf0[i_as];
 #pragma unroll
-    for (int q = 0; q < 9; q++) A[q] = A[q] * ratio;
+    for (int q = 0; q < 9; q++) V[q + C::i5] = V[q + C::i5] * ratio;
   }
-  double e_elast = 0.0, ael_t[N];
+  double e_elast = 0.0;
 #pragma unroll
   for (int iv = 0; iv < N; ++iv) {
-    ael_t[iv] = (k.mu[iv] != 0.0) ? elastic_energy(G, Gmag, k.mu[iv], false) : 0.0;
-    const double eK = ael_t[iv] / (ar[iv]);
-    const double Ys = ar[iv] / rho;
+    // a zero elastic energy adds a zero (where the quotients are defined)
+    if (f64::abs_bits(ael[iv]) == 0 && f64::moderate(ar[iv]) && f64::moderate(rho)) continue;
+    const double eK = ael[iv] / (ar[iv]);
+    const double Ys = f64::div(ar[iv], rr);
     e_elast += Ys * eK;
   }
-  const double e_hyd = rE / rho - 0.5 * (u * u + v * v + w * w) - e_elast;
+  const double e_hyd = f64::div(rE, rr) - 0.5 * (u * u + v * v + w * w) - e_elast;
   double num = 0.0, den = 0.0;
 #pragma unroll
   for (int iv = 0; iv < N; ++iv) {
-    num += avf[iv] * k.gamma[iv] * k.pinf[iv] / (k.gamma[iv] - 1.0);
-    den += avf[iv] / (k.gamma[iv] - 1.0);
+    const f64::Rcp g1{k.gm1[iv], k.ig1[iv]};
+    num += f64::div(avf[iv] * k.gamma[iv] * k.pinf[iv], g1);
+    den += f64::div(avf[iv], g1);
   }
   const double p_relaxed = (rho * e_hyd - num) / den;
 #pragma unroll
   for (int iv = 0; iv < N - 1; ++iv) {
-    if (isnan(avf[iv])) st |= FFV_ST_NAN;
+    if (f64::is_nan(avf[iv])) st |= FFV_ST_NAN;
     V[iv + C::i3] = avf[iv];
   }
 #pragma unroll
   for (int iv = 0; iv < N; iv++) {
-    const double a2 = (avf[iv] * (p_relaxed + k.gamma[iv] * k.pinf[iv]) / (k.gamma[iv] - 1.0)) + ael_t[iv];
-    if (isnan(a2)) st |= FFV_ST_NAN;
+    const f64::Rcp g1{k.gm1[iv], k.ig1[iv]};
+    const double a2 = f64::div(avf[iv] * (p_relaxed + k.gpi[iv]), g1) + ael[iv];
+    if (f64::is_nan(a2)) st |= FFV_ST_NAN;
     V[iv + C::i4] = a2;
   }
-#pragma unroll
-  for (int q = 0; q < 9; ++q) V[q + C::i5] = A[q];
   return st;
 }
 
@@ -629,24 +792,13 @@ __device__ unsigned relaxationvec(const M5Consts &k, double *V) {
 template <int N>
 __device__ __forceinline__ void avf_limit(const M5Consts &k, double *S) {
   using C = K5<N>;
-  const double lo = k.amin / 100.0, hi = 1.0 - (k.amin / 100.0);
   double sum = 0.0;
 #pragma unroll
   for (int v = 0; v < N - 1; ++v) {
-    double a = S[C::i3 + v];
-    if (a <= lo) a = lo;
-    else if (a >= hi) a = hi;
-    S[C::i3 + v] = a;
-    sum += a;
+    S[C::i3 + v] = clamp_vf(k, S[C::i3 + v]);
+    sum = v ? sum + S[C::i3 + v] : S[C::i3 + v];
   }
-  if (sum > hi) {
-    const double dif = sum - hi;
-#pragma unroll
-    for (int j = 0; j < N - 1; ++j) {
-      const double a = S[C::i3 + j];
-      S[C::i3 + j] = a - (a / sum) * dif;
-    }
-  }
+  if (f64::gt(sum, k.hi)) scale_vf<N>(k, S + C::i3, sum);
 }
 
 template <int N>
@@ -656,44 +808,25 @@ __device__ __forceinline__ void load_state(const double *__restrict__ S, int64_t
   for (int v = 0; v < K5<N>::NEQ; v++) U[v] = S[(int64_t)v * n + c];
 }
 
-// m5_facevalues_MUSCL.c:3-45 (iside 1): value across face f, volume fractions limited
+// m5_facevalues_MUSCL.c:3-45 (iside 1): value across face f, volume fractions limited.  At a
+// boundary the ghost's state vector is the cell's own with the clamped volume fractions of
+// m5_facevalues.c:46-80 (the bc only changes the ghost's primitive velocity).
 template <int N>
-__device__ void value_across(const M5Consts &k, const ffv_dmesh &m, const double *__restrict__ S,
-                             int64_t c, int f, uint32_t kind, const double *Sc, double *X) {
+__device__ __forceinline__ void value_across(const M5Consts &k, const ffv_dmesh &m,
+                                             const double *__restrict__ S, int64_t c, int f,
+                                             uint32_t kind, const double *Sc, double *X) {
   using C = K5<N>;
   if (kind & FFV_FK_BC) {
-    // the ghost's state vector: the cell's own with the clamped volume fractions of
-    // m5_facevalues.c:46-80 (the bc only changes the ghost's primitive velocity)
-    const double lo = k.amin / 100.0, hi = 1.0 - (k.amin / 100.0);
 #pragma unroll
     for (int i = 0; i < C::NEQ; i++) X[i] = Sc[i];
-    double at[N], sum = 0.0;
-#pragma unroll
-    for (int i = 0; i < N - 1; ++i) {
-      at[i] = Sc[C::i3 + i];
-      if (at[i] <= lo) at[i] = lo;
-      else if (at[i] >= hi) at[i] = hi;
-      sum += at[i];
-    }
-    if (sum > hi) {
-      const double dif = sum - hi;
-#pragma unroll
-      for (int j = 0; j < N - 1; ++j) {
-        const double per = at[j] / sum;
-        at[j] = at[j] - per * dif;
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < N - 1; ++i) X[C::i3 + i] = at[i];
+    avf_limit<N>(k, X);
   } else if (kind == FFV_FK_FINER) {
     const int32_t *sg = m.sub + 4 * (int64_t)m.nbr[(int64_t)f * m.n + c];
+    const int64_t s0 = sg[0], s1 = sg[1], s2 = sg[2], s3 = sg[3];
 #pragma unroll
-    for (int i = 0; i < C::NEQ; i++) X[i] = 0.0;
-#pragma unroll 1
-    for (int q = 0; q < 4; q++) {
-      const int64_t o = sg[q];
-#pragma unroll
-      for (int i = 0; i < C::NEQ; i++) X[i] += S[(int64_t)i * m.n + o] / 4.0;
+    for (int i = 0; i < C::NEQ; i++) {
+      const double *Sv = S + (int64_t)i * m.n;
+      X[i] = ((Sv[s0] / 4.0 + Sv[s1] / 4.0) + Sv[s2] / 4.0) + Sv[s3] / 4.0;
     }
   } else {
     load_state<N>(S, m.n, m.nbr[(int64_t)f * m.n + c], X);
@@ -702,73 +835,106 @@ __device__ void value_across(const M5Consts &k, const ffv_dmesh &m, const double
 }
 
 // ------------------------------------------------------------------------------ kernels
+// m5_reconctruct.c:144-179: volume-fraction limits of a face state
 template <int N>
-__global__ void __launch_bounds__(128) m5_recon_face(ffv_dmesh m, ffv_geom g, M5Consts k,
-                                                     const double *__restrict__ S,
-                                                     double *__restrict__ SF,
-                                                     unsigned *__restrict__ status) {
-  using C = K5<N>;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 6 * m.n) return;
-  const int f = (int)(t / m.n);
-  const int64_t c = t - (int64_t)f * m.n;
-  const int fo = fr_opp(f);
-  const uint32_t info = m.info[c];
-  const int l = ffv_info_level(info);
-  const uint32_t kf = ffv_face_kind(info, f), ko = ffv_face_kind(info, fo);
-  double Sc[C::NEQ], SL[C::NEQ], X[C::NEQ], out[C::NEQ];
-  load_state<N>(S, m.n, c, Sc);
-#pragma unroll
-  for (int i = 0; i < C::NEQ; i++) SL[i] = Sc[i];
-  avf_limit<N>(k, SL);
-  value_across<N>(k, m, S, c, f, kf, Sc, X);
-  double df[C::NEQ];
-#pragma unroll
-  for (int i = 0; i < C::NEQ; i++) df[i] = X[i] - SL[i];
-  value_across<N>(k, m, S, c, fo, ko, Sc, X);
-  const double dp = g.dcc[l][face_class(kf)], dm = g.dcc[l][face_class(ko)];
-  const double cf = g.dcf[l][face_class(kf)];
-#pragma unroll
-  for (int i = 0; i < C::NEQ; i++) {
-    const double db = X[i] - SL[i];
-    double grad = 0.0;
-    if (!(kf & FFV_FK_BC)) {
-      if (fabs(df[i]) > 1e-10) {
-        const double product = (-db / dm) * (df[i] / dp);
-        if (product > 0.0) {
-          const double lim = (i >= C::i4 && i < C::i5) ? 0.0 : 1.0;
-          if (fabs(-db / dm) > fabs(df[i] / dp))
-            grad = lim * (df[i] / dp);
-          else
-            grad = lim * (-db / dm);
-        }
-      }
-    }
-    out[i] = SL[i] + cf * grad;
-  }
-  // m5_reconctruct.c:144-179: volume-fraction limits of the face state
-  const double lo = k.amin / 100.0;
-  double avf[N], sum = 0.0;
+__device__ __forceinline__ void face_vf_limit(const M5Consts &k, double *avf) {
+  const double top = 1.0 - (2.0 * k.lo);
+  double sum = 0.0;
 #pragma unroll
   for (int iv = 0; iv < N - 1; ++iv) {
-    avf[iv] = out[iv + C::i3];
-    if (avf[iv] <= lo) avf[iv] = lo;
-    else if (avf[iv] >= (1.0 - (2.0 * lo))) avf[iv] = 1.0 - (2.0 * lo);
-    sum += avf[iv];
+    if (f64::le(avf[iv], k.lo)) avf[iv] = k.lo;
+    else if (f64::ge(avf[iv], top)) avf[iv] = top;
+    sum = iv ? sum + avf[iv] : avf[iv];
   }
-  if (sum >= (1.0 - lo)) {
-    const double dif = sum - (1.0 - lo);
+  if (f64::ge(sum, k.hi)) scale_vf<N>(k, avf, sum);
+}
+
+// The limited, not yet relaxed states of the two faces of one axis (blockIdx.y) of every cell:
+// both faces' increments come from the same two one-sided slopes.  Between neighbours of the
+// cell's own level at a power-of-two spacing the limiter works on bit patterns
+// (f64::minmod_pair): four FP64 instructions per variable and axis, against ~50 with four divisions
+// per face.  The internal energies keep the cell's value (the reference multiplies their slope
+// by zero).  The states go to memory and m5_relax_faces relaxes them there: with six face
+// states per cell in flight separately the FP64 pipe has more warps to take from, and the
+// extra traffic (2 KB per cell) is 2 % of the FP64 time.
+template <int N, int FA, int FB>
+__device__ __forceinline__ void slopes_axis(const ffv_dmesh &m, const ffv_geom &g,
+                                            const M5Consts &k, const double *__restrict__ S,
+                                            double *__restrict__ SF, int64_t c) {
+  using C = K5<N>;
+  static_assert(fr_opp(FA) == FB, "opposite faces");
+  const uint32_t info = m.info[c];
+  const int l = ffv_info_level(info);
+  const uint32_t ka = ffv_face_kind(info, FA), kb = ffv_face_kind(info, FB);
+  double SL[C::NEQ], XA[C::NEQ], XB[C::NEQ];
+  load_state<N>(S, m.n, c, SL);
+  value_across<N>(k, m, S, c, FA, ka, SL, XA);
+  value_across<N>(k, m, S, c, FB, kb, SL, XB);
+  avf_limit<N>(k, SL);
+  const bool plain = ka == FFV_FK_SAME && kb == FFV_FK_SAME && ((g.pow2 >> l) & 1u);
+  const f64::Rcp da{g.dcc[l][face_class(ka)], g.rdcc[l][face_class(ka)]};
+  const f64::Rcp db{g.dcc[l][face_class(kb)], g.rdcc[l][face_class(kb)]};
+  const double fa = g.dcf[l][face_class(ka)], fb = g.dcf[l][face_class(kb)];
+  const bool ba = (ka & FFV_FK_BC) != 0, bb = (kb & FFV_FK_BC) != 0;
 #pragma unroll
-    for (int j = 0; j < N - 1; ++j) {
-      const double per = avf[j] / sum;
-      avf[j] = avf[j] - per * dif;
+  for (int i = 0; i < C::NEQ; i++) {
+    double cA = 0.0, cB = 0.0;
+    if (i < C::i4 || i >= C::i5) {
+      const double dA = XA[i] - SL[i], dB = XB[i] - SL[i];
+      if (plain) {
+        f64::minmod_pair(dA, dB, da.r, cA, cB);
+      } else if (!(ba || bb) || (i >= C::i3 && i < C::i4)) {
+        // (next to a boundary only a volume fraction scaled twice can differ from the cell's: the
+        // other variables' slopes there are 0 / 0)
+        const double a = f64::div(dA, da), b = f64::div(dB, db);
+        const bool opposed = f64::gt0(f64::neg(b) * a);
+        const double ga = f64::abs_gt(b, a) ? a : f64::neg(b);
+        const double gb = f64::abs_gt(a, b) ? b : f64::neg(a);
+        if (!ba && opposed && f64::abs_gt(dA, 1e-10)) cA = fa * ga;
+        if (!bb && opposed && f64::abs_gt(dB, 1e-10)) cB = fb * gb;
+      }
     }
+    XA[i] = SL[i] + cA;
+    XB[i] = SL[i] + cB;
   }
+  face_vf_limit<N>(k, XA + C::i3);
+  face_vf_limit<N>(k, XB + C::i3);
 #pragma unroll
-  for (int iv = 0; iv < N - 1; ++iv) out[iv + C::i3] = avf[iv];
-  const unsigned st = relaxationvec<N>(k, out);
+  for (int i = 0; i < C::NEQ; i++) {
+    SF[((int64_t)FA * C::NEQ + i) * m.n + c] = XA[i];
+    SF[((int64_t)FB * C::NEQ + i) * m.n + c] = XB[i];
+  }
+}
+
+template <int N>
+__global__ void __launch_bounds__(128) m5_recon_slopes(ffv_dmesh m, ffv_geom g, M5Consts k,
+                                                       const double *__restrict__ S,
+                                                       double *__restrict__ SF) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= m.n) return;
+  if (blockIdx.y == 0) slopes_axis<N, 0, 2>(m, g, k, S, SF, c);
+  else if (blockIdx.y == 1) slopes_axis<N, 3, 1>(m, g, k, S, SF, c);
+  else slopes_axis<N, 4, 5>(m, g, k, S, SF, c);
+}
+
+// Pressure relaxation of every face state (blockIdx.y the face), in place.  FP64 pipe 84 % busy; a
+// warp runs as long as its slowest lane's Newton iteration (3.9 iterations on the wall mesh, 6 on
+// the bubble's, the mean lane 2.8 and 3.9).  Slopes and relaxation in one kernel with the plain
+// arithmetic took 11.35 ms per stage on the wall mesh (0.41 M cells); now 0.58 + 5.0 ms, and in
+// the reference's form on the bubble mesh (51,584 cells) 1.94-2.54 ms against 0.11 + 1.5-2.1 ms.
+template <int N, bool FAST>
+__global__ void __launch_bounds__(128) m5_relax_faces(int64_t n, M5Consts k, double *SF,
+                                                      unsigned *__restrict__ status) {
+  using C = K5<N>;
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  double *U = SF + (int64_t)blockIdx.y * C::NEQ * n + c;
+  double V[C::NEQ];
 #pragma unroll
-  for (int i = 0; i < C::NEQ; i++) SF[((int64_t)f * C::NEQ + i) * m.n + c] = out[i];
+  for (int i = 0; i < C::NEQ; i++) V[i] = U[(int64_t)i * n];
+  const unsigned st = relaxationvec<N, FAST>(k, V);
+#pragma unroll
+  for (int i = C::i3; i < C::NEQ; i++) U[(int64_t)i * n] = V[i];  // the rest is unchanged
   if (st) atomicOr(status, st);
 }
 
@@ -779,8 +945,10 @@ __device__ __forceinline__ void load_face_state(const double *__restrict__ SF, i
   for (int v = 0; v < K5<N>::NEQ; v++) U[v] = SF[((int64_t)f * K5<N>::NEQ + v) * n + c];
 }
 
-// face flux of cell c through face F (all subfaces), the reference's reuse included
-template <int N, int F>
+// Face flux of cell c through face F (all subfaces), the reference's reuse included.  FP64 pipe
+// 79 % busy; wall mesh (0.41 M cells) 6.2 -> 3.6 ms per stage, bubble mesh (51,584 cells) 0.90 ->
+// 0.40 ms by one solver evaluation per warp, shared reciprocals and the fluid states' zero terms.
+template <int N, int ORDER, int F>
 __device__ void face_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
                           const double *__restrict__ S, const double *__restrict__ SF, int64_t c,
                           uint32_t info, double *ff, double uf[3], double &gfm_face,
@@ -789,13 +957,11 @@ __device__ void face_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts 
   constexpr int FO = fr_opp(F);
   const uint32_t kind = ffv_face_kind(info, F);
   const int l = ffv_info_level(info);
-  double U[C::NEQ], Sc[C::NEQ], So[C::NEQ];
+  double U[C::NEQ];
 #pragma unroll
   for (int iv = 0; iv < C::NEQ; iv++) ff[iv] = 0.0;
   uf[0] = uf[1] = uf[2] = 0.0;
   gfm_face = 0.0;
-  Sol<N> L, R;
-  load_state<N>(S, m.n, c, Sc);
   if (kind == FFV_FK_SAME && m.nbr[(int64_t)F * m.n + c] < c) {
     // 1:1 face whose neighbour comes first in leaf order: the neighbour's thread evaluates
     // it (face F^1 of the neighbour) and m5_cell_update takes the negative, as the
@@ -803,43 +969,49 @@ __device__ void face_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts 
     owner = false;
     return;
   }
+  const auto phi_at = [&](int64_t o) {
+    return phi0_of<N>(k, S[(int64_t)C::i3 * m.n + o], N > 2 ? S[(int64_t)(C::i3 + 1) * m.n + o] : 0.0);
+  };
+  Sol<N> L, R;
   if (kind == (FFV_FK_BC | FFV_BC_SYMMETRY)) {
     // the cell's own state, not the face state; the HLLC flux the reference computes first
     // for this face is discarded (m5_hllc.c:59-63)
-    make_sol<N>(k, Sc, Sc, false, L);
+    load_state<N>(S, m.n, c, U);
+    make_sol<N>(k, U, 0.0, false, L);
     symmetry_acc<F, N>(L, k.flux_form == FFV_FLUX_CONSISTENT, g.area[l], ff, uf);
     return;
   }
-  if (k.order == 2) load_face_state<N>(SF, m.n, F, c, U);
-  make_sol<N>(k, k.order == 2 ? U : Sc, Sc, k.order == 2, L);
-  if (kind & FFV_FK_BC) {
-    const int bc = (int)(kind & 7u);
-    ghost<F, N>(L, bc, R);
-    const bool gfm = L.phi0 * R.phi0 < 0.0;
-    if (gfm) gfm_face = 1.0;
-    st |= hllc_acc<F, N>(k, L, R, bc, gfm, g.area[l], ff, uf);
-    return;
-  }
+  if (ORDER == 2) load_face_state<N>(SF, m.n, F, c, U);
+  else load_state<N>(S, m.n, c, U);
+  make_sol<N>(k, U, phi_at(c), ORDER == 2, L);
+  // one solver call site for the boundary (the ghost state) and the interior faces (the
+  // neighbour's state, or each of four finer neighbours' in turn)
+  const int bc = (kind & FFV_FK_BC) ? (int)(kind & 7u) : 0;
   const int nsub = kind == FFV_FK_FINER ? 4 : 1;
   const double A = kind == FFV_FK_FINER ? g.area[l + 1] : g.area[l];
+  const double share = kind == FFV_FK_FINER ? 0.25 : 1.0;
   const int32_t *sg = kind == FFV_FK_FINER ? m.sub + 4 * (int64_t)m.nbr[(int64_t)F * m.n + c] : nullptr;
 #pragma unroll 1
   for (int q = 0; q < nsub; q++) {
-    const int64_t o = sg ? sg[q] : m.nbr[(int64_t)F * m.n + c];
-    load_state<N>(S, m.n, o, So);
-    if (k.order == 2) load_face_state<N>(SF, m.n, FO, o, U);
-    make_sol<N>(k, k.order == 2 ? U : So, So, k.order == 2, R);
-    const bool gfm = L.phi0 * R.phi0 < 0.0;
+    if (bc) {
+      ghost<F, N>(L, bc, R);
+    } else {
+      const int64_t o = sg ? sg[q] : m.nbr[(int64_t)F * m.n + c];
+      if (ORDER == 2) load_face_state<N>(SF, m.n, FO, o, U);
+      else load_state<N>(S, m.n, o, U);
+      make_sol<N>(k, U, phi_at(o), ORDER == 2, R);
+    }
+    const bool gfm = (f64::gt0(L.phi0) && f64::lt0(R.phi0)) || (f64::lt0(L.phi0) && f64::gt0(R.phi0));
     if (gfm) gfm_face = 1.0;
     double un[3];
-    st |= hllc_acc<F, N>(k, L, R, 0, gfm, A, ff, un);
-    uf[0] = un[0] / ((double)nsub);
-    uf[1] = un[1] / ((double)nsub);
-    uf[2] = un[2] / ((double)nsub);
+    st |= hllc_acc<F, N>(k, L, R, bc, gfm, A, ff, un);
+    uf[0] = un[0] * share;
+    uf[1] = un[1] * share;
+    uf[2] = un[2] * share;
   }
 }
 
-template <int N>
+template <int N, int ORDER>
 __global__ void __launch_bounds__(128) m5_face_flux(ffv_dmesh m, ffv_geom g, M5Consts k,
                                                     const double *__restrict__ S,
                                                     const double *__restrict__ SF,
@@ -857,12 +1029,12 @@ __global__ void __launch_bounds__(128) m5_face_flux(ffv_dmesh m, ffv_geom g, M5C
   unsigned st = 0;
   bool owner = true;
   switch (f) {
-    case 0: face_flux<N, 0>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
-    case 1: face_flux<N, 1>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
-    case 2: face_flux<N, 2>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
-    case 3: face_flux<N, 3>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
-    case 4: face_flux<N, 4>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
-    default: face_flux<N, 5>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
+    case 0: face_flux<N, ORDER, 0>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
+    case 1: face_flux<N, ORDER, 1>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
+    case 2: face_flux<N, ORDER, 2>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
+    case 3: face_flux<N, ORDER, 3>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
+    case 4: face_flux<N, ORDER, 4>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
+    default: face_flux<N, ORDER, 5>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
   }
   if (owner) {
 #pragma unroll
@@ -874,49 +1046,41 @@ __global__ void __launch_bounds__(128) m5_face_flux(ffv_dmesh m, ffv_geom g, M5C
   if (st) atomicOr(status, st);
 }
 
-// residual sum and non-conservative terms (m5_residual.c:171-214) for face F
+// Residual sum and non-conservative terms (m5_residual.c:171-214) for face F.  The reference
+// multiplies every component with the unit normal's; on a Cartesian forest two of the three are
+// zero and the third +-1, so one component's terms remain: u . n = sg u_a, and of the
+// deformation's terms those of the face's axis.
 template <int N, int F>
 __device__ __forceinline__ void nonconservative(const ffv_geom &g, const Sol<N> &Cs,
                                                 const double (*ast)[3][3], uint32_t info, int l,
-                                                double un, double vn, double wn, double *rhs) {
+                                                const double un[3], double *rhs) {
   using C = K5<N>;
   const uint32_t kind = ffv_face_kind(info, F);
-  double Area_f = 0.0;
-  if (kind == FFV_FK_FINER) {
+  // (the reference sums four subface areas: a power-of-two multiple, the same double)
+  const double Af = kind == FFV_FK_FINER ? 4.0 * g.area[l + 1] : g.area[l];
+  constexpr int a = Fr<F, 0>::ax, b = a == 0 ? 1 : 0, d = a == 2 ? 1 : 2;
+  constexpr int sg = Fr<F, 0>::sg;
 #pragma unroll
-    for (int q = 0; q < 4; q++) Area_f += g.area[l + 1];
-  } else {
-    Area_f += g.area[l];
-  }
-  constexpr int a = Fr<F, 0>::ax, sg = Fr<F, 0>::sg;
-  // with n the signed unit axis, u_nc*nx + v_nc*ny + w_nc*nz keeps one term
-  const double nn[3] = {a == 0 ? (double)sg : 0.0, a == 1 ? (double)sg : 0.0, a == 2 ? (double)sg : 0.0};
-  const double nx = nn[0], ny = nn[1], nz = nn[2];
-#pragma unroll
-  for (int iv = 0; iv < N - 1; ++iv) {
-    const double s = Cs.avf[iv];
-    rhs[C::i3 + iv] += Area_f * (s * un * nx + s * vn * ny + s * wn * nz);
-  }
+  for (int iv = 0; iv < N - 1; ++iv) rhs[C::i3 + iv] += Af * sgn<sg>(Cs.avf[iv] * un[a]);
 #pragma unroll
   for (int iv = 0; iv < N; ++iv) {
     const double(*t)[3] = ast[iv];
-    rhs[C::i4 + iv] += Area_f * (t[0][0] * un * nx + t[0][1] * vn * nx + t[0][2] * wn * nx +
-                                 t[1][0] * un * ny + t[1][1] * vn * ny + t[1][2] * wn * ny +
-                                 t[2][0] * un * nz + t[2][1] * vn * nz + t[2][2] * wn * nz);
+    double x;
+    if (Cs.flat) x = sgn<sg>(t[a][a] * un[a]);  // a pressure
+    else x = sgn<sg>(t[a][0] * un[0]) + sgn<sg>(t[a][1] * un[1]) + sgn<sg>(t[a][2] * un[2]);
+    rhs[C::i4 + iv] += Af * x;
   }
-  const double *Am = Cs.A;
-  const double A1 = Am[0], A2 = Am[1], A3 = Am[2], B1 = Am[3], B2 = Am[4], B3 = Am[5],
-               C1 = Am[6], C2 = Am[7], C3 = Am[8];
+  if (Cs.flat) return;
+  // row a: the other two rows with their velocities, the second subtracted
+  // (m5_residual.c:199-214); the other rows: themselves with the normal velocity
+  const double *A = Cs.A;
   double *R5 = rhs + C::i5;
-  R5[0] += Area_f * ((A1 * vn * ny + A1 * wn * nz) + B1 * vn * nx - C1 * wn * nx);
-  R5[1] += Area_f * ((A2 * vn * ny + A2 * wn * nz) + B2 * vn * nx - C2 * wn * nx);
-  R5[2] += Area_f * ((A3 * vn * ny + A3 * wn * nz) + B3 * vn * nx - C3 * wn * nx);
-  R5[3] += Area_f * ((B1 * un * nx + B1 * wn * nz) + A1 * un * ny - C1 * wn * ny);
-  R5[4] += Area_f * ((B2 * un * nx + B2 * wn * nz) + A2 * un * ny - C2 * wn * ny);
-  R5[5] += Area_f * ((B3 * un * nx + B3 * wn * nz) + A3 * un * ny - C3 * wn * ny);
-  R5[6] += Area_f * ((C1 * un * nx + C1 * vn * ny) + A1 * un * nz - B1 * vn * nz);
-  R5[7] += Area_f * ((C2 * un * nx + C2 * vn * ny) + A2 * un * nz - B2 * vn * nz);
-  R5[8] += Area_f * ((C3 * un * nx + C3 * vn * ny) + A3 * un * nz - B3 * vn * nz);
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    R5[3 * a + j] += Af * (sgn<sg>(A[3 * b + j] * un[b]) + sgn<-sg>(A[3 * d + j] * un[d]));
+    R5[3 * b + j] += Af * sgn<sg>(A[3 * b + j] * un[a]);
+    R5[3 * d + j] += Af * sgn<sg>(A[3 * d + j] * un[a]);
+  }
 }
 
 template <int N>
@@ -924,7 +1088,7 @@ __device__ __forceinline__ void clamp_zerou(const M5Consts &k, double *s, const 
   using C = K5<N>;
 #pragma unroll
   for (int v = 0; v < N; v++)
-    if (s[C::i0 + v] < 0.0) s[C::i0 + v] = sn[C::i0 + v];
+    if (f64::lt0(s[C::i0 + v])) s[C::i0 + v] = sn[C::i0 + v];
   constexpr int e5 = C::i5;
   if (k.zerou[0]) {
     s[C::i1 + 0] = sn[C::i1 + 0];
@@ -942,12 +1106,12 @@ __device__ __forceinline__ void clamp_zerou(const M5Consts &k, double *s, const 
 
 // residual + RK stage (m5_RK.c): writes RHS and the new state into Snew; stage-1 cells
 // whose solid fraction crosses AVF_LIM get the partial update and a flag for m5_gfm_seq
-template <int N, typename TF>
+template <int N>
 __global__ void __launch_bounds__(128) m5_cell_update(ffv_dmesh m, ffv_geom g, M5Consts k,
                                                       const double *__restrict__ S,
                                                       double *__restrict__ SN,
-                                                      const TF *__restrict__ FF,
-                                                      const TF *__restrict__ UF,
+                                                      const double *__restrict__ FF,
+                                                      const double *__restrict__ UF,
                                                       double *__restrict__ RHS,
                                                       double *__restrict__ Snew,
                                                       uint8_t *__restrict__ flag,
@@ -962,45 +1126,44 @@ __global__ void __launch_bounds__(128) m5_cell_update(ffv_dmesh m, ffv_geom g, M
   load_state<N>(S, m.n, c, s);
   Sol<N> Cs;
   double ast[N][3][3];
-  make_sol<N>(k, s, s, false, Cs, ast);
+  make_sol<N>(k, s, 0.0, false, Cs, ast);
 #pragma unroll
   for (int iv = 0; iv < C::NEQ; iv++) rhs[iv] = 0.0;
 #define FACE(F)                                                                          \
   {                                                                                      \
     int64_t fc = c;                                                                      \
     int ff = F;                                                                          \
-    double sg = 1.0;                                                                     \
+    bool other = false;                                                                  \
     if (ffv_face_kind(info, F) == FFV_FK_SAME) {                                         \
       const int64_t o = m.nbr[(int64_t)F * m.n + c];                                     \
       if (o < c) {                                                                       \
         fc = o;                                                                          \
         ff = fr_opp(F);                                                                  \
-        sg = -1.0;                                                                       \
+        other = true;                                                                    \
       }                                                                                  \
     }                                                                                    \
     _Pragma("unroll") for (int iv = 0; iv < C::NEQ; iv++) {                              \
-      const double x = (double)FF[((int64_t)ff * C::NEQ + iv) * m.n + fc];               \
-      rhs[iv] += sg < 0.0 ? -x : x;                                                      \
+      const double x = FF[((int64_t)ff * C::NEQ + iv) * m.n + fc];                       \
+      rhs[iv] += other ? f64::neg(x) : x;                                                \
     }                                                                                    \
-    const double u0 = (double)UF[((int64_t)ff * 3 + 0) * m.n + fc];                      \
-    const double u1 = (double)UF[((int64_t)ff * 3 + 1) * m.n + fc];                      \
-    const double u2 = (double)UF[((int64_t)ff * 3 + 2) * m.n + fc];                      \
-    nonconservative<N, F>(g, Cs, ast, info, l, sg < 0.0 ? -u0 : u0, sg < 0.0 ? -u1 : u1, \
-                          sg < 0.0 ? -u2 : u2, rhs);                                     \
+    double un[3];                                                                        \
+    _Pragma("unroll") for (int d = 0; d < 3; d++) {                                      \
+      const double x = UF[((int64_t)ff * 3 + d) * m.n + fc];                             \
+      un[d] = other ? f64::neg(x) : x;                                                   \
+    }                                                                                    \
+    nonconservative<N, F>(g, Cs, ast, info, l, un, rhs);                                 \
   }
   FACE(0) FACE(1) FACE(2) FACE(3) FACE(4) FACE(5)
 #undef FACE
   // a non-positive density in the stage's input is reported (the arithmetic is untouched)
-  double rho_in = 0.0;
-#pragma unroll
-  for (int v = 0; v < N; ++v) rho_in += s[C::i0 + v];
-  unsigned st = rho_in <= 0.0 ? FFV_ST_NEG_DENSITY : 0u;
+  unsigned st = f64::le0(Cs.r) ? FFV_ST_NEG_DENSITY : 0u;
 #pragma unroll
   for (int iv = 0; iv < C::NEQ; iv++) {
-    if (isnan(rhs[iv])) st |= FFV_ST_NAN;
+    if (f64::is_nan(rhs[iv])) st |= FFV_ST_NAN;
     RHS[(int64_t)iv * m.n + c] = rhs[iv];
   }
-  const double dt = *dtp, V = g.vol[l];
+  const double dt = *dtp, iV = g.inv_vol[l];
+  const f64::Rcp V{g.vol[l], iV};
   double sn[C::NEQ];
   if (irk == 1) {
 #pragma unroll
@@ -1018,30 +1181,20 @@ __global__ void __launch_bounds__(128) m5_cell_update(ffv_dmesh m, ffv_geom g, M
       if (k.mu[v] != 0.0) {
         const int e = C::i3 + v;
         const double phi_old = s[e] - k.avf_lim;
-        const double buf = (1.0 / V) * rhs[e];
+        const double buf = iV * rhs[e];
         const double as_new = sn[e] + dt * buf;
         if (phi_old * (as_new - k.avf_lim) < 0.0) gfm = true;
       }
     }
-    if (gfm) {
-#pragma unroll
-      for (int e = C::i2; e < C::NEQ; e++) s[e] = sn[e] + dt * ((1.0 / V) * rhs[e]);
-    } else {
-#pragma unroll
-      for (int e = 0; e < C::NEQ; e++) s[e] = sn[e] + dt * ((1.0 / V) * rhs[e]);
-    }
-  } else if (irk == 2) {
 #pragma unroll
     for (int e = 0; e < C::NEQ; e++)
-      s[e] = (3.0 / 4.0) * sn[e] + (1.0 / 4.0) * s[e] + (1.0 / 4.0) * dt * rhs[e] / V;
-  } else if (irk == 3) {
-#pragma unroll
-    for (int e = 0; e < C::NEQ; e++)
-      s[e] = (1.0 / 3.0) * sn[e] + (2.0 / 3.0) * s[e] + (2.0 / 3.0) * dt * rhs[e] / V;
+      if (!gfm || e >= C::i2) s[e] = sn[e] + dt * (iV * rhs[e]);
   } else {
+    const double a = irk == 2 ? 3.0 / 4.0 : (irk == 3 ? 1.0 / 3.0 : 1.0 / 2.0);
+    const double b = irk == 2 ? 1.0 / 4.0 : (irk == 3 ? 2.0 / 3.0 : 1.0 / 2.0);
+    const double bdt = b * dt;
 #pragma unroll
-    for (int e = 0; e < C::NEQ; e++)
-      s[e] = (1.0 / 2.0) * sn[e] + (1.0 / 2.0) * s[e] + (1.0 / 2.0) * dt * rhs[e] / V;
+    for (int e = 0; e < C::NEQ; e++) s[e] = a * sn[e] + b * s[e] + f64::div(bdt * rhs[e], V);
   }
   if (!gfm) clamp_zerou<N>(k, s, sn);
 #pragma unroll
@@ -1051,7 +1204,7 @@ __global__ void __launch_bounds__(128) m5_cell_update(ffv_dmesh m, ffv_geom g, M
 }
 
 // cell pressure relaxation (m5_relaxation_solid.c:16-32); flags solid-fraction crossings
-template <int N>
+template <int N, bool FAST>
 __global__ void __launch_bounds__(128) m5_relax_cell(int64_t n, M5Consts k,
                                                      const double *__restrict__ Sin,
                                                      double *__restrict__ Sout,
@@ -1063,7 +1216,7 @@ __global__ void __launch_bounds__(128) m5_relax_cell(int64_t n, M5Consts k,
   double s[C::NEQ];
   load_state<N>(Sin, n, c, s);
   const double phi_old = s[C::i3] - k.avf_lim;
-  const unsigned st = relaxationvec<N>(k, s);
+  const unsigned st = relaxationvec<N, FAST>(k, s);
   // the plastic return where the reference's prototype would run it (m5_relaxation_solid.c:14),
   // after the relaxation so that the stored state lies on or inside the yield surface
   if (k.plastic) plastic_return<N>(k, s);
@@ -1104,7 +1257,7 @@ __global__ void __launch_bounds__(32) m5_gfm_seq(ffv_dmesh m, ffv_geom g, M5Cons
 #pragma unroll
     for (int e = 0; e < C::NEQ; e++) own[e] = s_own[e];
     Sol<N> L;
-    make_sol<N>(k, own, own, false, L);
+    make_sol<N>(k, own, phi0_state<N>(k, own), false, L);
     if (lane < 6) {
       const int f = lane;
       const uint32_t kind = ffv_face_kind(info, f);
@@ -1126,7 +1279,7 @@ __global__ void __launch_bounds__(32) m5_gfm_seq(ffv_dmesh m, ffv_geom g, M5Cons
                                                  : m.nbr[(int64_t)f * m.n + c];
           double so[C::NEQ];
           load_state<N>(o < c ? Snew : Sold, m.n, o, so);
-          make_sol<N>(k, so, so, false, R);
+          make_sol<N>(k, so, phi0_state<N>(k, so), false, R);
         }
         phiR = R.phi0;
         vr[0] = R.u;
@@ -1325,7 +1478,7 @@ __global__ void m5_cfl_kernel(ffv_dmesh m, ffv_geom g, M5Consts k, const double 
     double s[K5<N>::NEQ];
     load_state<N>(S, m.n, c, s);
     Sol<N> q;
-    make_sol<N>(k, s, s, false, q);
+    make_sol<N>(k, s, 0.0, false, q);
     const double sp = fmax(fmax(fabs(q.u), fabs(q.v)), fabs(q.w)) + sqrt(q.c2);
     const double dt = g.h[ffv_info_level(m.info[c])] / sp;
     best = (dt < best || isnan(dt)) ? dt : best;
@@ -1456,7 +1609,7 @@ __global__ void __launch_bounds__(128) m5_tag_prims(int64_t n, M5Consts k,
   double s[C::NEQ];
   load_state<N>(S, n, c, s);
   Sol<N> q;
-  make_sol<N>(k, s, s, false, q);
+  make_sol<N>(k, s, 0.0, false, q);
   double p = 0.0;
 #pragma unroll
   for (int iv = 0; iv < N; ++iv) p += q.avf[iv] * q.p[iv];
@@ -1523,7 +1676,7 @@ __global__ void __launch_bounds__(128) m5_export_fields(int64_t n, M5Consts k,
   double s[C::NEQ];
   load_state<N>(S, n, c, s);
   Sol<N> q;
-  make_sol<N>(k, s, s, false, q);
+  make_sol<N>(k, s, 0.0, false, q);
   double p = 0.0;
 #pragma unroll
   for (int iv = 0; iv < N; ++iv) p += q.avf[iv] * q.p[iv];
@@ -1551,7 +1704,7 @@ __global__ void __launch_bounds__(128) m5_export_fields(int64_t n, M5Consts k,
 
 // merged cells of a mesh adaptation (map < 0): the reference's relaxation of the merged
 // state (merge.c:52-57)
-template <int N>
+template <int N, bool FAST>
 __global__ void __launch_bounds__(128) m5_relax_merged(int64_t n, M5Consts k,
                                                        const int64_t *__restrict__ map,
                                                        double *__restrict__ S) {
@@ -1560,7 +1713,7 @@ __global__ void __launch_bounds__(128) m5_relax_merged(int64_t n, M5Consts k,
   if (c >= n || map[c] >= 0) return;
   double s[C::NEQ];
   load_state<N>(S, n, c, s);
-  relaxationvec<N>(k, s);
+  relaxationvec<N, FAST>(k, s);
 #pragma unroll
   for (int e = 0; e < C::NEQ; e++) S[(int64_t)e * n + c] = s[e];
 }
@@ -1570,8 +1723,9 @@ __global__ void __launch_bounds__(128) m5_relax_merged(int64_t n, M5Consts k,
 void ffv_m5_relax_merged(int64_t n, const M5Consts &k, const int64_t *map, double *S,
                          cudaStream_t st) {
   const unsigned gc = (unsigned)((n + 127) / 128);
-  if (k.nmat == 2) m5_relax_merged<2><<<gc, 128, 0, st>>>(n, k, map, S);
-  else m5_relax_merged<3><<<gc, 128, 0, st>>>(n, k, map, S);
+  const bool fast = k.flux_form == FFV_FLUX_CONSISTENT;
+  if (k.nmat == 2) (fast ? m5_relax_merged<2, true> : m5_relax_merged<2, false>)<<<gc, 128, 0, st>>>(n, k, map, S);
+  else (fast ? m5_relax_merged<3, true> : m5_relax_merged<3, false>)<<<gc, 128, 0, st>>>(n, k, map, S);
 }
 
 void ffv_m5_export_fields(int64_t n, const M5Consts &k, const double *S, double *F,
@@ -1610,7 +1764,7 @@ void ffv_m5_cfl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const 
 int ffv_m5_neq(int nmat) { return 3 * nmat + 12; }
 
 // kernel names in launch order, for ffv_profile_stage
-static const char *k_names[] = {"m5_recon_face", "m5_face_flux",  "m5_cell_update",
+static const char *k_names[] = {"m5_recon_slopes", "m5_face_flux",  "m5_cell_update",
                                 "flag_count",    "flag_scan",     "flag_scatter",
                                 "m5_gfm_seq",    "m5_relax_cell", "flag_count",
                                 "flag_scan",     "flag_scatter",  "m5_gfm_seq(relax)"};
@@ -1637,7 +1791,7 @@ static void stage_impl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
   const unsigned nb = (unsigned)((m.n + CB - 1) / CB);
   Rec rec{ev, 0, names, st};
   if (ev) cudaEventRecord(ev[0], st);
-  const bool f32 = k.precision == FFV_FP32_FLUX;
+  const bool f32 = k.precision == FFV_FP32_FLUX, fast = k.flux_form == FFV_FLUX_CONSISTENT;
   // the FP32 form keeps its face states and fluxes in the same buffers, as floats
   float *SFf = (float *)b.SF, *FFf = (float *)b.FF, *UFf = (float *)b.UF;
   if (k.order == 2) {
@@ -1646,21 +1800,27 @@ static void stage_impl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
       ffv_m5f_shadow(m.n, k, b.S, (float *)b.RHS, st);
       rec("m5f_shadow");
       ffv_m5f_recon(m, g, k, b.S, (float *)b.RHS, SFf, b.status, st);
+      rec("m5f_recon_face");
     } else {
-      m5_recon_face<N><<<gf, tpb, 0, st>>>(m, g, k, b.S, b.SF, b.status);
+      m5_recon_slopes<N><<<dim3(gc, 3), tpb, 0, st>>>(m, g, k, b.S, b.SF);
+      rec(k_names[0]);
+      (fast ? m5_relax_faces<N, true> : m5_relax_faces<N, false>)<<<dim3(gc, 6), tpb, 0, st>>>(
+          m.n, k, b.SF, b.status);
+      rec("m5_relax_faces");
     }
-    rec(f32 ? "m5f_recon_face" : k_names[0]);
   }
   if (f32)
     ffv_m5f_flux(m, g, k, b.S, k.order == 2 ? (const float *)b.RHS : nullptr, SFf, FFf, UFf, b.GF,
                  b.status, st);
-  else m5_face_flux<N><<<gf, tpb, 0, st>>>(m, g, k, b.S, b.SF, b.FF, b.UF, b.GF, b.status);
+  else
+    (k.order == 2 ? m5_face_flux<N, 2> : m5_face_flux<N, 1>)<<<gf, tpb, 0, st>>>(
+        m, g, k, b.S, b.SF, b.FF, b.UF, b.GF, b.status);
   rec(f32 ? "m5f_face_flux" : k_names[1]);
   if (f32)
     ffv_m5f_cell_update(m, g, k, b.S, b.SN, FFf, UFf, b.RHS, b.Snew, b.flag, b.dt, irk, b.status,
                         st);
   else
-    m5_cell_update<N, double><<<gc, tpb, 0, st>>>(m, g, k, b.S, b.SN, b.FF, b.UF, b.RHS, b.Snew,
+    m5_cell_update<N><<<gc, tpb, 0, st>>>(m, g, k, b.S, b.SN, b.FF, b.UF, b.RHS, b.Snew,
                                                   b.flag, b.dt, irk, b.status);
   rec(f32 ? "m5f_cell_update" : k_names[2]);
   if (irk == 1) {
@@ -1675,7 +1835,9 @@ static void stage_impl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
     rec(k_names[6]);
   }
   if (f32) ffv_m5f_relax_cell(m.n, k, b.Snew, b.S, b.flag, b.status, st);
-  else m5_relax_cell<N><<<gc, tpb, 0, st>>>(m.n, k, b.Snew, b.S, b.flag, b.status);
+  else
+    (fast ? m5_relax_cell<N, true> : m5_relax_cell<N, false>)<<<gc, tpb, 0, st>>>(
+        m.n, k, b.Snew, b.S, b.flag, b.status);
   rec(f32 ? "m5f_relax_cell" : k_names[7]);
   flag_count<<<nb, CB, 0, st>>>(m.n, b.flag, b.bcount);
   rec(k_names[8]);
@@ -1697,6 +1859,6 @@ void ffv_m5_fp64_stage(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
 }
 
 int ffv_m5_launches_per_stage(const M5Consts &k, int irk) {
-  const int recon = k.order == 2 ? (k.precision == FFV_FP32_FLUX ? 2 : 1) : 0;
+  const int recon = k.order == 2 ? 2 : 0;
   return recon + 2 + (irk == 1 ? 4 : 0) + 1 + 4;
 }

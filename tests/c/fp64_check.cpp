@@ -47,6 +47,8 @@ static void two(double x, double y) {
   if (!std::isnan(y) && y != 0.0) {
     expect(f64::lt(x, y) == (x < y), "lt", x, y);
     expect(f64::le(x, y) == (x <= y), "le", x, y);
+    expect(f64::gt(x, y) == (x > y), "gt", x, y);
+    expect(f64::ge(x, y) == (x >= y), "ge", x, y);
   }
   expect(same(f64::div(x, f64::rcp(y)), x / y), "div", x, y);
 }
