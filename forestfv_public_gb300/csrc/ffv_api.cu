@@ -4,6 +4,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <array>
 #include <new>
 
 #include "ffv_device.cuh"
@@ -23,8 +24,13 @@ struct ffv_ctx {
   int32_t *d_nbr, *d_sub;
   double *d_S, *d_SN, *d_SF, *d_dt;
   // model 5 only
-  double *d_Snew, *d_FF, *d_UF, *d_GF, *d_RHS;
-  uint8_t *d_flag;
+  double *d_Snew, *d_FF, *d_UF, *d_RHS;
+  uint8_t *d_GF, *d_flag;
+  // the mesh's listed faces (ffv_face_list): n pairs' room behind GF (0.2 to 0.4 n are usual), a
+  // buffer of its own where a mesh has more
+  int32_t *d_flist, *d_flist_own;
+  int64_t cap_flist_own;
+  ffv_face_list flist;
   int32_t *d_list, *d_bcount, *d_count;
   M5Consts m5;
   // refinement tags
@@ -70,6 +76,9 @@ void free_mesh_buffers(ffv_ctx *c) {
   cudaFree(c->d_list);
   cudaFree(c->d_bcount);
   cudaFree(c->d_count);
+  cudaFree(c->d_flist_own);
+  c->d_flist = c->d_flist_own = nullptr;
+  c->cap_flist_own = 0;
   cudaFree(c->d_SI);
   cudaFree(c->d_SItmp);
   cudaFree(c->d_split);
@@ -79,8 +88,8 @@ void free_mesh_buffers(ffv_ctx *c) {
   c->d_info = nullptr;
   c->d_nbr = c->d_sub = nullptr;
   c->d_S = c->d_SN = c->d_SF = nullptr;
-  c->d_Snew = c->d_FF = c->d_UF = c->d_GF = c->d_RHS = nullptr;
-  c->d_flag = nullptr;
+  c->d_Snew = c->d_FF = c->d_UF = c->d_RHS = nullptr;
+  c->d_GF = c->d_flag = nullptr;
   c->d_list = c->d_bcount = c->d_count = nullptr;
   c->cap = c->cap_nsub = 0;
   if (c->graph_valid) cudaGraphExecDestroy(c->graph);
@@ -106,15 +115,16 @@ int alloc_mesh_buffers(ffv_ctx *c) {
     if (cudaMalloc(&c->d_Snew, sizeof(double) * c->neq * n) != cudaSuccess ||
         cudaMalloc(&c->d_FF, sizeof(double) * 6 * c->neq * n) != cudaSuccess ||
         cudaMalloc(&c->d_UF, sizeof(double) * 18 * n) != cudaSuccess ||
-        cudaMalloc(&c->d_GF, sizeof(double) * 6 * n) != cudaSuccess ||
+        cudaMalloc(&c->d_GF, (((6 * n + 3) & ~(int64_t)3) + 4 * n)) != cudaSuccess ||
         cudaMalloc(&c->d_RHS, sizeof(double) * c->neq * n) != cudaSuccess ||
         cudaMalloc(&c->d_flag, n) != cudaSuccess ||
         cudaMalloc(&c->d_list, sizeof(int32_t) * n) != cudaSuccess ||
         cudaMalloc(&c->d_bcount, sizeof(int32_t) * nb) != cudaSuccess ||
-        cudaMalloc(&c->d_count, sizeof(int32_t)) != cudaSuccess) {
+        cudaMalloc(&c->d_count, sizeof(int32_t) * 16) != cudaSuccess) {  // count, 12 cursors
       free_mesh_buffers(c);
       return FFV_ERR_NOMEM;
     }
+    c->d_flist = (int32_t *)(c->d_GF + ((6 * n + 3) & ~(int64_t)3));
   }
   return FFV_OK;
 }
@@ -139,8 +149,8 @@ int launch_stage(ffv_ctx *c, int irk, cudaEvent_t *ev = nullptr) {
   }
   if (c->p.model == 5) {
     ffv_m5_bufs mb{c->d_S,   c->d_SN,   c->d_Snew, c->d_SF,     c->d_FF,    c->d_UF,
-                   c->d_GF,  c->d_RHS,  c->d_dt,   c->d_flag,   c->d_list,  c->d_bcount,
-                   c->d_count, c->d_status};
+                   c->d_RHS, c->d_dt,   c->d_GF,   c->d_flag,   c->d_list,  c->d_bcount,
+                   c->d_count, c->d_status, c->flist};
     ffv_m5_fp64_stage(c->dm, c->geom, c->m5, mb, irk, c->stream, ev, c->knames);
     return cuda_rc(cudaGetLastError());
   }
@@ -169,6 +179,77 @@ int build_graph(ffv_ctx *c) {
   CK(e);
   c->graph_valid = 1;
   return FFV_OK;
+}
+
+// the group of a cell's face in the list of faces (ffv_face_list), -1 for a face shared with one
+// cell of the same level
+__device__ __forceinline__ int face_group(uint32_t info, int f) {
+  const uint32_t kind = ffv_face_kind(info, f);
+  return kind == FFV_FK_SAME ? -1 : 2 * f + (kind == FFV_FK_FINER ? 1 : 0);
+}
+
+// The list: a block reserves its pairs' places in each group with one atomic on the group's
+// cursor, so that a block's pairs stay together (the order of the blocks is not fixed; nothing
+// depends on it).
+__global__ void __launch_bounds__(256) list_faces(int64_t n, const uint32_t *__restrict__ info,
+                                                  int32_t *__restrict__ cursor,
+                                                  int32_t *__restrict__ cells) {
+  __shared__ int base[12], warp_at[12][8];
+  const int64_t c = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  const uint32_t in = c < n ? info[c] : 0u;  // past the end: no listed face
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned mask[12];
+#pragma unroll
+  for (int g = 0; g < 12; g++) {
+    mask[g] = __ballot_sync(0xffffffffu, face_group(in, g >> 1) == g);
+    if (lane == 0) warp_at[g][warp] = __popc(mask[g]);
+  }
+  __syncthreads();
+  if (threadIdx.x < 12) {
+    int t = 0;
+    for (int w = 0; w < 8; w++) {
+      const int x = warp_at[threadIdx.x][w];
+      warp_at[threadIdx.x][w] = t;
+      t += x;
+    }
+    base[threadIdx.x] = t ? atomicAdd(cursor + threadIdx.x, t) : 0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int g = 0; g < 12; g++)
+    if ((mask[g] >> lane) & 1u)
+      cells[base[g] + warp_at[g][warp] + __popc(mask[g] & ((1u << lane) - 1u))] = (int32_t)c;
+}
+
+// the list of a mesh with count[g] pairs per group, on the context's stream (after its info
+// words are on the device); the ghost-fluid flags of faces nothing evaluates stay zero
+int build_face_list(ffv_ctx *c, const int64_t count[12]) {
+  ffv_face_list &l = c->flist;
+  l.off[0] = l.block[0] = 0;
+  for (int g = 0; g < 12; g++) {
+    const int64_t threads = count[g] * ((g & 1) ? 4 : 1);
+    l.off[g + 1] = l.off[g] + (int32_t)count[g];
+    l.block[g + 1] = l.block[g] + (int32_t)((threads + FFV_LIST_TPB - 1) / FFV_LIST_TPB);
+  }
+  const int64_t total = l.off[12];
+  int32_t *cells = c->d_flist;
+  if (total > c->cap) {
+    if (total > c->cap_flist_own) {
+      cudaFree(c->d_flist_own);
+      c->d_flist_own = nullptr;
+      c->cap_flist_own = 0;
+      if (cudaMalloc(&c->d_flist_own, sizeof(int32_t) * (total + total / 4)) != cudaSuccess)
+        return FFV_ERR_NOMEM;
+      c->cap_flist_own = total + total / 4;
+    }
+    cells = c->d_flist_own;
+  }
+  l.cells = cells;
+  CK(cudaMemsetAsync(c->d_GF, 0, 6 * c->n, c->stream));
+  if (total == 0) return FFV_OK;
+  CK(cudaMemcpyAsync(c->d_count + 1, l.off, sizeof(int32_t) * 12, cudaMemcpyHostToDevice, c->stream));
+  list_faces<<<(unsigned)((c->n + 255) / 256), 256, 0, c->stream>>>(c->n, c->d_info, c->d_count + 1, cells);
+  return cuda_rc(cudaGetLastError());
 }
 
 // CFL: dt = cfl * min over cells of h / max_a(|u_a| + c)  (no reference counterpart:
@@ -474,10 +555,21 @@ int ffv_set_mesh(ffv_ctx *c, const ffv_mesh *m) {
     free_mesh_buffers(c);
     return FFV_ERR_NOMEM;
   }
-  parallel_chunks(n, host_threads(), [&](int, int64_t a, int64_t b) {
+  // (and the listed faces per group, for model 5)
+  std::vector<std::array<int64_t, 12>> part((size_t)host_threads());
+  parallel_chunks(n, host_threads(), [&](int t, int64_t a, int64_t b) {
+    std::array<int64_t, 12> k{};
     for (int64_t i = a; i < b; i++)
-      for (int f = 0; f < 6; f++) nbr_t[(int64_t)f * n + i] = m->nbr[6 * i + f];
+      for (int f = 0; f < 6; f++) {
+        nbr_t[(int64_t)f * n + i] = m->nbr[6 * i + f];
+        const uint32_t kind = ffv_face_kind(m->info[i], f);
+        if (kind != FFV_FK_SAME) k[2 * f + (kind == FFV_FK_FINER)]++;
+      }
+    part[t] = k;
   });
+  int64_t listed[12] = {};
+  for (const auto &k : part)
+    for (int g = 0; g < 12; g++) listed[g] += k[g];
   cudaError_t e = cudaMemcpy(c->d_info, m->info, sizeof(uint32_t) * n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaMemcpy(c->d_nbr, nbr_t, sizeof(int32_t) * 6 * n, cudaMemcpyHostToDevice);
@@ -491,6 +583,13 @@ int ffv_set_mesh(ffv_ctx *c, const ffv_mesh *m) {
   c->n = n;
   c->dm = ffv_dmesh{n, c->d_info, c->d_nbr, c->d_sub};
   ffv_fill_geom(m, &c->geom);
+  if (c->p.model == 5) {
+    rc = build_face_list(c, listed);
+    if (rc != FFV_OK) {
+      free_mesh_buffers(c);
+      return rc;
+    }
+  }
   c->have_mesh = 1;
   return FFV_OK;
 }

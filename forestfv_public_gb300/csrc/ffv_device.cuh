@@ -54,6 +54,39 @@ struct ffv_dmesh {
   const int32_t *__restrict__ sub;    // [4 nsub]
 };
 
+// The (cell, face) pairs of a mesh whose face is not shared with one cell of the same level --
+// boundary, coarser and finer faces -- grouped by face and by whether the neighbours are finer
+// (group 2 f + finer), each group padded to whole blocks of FFV_LIST_TPB threads, four threads per
+// pair in the finer groups.  A kernel over cells and faces would meet such pairs as single lanes of
+// a warp.
+#define FFV_LIST_TPB 128
+struct ffv_face_list {
+  const int32_t *cells;
+  int32_t off[13];    // group g: cells[off[g] .. off[g + 1])
+  int32_t block[13];  // its blocks of a launch over the whole list
+};
+
+// the face of this block of a launch over the list, and this thread's cell; live: it has one
+__device__ __forceinline__ int ffv_listed_face(const ffv_face_list &fl, int64_t &c, bool &live,
+                                               bool &finer) {
+  int g = 0;
+#pragma unroll
+  for (int i = 1; i < 12; i++)
+    if ((int)blockIdx.x >= fl.block[i]) g = i;
+  // (empty groups share their first block with the next group that has any)
+  finer = g & 1;
+  const int t = ((int)blockIdx.x - fl.block[g]) * FFV_LIST_TPB + (int)threadIdx.x;
+  const int at = fl.off[g] + (finer ? t >> 2 : t);
+  live = at < fl.off[g + 1];
+  c = live ? fl.cells[at] : 0;
+  return g >> 1;
+}
+
+// The faces towards a neighbour of the same level that comes later in leaf order.  The order is
+// a Morton order, in which a neighbour one step along an axis comes later than the cell and one
+// step back earlier, so these are the faces of the three positive sides.
+__host__ __device__ constexpr int owner_face(int axis) { return axis == 0 ? 2 : axis == 1 ? 1 : 5; }
+
 // host-side helpers implemented in ffv_api.cu
 int ffv_check_frames(const ffv_mesh *m);
 void ffv_fill_geom(const ffv_mesh *m, ffv_geom *g);

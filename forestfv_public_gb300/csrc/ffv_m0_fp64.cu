@@ -175,11 +175,6 @@ __device__ __forceinline__ void load_face(const double *__restrict__ FS, int64_t
     U[v] = ORDER == 2 ? FS[((int64_t)f * NV + v) * n + c] : FS[(int64_t)v * n + c];
 }
 
-// The faces towards a neighbour of the same level that comes later in leaf order.  The order is
-// a Morton order, in which a neighbour one step along an axis comes later than the cell and one
-// step back earlier, so these are the faces of the three positive sides.
-__host__ __device__ constexpr int owner_face(int axis) { return axis == 0 ? 2 : axis == 1 ? 1 : 5; }
-
 // The flux of the positive face of one axis (blockIdx.y) of every cell with a neighbour of its
 // own level there, into that face's slots of SF: five values over the cell's own face state,
 // which this thread alone reads (order 1: over slots that hold nothing).  About 190 FP64

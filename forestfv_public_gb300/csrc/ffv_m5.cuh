@@ -44,10 +44,12 @@ struct M5Consts {
 };
 
 struct ffv_m5_bufs {
-  double *S, *SN, *Snew, *SF, *FF, *UF, *GF, *RHS, *dt;
-  uint8_t *flag;
+  double *S, *SN, *Snew, *SF, *FF, *UF, *RHS, *dt;
+  uint8_t *GF, *flag;  // GF [6][n]: ghost-fluid faces, as the cell that evaluates the face sees them
+
   int32_t *list, *bcount, *count;
   unsigned int *status;
+  ffv_face_list list_faces;
 };
 
 int ffv_m5_neq(int nmat);
@@ -66,10 +68,14 @@ int ffv_m5_launches_per_stage(const M5Consts &k, int irk);
 void ffv_m5f_shadow(int64_t n, const M5Consts &k, const double *S, float *Sf, cudaStream_t st);
 void ffv_m5f_recon(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
                    const float *Sf, float *SFf, unsigned *status, cudaStream_t st);
+// the faces between cells of one level, and the listed others
 // Sf: the FP32 copy of the state (order 2), or nullptr (order 1: phi0 from S)
 void ffv_m5f_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
-                  const float *Sf, const float *SFf, float *FFf, float *UFf, double *GF,
+                  const float *Sf, const float *SFf, float *FFf, float *UFf, uint8_t *GF,
                   unsigned *status, cudaStream_t st);
+void ffv_m5f_listed_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
+                         const float *Sf, const float *SFf, float *FFf, float *UFf, uint8_t *GF,
+                         const ffv_face_list &fl, unsigned *status, cudaStream_t st);
 // residual + RK stage of the FP32-flux form (the face fluxes of all but the deformation
 // summed in FP64)
 void ffv_m5f_cell_update(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,

@@ -1114,11 +1114,15 @@ __device__ __forceinline__ void record_of_cell(const M5Consts &k, const double *
   write_record<N>(k, V, nullptr, U, 1);
 }
 
+// Flux of cell c through face F -- its only neighbour there (same level or coarser), boundary or
+// finer neighbour q -- into ff (area-weighted, from zero), the face velocity into un.  Returns
+// whether it is a ghost-fluid face.
 template <int N, int F>
-__device__ void face_flux_f(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
-                            const double *__restrict__ S, const float *__restrict__ Sf,
-                            const float *__restrict__ SF, int64_t c, uint32_t info, float *ff,
-                            float uf[3], double &gfm_face, unsigned &st, bool &owner) {
+__device__ __forceinline__ bool face_flux_f(const ffv_dmesh &m, const ffv_geom &g,
+                                            const M5Consts &k, const double *__restrict__ S,
+                                            const float *__restrict__ Sf,
+                                            const float *__restrict__ SF, int64_t c, uint32_t info,
+                                            int q, float *ff, float un[3], unsigned &st) {
   using C = K5<N>;
   using RL = RecL<N>;
   constexpr int FO = fr_opp(F);
@@ -1126,54 +1130,68 @@ __device__ void face_flux_f(const ffv_dmesh &m, const ffv_geom &g, const M5Const
   const int l = ffv_info_level(info);
 #pragma unroll
   for (int iv = 0; iv < C::NEQ; iv++) ff[iv] = 0.0f;
-  uf[0] = uf[1] = uf[2] = 0.0f;
-  gfm_face = 0.0;
-  if (kind == FFV_FK_SAME && m.nbr[(int64_t)F * m.n + c] < c) {
-    owner = false;  // evaluated by the neighbour (flux reuse, m5_residual.c:80-99)
-    return;
-  }
   float U[RL::SIZE];
   SolF<N> L, R;
   if (kind == (FFV_FK_BC | FFV_BC_SYMMETRY)) {  // the cell's own state (m5_hllc.c:59-63)
     record_of_cell<N>(k, S, m.n, c, U);
     make_sol_f<N>(k, U, 0.0f, L);
-    symmetry_acc_f<F, N>(L, k.flux_form == FFV_FLUX_CONSISTENT, g.area_f[l], ff, uf);
-    return;
+    symmetry_acc_f<F, N>(L, k.flux_form == FFV_FLUX_CONSISTENT, g.area_f[l], ff, un);
+    return false;
   }
   if (k.order == 2) load_record<N>(SF, m.n, F, c, U);
   else record_of_cell<N>(k, S, m.n, c, U);
   make_sol_f<N>(k, U, Sf ? cell_phi0_f<N>(k, Sf, m.n, c) : (float)cell_phi0<N>(k, S, m.n, c), L);
-  // one solver call site for the boundary (the ghost state) and the interior faces (the
-  // neighbour's record, or each of four finer neighbours' in turn; the face velocity is the
-  // last subface's divided by four, m5_residual.c:163-165)
-  const bool bnd = (kind & FFV_FK_BC) != 0;
-  const int bc = bnd ? (int)(kind & 7u) : 0;
-  const int nsub = kind == FFV_FK_FINER ? 4 : 1;
-  const float A = kind == FFV_FK_FINER ? g.area_f[l + 1] : g.area_f[l];
-  const int32_t *sg = kind == FFV_FK_FINER ? m.sub + 4 * (int64_t)m.nbr[(int64_t)F * m.n + c] : nullptr;
-  const float inv = 1.0f / (float)nsub;
-#pragma unroll 1
-  for (int q = 0; q < nsub; q++) {
-    if (bnd) {
-      ghost_f<F, N>(L, bc, R);
-    } else {
-      const int64_t o = sg ? sg[q] : m.nbr[(int64_t)F * m.n + c];
-      if (k.order == 2) load_record<N>(SF, m.n, FO, o, U);
-      else record_of_cell<N>(k, S, m.n, o, U);
-      make_sol_f<N>(k, U, Sf ? cell_phi0_f<N>(k, Sf, m.n, o) : (float)cell_phi0<N>(k, S, m.n, o), R);
-    }
-    const bool gfm = L.phi0 * R.phi0 < 0.0f;
-    if (gfm) gfm_face = 1.0;
-    float un[3];
-    st |= hllc_acc_f<F, N>(k, L, R, bc, gfm, A, ff, un);
-    uf[0] = un[0] * inv;
-    uf[1] = un[1] * inv;
-    uf[2] = un[2] * inv;
+  const int bc = (kind & FFV_FK_BC) ? (int)(kind & 7u) : 0;
+  if (bc) {
+    ghost_f<F, N>(L, bc, R);
+  } else {
+    int64_t o = m.nbr[(int64_t)F * m.n + c];
+    if (kind == FFV_FK_FINER) o = m.sub[4 * o + q];
+    if (k.order == 2) load_record<N>(SF, m.n, FO, o, U);
+    else record_of_cell<N>(k, S, m.n, o, U);
+    make_sol_f<N>(k, U, Sf ? cell_phi0_f<N>(k, Sf, m.n, o) : (float)cell_phi0<N>(k, S, m.n, o), R);
   }
+  const bool gfm = L.phi0 * R.phi0 < 0.0f;
+  st |= hllc_acc_f<F, N>(k, L, R, bc, gfm, g.area_f[kind == FFV_FK_FINER ? l + 1 : l], ff, un);
+  return gfm;
 }
 
-// 4 blocks of 128 threads per SM (128 registers instead of 164): 6 % faster despite a few
-// hundred bytes of spill
+template <int N>
+__device__ __forceinline__ void store_flux_f(int64_t n, int f, int64_t c, const float *ff,
+                                             const float un[3], bool gfm, float *__restrict__ FF,
+                                             float *__restrict__ UF, uint8_t *__restrict__ GF) {
+  using C = K5<N>;
+#pragma unroll
+  for (int iv = 0; iv < C::NEQ; iv++) FF[((int64_t)f * C::NEQ + iv) * n + c] = ff[iv];
+#pragma unroll
+  for (int d = 0; d < 3; d++) UF[((int64_t)f * 3 + d) * n + c] = un[d];
+  GF[(int64_t)f * n + c] = gfm ? 1 : 0;
+}
+
+template <int N, int F>
+__device__ __forceinline__ void owner_flux_f(const ffv_dmesh &m, const ffv_geom &g,
+                                             const M5Consts &k, const double *__restrict__ S,
+                                             const float *__restrict__ Sf,
+                                             const float *__restrict__ SF, float *__restrict__ FF,
+                                             float *__restrict__ UF, uint8_t *__restrict__ GF,
+                                             unsigned *status) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= m.n) return;
+  const uint32_t info = m.info[c];
+  // a 1:1 face is evaluated by its earlier cell (flux reuse, m5_residual.c:80-99)
+  if (ffv_face_kind(info, F) != FFV_FK_SAME || m.nbr[(int64_t)F * m.n + c] < c) return;
+  float ff[K5<N>::NEQ], un[3];
+  unsigned st = 0;
+  const bool gfm = face_flux_f<N, F>(m, g, k, S, Sf, SF, c, info, 0, ff, un, st);
+  store_flux_f<N>(m.n, F, c, ff, un, gfm, FF, UF, GF);
+  if (st) atomicOr(status, st);
+}
+
+// The faces between cells of one level, each once: the positive face of one axis (blockIdx.y).
+// Bound by memory latency at 4 blocks of 128 threads per SM (118 registers).  Without the loop over
+// finer neighbours the kernel needs no spills (it took ~900 bytes per thread), and the listed
+// faces no longer run as single lanes of its warps: together 34.8 -> 30.9 ms per step on the wall
+// mesh of 10.1 M cells, 6.66 -> 5.85 ms on the bubble mesh of 2.3 M.
 template <int N>
 __global__ void __launch_bounds__(128, 4) m5f_face_flux(ffv_dmesh m, ffv_geom g, M5Consts k,
                                                      const double *__restrict__ S,
@@ -1181,34 +1199,64 @@ __global__ void __launch_bounds__(128, 4) m5f_face_flux(ffv_dmesh m, ffv_geom g,
                                                      const float *__restrict__ SF,
                                                      float *__restrict__ FF,
                                                      float *__restrict__ UF,
-                                                     double *__restrict__ GF,
+                                                     uint8_t *__restrict__ GF,
                                                      unsigned *__restrict__ status) {
+  if (blockIdx.y == 0) owner_flux_f<N, owner_face(0)>(m, g, k, S, Sf, SF, FF, UF, GF, status);
+  else if (blockIdx.y == 1) owner_flux_f<N, owner_face(1)>(m, g, k, S, Sf, SF, FF, UF, GF, status);
+  else owner_flux_f<N, owner_face(2)>(m, g, k, S, Sf, SF, FF, UF, GF, status);
+}
+
+template <int N, int F>
+__device__ __forceinline__ void listed_flux_f(const ffv_dmesh &m, const ffv_geom &g,
+                                              const M5Consts &k, const double *__restrict__ S,
+                                              const float *__restrict__ Sf,
+                                              const float *__restrict__ SF, int64_t c, bool finer,
+                                              bool live, float *__restrict__ FF,
+                                              float *__restrict__ UF, uint8_t *__restrict__ GF,
+                                              unsigned *status) {
   using C = K5<N>;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 6 * m.n) return;
-  const int f = (int)(t / m.n);
-  const int64_t c = t - (int64_t)f * m.n;
-  const uint32_t info = m.info[c];
-  float ff[C::NEQ], uf[3];
-  double gf = 0.0;
+  const int q = finer ? (int)(threadIdx.x & 3) : 0;
+  float ff[C::NEQ], un[3] = {0.0f, 0.0f, 0.0f};
   unsigned st = 0;
-  bool owner = true;
-  switch (f) {
-    case 0: face_flux_f<N, 0>(m, g, k, S, Sf, SF, c, info, ff, uf, gf, st, owner); break;
-    case 1: face_flux_f<N, 1>(m, g, k, S, Sf, SF, c, info, ff, uf, gf, st, owner); break;
-    case 2: face_flux_f<N, 2>(m, g, k, S, Sf, SF, c, info, ff, uf, gf, st, owner); break;
-    case 3: face_flux_f<N, 3>(m, g, k, S, Sf, SF, c, info, ff, uf, gf, st, owner); break;
-    case 4: face_flux_f<N, 4>(m, g, k, S, Sf, SF, c, info, ff, uf, gf, st, owner); break;
-    default: face_flux_f<N, 5>(m, g, k, S, Sf, SF, c, info, ff, uf, gf, st, owner); break;
-  }
-  if (owner) {
+  bool gfm = false;
+  if (live) gfm = face_flux_f<N, F>(m, g, k, S, Sf, SF, c, m.info[c], q, ff, un, st);
+  if (finer) {
+    // four lanes hold the four subfaces: their sum in order, the last one's velocity divided by
+    // four (m5_residual.c:163-165)
+    const int first = (threadIdx.x & 31) & ~3;
 #pragma unroll
-    for (int iv = 0; iv < C::NEQ; iv++) FF[((int64_t)f * C::NEQ + iv) * m.n + c] = ff[iv];
+    for (int iv = 0; iv < C::NEQ; iv++) {
+      const float x = ff[iv];
+      float sum = __shfl_sync(0xffffffffu, x, first);
 #pragma unroll
-    for (int d = 0; d < 3; d++) UF[((int64_t)f * 3 + d) * m.n + c] = uf[d];
+      for (int j = 1; j < 4; j++) sum += __shfl_sync(0xffffffffu, x, first + j);
+      ff[iv] = sum;
+    }
+#pragma unroll
+    for (int d = 0; d < 3; d++) un[d] = __shfl_sync(0xffffffffu, un[d], first + 3) * 0.25f;
+    gfm = (__ballot_sync(0xffffffffu, gfm) >> first) & 15u;
   }
-  GF[(int64_t)f * m.n + c] = gf;
+  if (live && q == 0) store_flux_f<N>(m.n, F, c, ff, un, gfm, FF, UF, GF);
   if (st) atomicOr(status, st);
+}
+
+// the boundary, coarser and finer faces, from the mesh's list of them
+template <int N>
+__global__ void __launch_bounds__(FFV_LIST_TPB, 4) m5f_listed_flux(
+    ffv_dmesh m, ffv_geom g, M5Consts k, ffv_face_list fl, const double *__restrict__ S,
+    const float *__restrict__ Sf, const float *__restrict__ SF, float *__restrict__ FF,
+    float *__restrict__ UF, uint8_t *__restrict__ GF, unsigned *__restrict__ status) {
+  int64_t c;
+  bool live, finer;
+  const int f = ffv_listed_face(fl, c, live, finer);
+  switch (f) {
+    case 0: listed_flux_f<N, 0>(m, g, k, S, Sf, SF, c, finer, live, FF, UF, GF, status); break;
+    case 1: listed_flux_f<N, 1>(m, g, k, S, Sf, SF, c, finer, live, FF, UF, GF, status); break;
+    case 2: listed_flux_f<N, 2>(m, g, k, S, Sf, SF, c, finer, live, FF, UF, GF, status); break;
+    case 3: listed_flux_f<N, 3>(m, g, k, S, Sf, SF, c, finer, live, FF, UF, GF, status); break;
+    case 4: listed_flux_f<N, 4>(m, g, k, S, Sf, SF, c, finer, live, FF, UF, GF, status); break;
+    default: listed_flux_f<N, 5>(m, g, k, S, Sf, SF, c, finer, live, FF, UF, GF, status); break;
+  }
 }
 
 // ZEROU masks and positivity (m5_RK.c), as the FP64 form's clamp_zerou
@@ -1525,12 +1573,21 @@ void ffv_m5f_recon(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, con
 }
 
 void ffv_m5f_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
-                  const float *Sf, const float *SFf, float *FFf, float *UFf, double *GF,
-                  unsigned *status,
-                  cudaStream_t st) {
-  const unsigned blocks = (unsigned)((6 * m.n + 127) / 128);
+                  const float *Sf, const float *SFf, float *FFf, float *UFf, uint8_t *GF,
+                  unsigned *status, cudaStream_t st) {
+  const dim3 blocks((unsigned)((m.n + 127) / 128), 3);
   if (k.nmat == 2) m5f_face_flux<2><<<blocks, 128, 0, st>>>(m, g, k, S, Sf, SFf, FFf, UFf, GF, status);
   else m5f_face_flux<3><<<blocks, 128, 0, st>>>(m, g, k, S, Sf, SFf, FFf, UFf, GF, status);
+}
+
+void ffv_m5f_listed_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
+                         const float *Sf, const float *SFf, float *FFf, float *UFf, uint8_t *GF,
+                         const ffv_face_list &fl, unsigned *status, cudaStream_t st) {
+  const unsigned blocks = (unsigned)fl.block[12];
+  if (k.nmat == 2)
+    m5f_listed_flux<2><<<blocks, FFV_LIST_TPB, 0, st>>>(m, g, k, fl, S, Sf, SFf, FFf, UFf, GF, status);
+  else
+    m5f_listed_flux<3><<<blocks, FFV_LIST_TPB, 0, st>>>(m, g, k, fl, S, Sf, SFf, FFf, UFf, GF, status);
 }
 
 void ffv_m5f_cell_update(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,

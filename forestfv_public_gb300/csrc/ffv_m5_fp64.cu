@@ -945,14 +945,13 @@ __device__ __forceinline__ void load_face_state(const double *__restrict__ SF, i
   for (int v = 0; v < K5<N>::NEQ; v++) U[v] = SF[((int64_t)f * K5<N>::NEQ + v) * n + c];
 }
 
-// Face flux of cell c through face F (all subfaces), the reference's reuse included.  FP64 pipe
-// 79 % busy; wall mesh (0.41 M cells) 6.2 -> 3.6 ms per stage, bubble mesh (51,584 cells) 0.90 ->
-// 0.40 ms by one solver evaluation per warp, shared reciprocals and the fluid states' zero terms.
+// Flux of cell c through face F -- its only neighbour there (same level or coarser), boundary or
+// finer neighbour q -- into ff (area-weighted, from zero), the face velocity into un.  Returns
+// whether it is a ghost-fluid face.
 template <int N, int ORDER, int F>
-__device__ void face_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
+__device__ bool face_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
                           const double *__restrict__ S, const double *__restrict__ SF, int64_t c,
-                          uint32_t info, double *ff, double uf[3], double &gfm_face,
-                          unsigned &st, bool &owner) {
+                          uint32_t info, int q, double *ff, double un[3], unsigned &st) {
   using C = K5<N>;
   constexpr int FO = fr_opp(F);
   const uint32_t kind = ffv_face_kind(info, F);
@@ -960,15 +959,6 @@ __device__ void face_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts 
   double U[C::NEQ];
 #pragma unroll
   for (int iv = 0; iv < C::NEQ; iv++) ff[iv] = 0.0;
-  uf[0] = uf[1] = uf[2] = 0.0;
-  gfm_face = 0.0;
-  if (kind == FFV_FK_SAME && m.nbr[(int64_t)F * m.n + c] < c) {
-    // 1:1 face whose neighbour comes first in leaf order: the neighbour's thread evaluates
-    // it (face F^1 of the neighbour) and m5_cell_update takes the negative, as the
-    // reference's flux reuse does (m5_residual.c:80-99); no ghost-fluid flag here
-    owner = false;
-    return;
-  }
   const auto phi_at = [&](int64_t o) {
     return phi0_of<N>(k, S[(int64_t)C::i3 * m.n + o], N > 2 ? S[(int64_t)(C::i3 + 1) * m.n + o] : 0.0);
   };
@@ -978,72 +968,130 @@ __device__ void face_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts 
     // for this face is discarded (m5_hllc.c:59-63)
     load_state<N>(S, m.n, c, U);
     make_sol<N>(k, U, 0.0, false, L);
-    symmetry_acc<F, N>(L, k.flux_form == FFV_FLUX_CONSISTENT, g.area[l], ff, uf);
-    return;
+    symmetry_acc<F, N>(L, k.flux_form == FFV_FLUX_CONSISTENT, g.area[l], ff, un);
+    return false;
   }
   if (ORDER == 2) load_face_state<N>(SF, m.n, F, c, U);
   else load_state<N>(S, m.n, c, U);
   make_sol<N>(k, U, phi_at(c), ORDER == 2, L);
-  // one solver call site for the boundary (the ghost state) and the interior faces (the
-  // neighbour's state, or each of four finer neighbours' in turn)
   const int bc = (kind & FFV_FK_BC) ? (int)(kind & 7u) : 0;
-  const int nsub = kind == FFV_FK_FINER ? 4 : 1;
-  const double A = kind == FFV_FK_FINER ? g.area[l + 1] : g.area[l];
-  const double share = kind == FFV_FK_FINER ? 0.25 : 1.0;
-  const int32_t *sg = kind == FFV_FK_FINER ? m.sub + 4 * (int64_t)m.nbr[(int64_t)F * m.n + c] : nullptr;
-#pragma unroll 1
-  for (int q = 0; q < nsub; q++) {
-    if (bc) {
-      ghost<F, N>(L, bc, R);
-    } else {
-      const int64_t o = sg ? sg[q] : m.nbr[(int64_t)F * m.n + c];
-      if (ORDER == 2) load_face_state<N>(SF, m.n, FO, o, U);
-      else load_state<N>(S, m.n, o, U);
-      make_sol<N>(k, U, phi_at(o), ORDER == 2, R);
-    }
-    const bool gfm = (f64::gt0(L.phi0) && f64::lt0(R.phi0)) || (f64::lt0(L.phi0) && f64::gt0(R.phi0));
-    if (gfm) gfm_face = 1.0;
-    double un[3];
-    st |= hllc_acc<F, N>(k, L, R, bc, gfm, A, ff, un);
-    uf[0] = un[0] * share;
-    uf[1] = un[1] * share;
-    uf[2] = un[2] * share;
+  if (bc) {
+    ghost<F, N>(L, bc, R);
+  } else {
+    int64_t o = m.nbr[(int64_t)F * m.n + c];
+    if (kind == FFV_FK_FINER) o = m.sub[4 * o + q];
+    if (ORDER == 2) load_face_state<N>(SF, m.n, FO, o, U);
+    else load_state<N>(S, m.n, o, U);
+    make_sol<N>(k, U, phi_at(o), ORDER == 2, R);
   }
+  const bool gfm = (f64::gt0(L.phi0) && f64::lt0(R.phi0)) || (f64::lt0(L.phi0) && f64::gt0(R.phi0));
+  st |= hllc_acc<F, N>(k, L, R, bc, gfm, g.area[kind == FFV_FK_FINER ? l + 1 : l], ff, un);
+  return gfm;
 }
 
+template <int N>
+__device__ __forceinline__ void store_flux(int64_t n, int f, int64_t c, const double *ff,
+                                           const double un[3], bool gfm, double *__restrict__ FF,
+                                           double *__restrict__ UF, uint8_t *__restrict__ GF) {
+  using C = K5<N>;
+#pragma unroll
+  for (int iv = 0; iv < C::NEQ; iv++) FF[((int64_t)f * C::NEQ + iv) * n + c] = ff[iv];
+#pragma unroll
+  for (int d = 0; d < 3; d++) UF[((int64_t)f * 3 + d) * n + c] = un[d];
+  GF[(int64_t)f * n + c] = gfm ? 1 : 0;
+}
+
+template <int N, int ORDER, int F>
+__device__ __forceinline__ void owner_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
+                                           const double *__restrict__ S,
+                                           const double *__restrict__ SF, double *__restrict__ FF,
+                                           double *__restrict__ UF, uint8_t *__restrict__ GF,
+                                           unsigned *status) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= m.n) return;
+  const uint32_t info = m.info[c];
+  // a 1:1 face is evaluated by its earlier cell, and m5_cell_update takes the negative for the
+  // other, as the reference's flux reuse does (m5_residual.c:80-99)
+  if (ffv_face_kind(info, F) != FFV_FK_SAME || m.nbr[(int64_t)F * m.n + c] < c) return;
+  double ff[K5<N>::NEQ], un[3];
+  unsigned st = 0;
+  const bool gfm = face_flux<N, ORDER, F>(m, g, k, S, SF, c, info, 0, ff, un, st);
+  store_flux<N>(m.n, F, c, ff, un, gfm, FF, UF, GF);
+  if (st) atomicOr(status, st);
+}
+
+// The faces between cells of one level, each once: the positive face of one axis (blockIdx.y).
+// FP64 pipe ~80 % busy; with the listed faces below 40.1 -> 19.5 ms per step on the wall mesh of
+// 0.41 M cells (21.3 before the list), 5.87 -> 3.83 ms on the bubble mesh of 51,584 (4.30).
 template <int N, int ORDER>
 __global__ void __launch_bounds__(128) m5_face_flux(ffv_dmesh m, ffv_geom g, M5Consts k,
                                                     const double *__restrict__ S,
                                                     const double *__restrict__ SF,
                                                     double *__restrict__ FF,
                                                     double *__restrict__ UF,
-                                                    double *__restrict__ GF,
+                                                    uint8_t *__restrict__ GF,
                                                     unsigned *__restrict__ status) {
+  if (blockIdx.y == 0) owner_flux<N, ORDER, owner_face(0)>(m, g, k, S, SF, FF, UF, GF, status);
+  else if (blockIdx.y == 1) owner_flux<N, ORDER, owner_face(1)>(m, g, k, S, SF, FF, UF, GF, status);
+  else owner_flux<N, ORDER, owner_face(2)>(m, g, k, S, SF, FF, UF, GF, status);
+}
+
+template <int N, int ORDER, int F>
+__device__ __forceinline__ void listed_flux(const ffv_dmesh &m, const ffv_geom &g,
+                                            const M5Consts &k, const double *__restrict__ S,
+                                            const double *__restrict__ SF, int64_t c, bool finer,
+                                            bool live, double *__restrict__ FF,
+                                            double *__restrict__ UF, uint8_t *__restrict__ GF,
+                                            unsigned *status) {
   using C = K5<N>;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 6 * m.n) return;
-  const int f = (int)(t / m.n);
-  const int64_t c = t - (int64_t)f * m.n;
-  const uint32_t info = m.info[c];
-  double ff[C::NEQ], uf[3], gf = 0.0;
+  const int q = finer ? (int)(threadIdx.x & 3) : 0;
+  double ff[C::NEQ], un[3] = {0.0, 0.0, 0.0};
   unsigned st = 0;
-  bool owner = true;
-  switch (f) {
-    case 0: face_flux<N, ORDER, 0>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
-    case 1: face_flux<N, ORDER, 1>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
-    case 2: face_flux<N, ORDER, 2>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
-    case 3: face_flux<N, ORDER, 3>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
-    case 4: face_flux<N, ORDER, 4>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
-    default: face_flux<N, ORDER, 5>(m, g, k, S, SF, c, info, ff, uf, gf, st, owner); break;
-  }
-  if (owner) {
+  bool gfm = false;
+  if (live) gfm = face_flux<N, ORDER, F>(m, g, k, S, SF, c, m.info[c], q, ff, un, st);
+  if (finer) {
+    // four lanes hold the four subfaces: their sum in order, the last one's velocity divided by
+    // four (m5_residual.c:163-165)
+    const int first = (threadIdx.x & 31) & ~3;
 #pragma unroll
-    for (int iv = 0; iv < C::NEQ; iv++) FF[((int64_t)f * C::NEQ + iv) * m.n + c] = ff[iv];
+    for (int iv = 0; iv < C::NEQ; iv++) {
+      const double x = ff[iv];
+      double sum = __shfl_sync(0xffffffffu, x, first);
 #pragma unroll
-    for (int d = 0; d < 3; d++) UF[((int64_t)f * 3 + d) * m.n + c] = uf[d];
+      for (int j = 1; j < 4; j++) sum += __shfl_sync(0xffffffffu, x, first + j);
+      ff[iv] = sum;
+    }
+#pragma unroll
+    for (int d = 0; d < 3; d++) un[d] = __shfl_sync(0xffffffffu, un[d], first + 3) * 0.25;
+    gfm = (__ballot_sync(0xffffffffu, gfm) >> first) & 15u;
   }
-  GF[(int64_t)f * m.n + c] = gf;
+  if (live && q == 0) store_flux<N>(m.n, F, c, ff, un, gfm, FF, UF, GF);
   if (st) atomicOr(status, st);
+}
+
+// The boundary, coarser and finer faces, from the mesh's list of them: on a refined mesh they are
+// 0.2 to 0.3 per cell, and as single lanes of the warps over all cells and faces they took a third
+// to a half of the kernel.
+template <int N, int ORDER>
+__global__ void __launch_bounds__(FFV_LIST_TPB) m5_listed_flux(ffv_dmesh m, ffv_geom g, M5Consts k,
+                                                               ffv_face_list fl,
+                                                               const double *__restrict__ S,
+                                                               const double *__restrict__ SF,
+                                                               double *__restrict__ FF,
+                                                               double *__restrict__ UF,
+                                                               uint8_t *__restrict__ GF,
+                                                               unsigned *__restrict__ status) {
+  int64_t c;
+  bool live, finer;
+  const int f = ffv_listed_face(fl, c, live, finer);
+  switch (f) {
+    case 0: listed_flux<N, ORDER, 0>(m, g, k, S, SF, c, finer, live, FF, UF, GF, status); break;
+    case 1: listed_flux<N, ORDER, 1>(m, g, k, S, SF, c, finer, live, FF, UF, GF, status); break;
+    case 2: listed_flux<N, ORDER, 2>(m, g, k, S, SF, c, finer, live, FF, UF, GF, status); break;
+    case 3: listed_flux<N, ORDER, 3>(m, g, k, S, SF, c, finer, live, FF, UF, GF, status); break;
+    case 4: listed_flux<N, ORDER, 4>(m, g, k, S, SF, c, finer, live, FF, UF, GF, status); break;
+    default: listed_flux<N, ORDER, 5>(m, g, k, S, SF, c, finer, live, FF, UF, GF, status); break;
+  }
 }
 
 // Residual sum and non-conservative terms (m5_residual.c:171-214) for face F.  The reference
@@ -1239,7 +1287,7 @@ __global__ void __launch_bounds__(32) m5_gfm_seq(ffv_dmesh m, ffv_geom g, M5Cons
                                                  double *__restrict__ Snew,
                                                  const double *__restrict__ SN,
                                                  const double *__restrict__ RHS,
-                                                 const double *__restrict__ GF,
+                                                 const uint8_t *__restrict__ GF,
                                                  const double *__restrict__ dtp, int relax) {
   using C = K5<N>;
   __shared__ double s_phiR[6], s_vel[6][3], s_own[C::NEQ];
@@ -1262,7 +1310,7 @@ __global__ void __launch_bounds__(32) m5_gfm_seq(ffv_dmesh m, ffv_geom g, M5Cons
       const int f = lane;
       const uint32_t kind = ffv_face_kind(info, f);
       double phiR = 0.0, vr[3] = {0.0, 0.0, 0.0};
-      if (GF[(int64_t)f * m.n + c] == 1.0) {
+      if (GF[(int64_t)f * m.n + c]) {
         Sol<N> R;
         if (kind & FFV_FK_BC) {
           const int bc = (int)(kind & 7u);
@@ -1318,7 +1366,7 @@ __global__ void __launch_bounds__(32) m5_gfm_seq(ffv_dmesh m, ffv_geom g, M5Cons
       double nxi = 0.0, nyi = 0.0, nzi = 0.0, total = 0.0, ug[6], vg[6], wg[6];
       int nint = 0;
       for (int f = 0; f < 6; f++) {
-        if (GF[(int64_t)f * m.n + c] == 1.0) {
+        if (GF[(int64_t)f * m.n + c]) {
           const double phi = (L.phi0 + s_phiR[f]) / 2.0;
           const double A = g.area[ffv_face_kind(info, f) == FFV_FK_FINER ? l + 1 : l];
           const int ax = fr_n_axis(f), sg = fr_n_sign(f);
@@ -1361,7 +1409,7 @@ __global__ void __launch_bounds__(32) m5_gfm_seq(ffv_dmesh m, ffv_geom g, M5Cons
         double vnl = 0.0, wnl = 0.0;
         int ft = 0;
         for (int f = 0; f < 6; f++) {
-          if (GF[(int64_t)f * m.n + c] == 1.0) {
+          if (GF[(int64_t)f * m.n + c]) {
             const double A = g.area[ffv_face_kind(info, f) == FFV_FK_FINER ? l + 1 : l];
             const double vl = ug[ft] * n1x + vg[ft] * n1y + wg[ft] * n1z;
             const double wl = ug[ft] * n2x + vg[ft] * n2y + wg[ft] * n2z;
@@ -1787,7 +1835,7 @@ static void stage_impl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
                        const ffv_m5_bufs &b, int irk, cudaStream_t st, cudaEvent_t *ev,
                        const char **names) {
   const int tpb = 128;
-  const unsigned gf = (unsigned)((6 * m.n + tpb - 1) / tpb), gc = (unsigned)((m.n + tpb - 1) / tpb);
+  const unsigned gc = (unsigned)((m.n + tpb - 1) / tpb);
   const unsigned nb = (unsigned)((m.n + CB - 1) / CB);
   Rec rec{ev, 0, names, st};
   if (ev) cudaEventRecord(ev[0], st);
@@ -1813,9 +1861,19 @@ static void stage_impl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
     ffv_m5f_flux(m, g, k, b.S, k.order == 2 ? (const float *)b.RHS : nullptr, SFf, FFf, UFf, b.GF,
                  b.status, st);
   else
-    (k.order == 2 ? m5_face_flux<N, 2> : m5_face_flux<N, 1>)<<<gf, tpb, 0, st>>>(
+    (k.order == 2 ? m5_face_flux<N, 2> : m5_face_flux<N, 1>)<<<dim3(gc, 3), tpb, 0, st>>>(
         m, g, k, b.S, b.SF, b.FF, b.UF, b.GF, b.status);
   rec(f32 ? "m5f_face_flux" : k_names[1]);
+  if (b.list_faces.block[12] > 0) {
+    if (f32)
+      ffv_m5f_listed_flux(m, g, k, b.S, k.order == 2 ? (const float *)b.RHS : nullptr, SFf, FFf, UFf,
+                          b.GF, b.list_faces, b.status, st);
+    else
+      (k.order == 2 ? m5_listed_flux<N, 2> : m5_listed_flux<N, 1>)
+          <<<b.list_faces.block[12], FFV_LIST_TPB, 0, st>>>(m, g, k, b.list_faces, b.S, b.SF, b.FF,
+                                                            b.UF, b.GF, b.status);
+  }
+  rec(f32 ? "m5f_listed_flux" : "m5_listed_flux");
   if (f32)
     ffv_m5f_cell_update(m, g, k, b.S, b.SN, FFf, UFf, b.RHS, b.Snew, b.flag, b.dt, irk, b.status,
                         st);
@@ -1860,5 +1918,5 @@ void ffv_m5_fp64_stage(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
 
 int ffv_m5_launches_per_stage(const M5Consts &k, int irk) {
   const int recon = k.order == 2 ? 2 : 0;
-  return recon + 2 + (irk == 1 ? 4 : 0) + 1 + 4;
+  return recon + 3 + (irk == 1 ? 4 : 0) + 1 + 4;
 }

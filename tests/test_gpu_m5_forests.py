@@ -13,6 +13,7 @@ from oracle import pyoracle
 pytestmark = pytest.mark.gpu
 
 CASES = {"one_cell": ((1, 1, 1), 1, 1.0), "row": ((7, 1, 1), 1, 0.125), "three_quarters": ((3, 2, 2), 2, 0.75),
+         "long_row": ((3000, 1, 1), 1, 0.125),  # more boundary faces than cells
          "hanging": None}
 
 
