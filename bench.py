@@ -229,16 +229,16 @@ def wall_tags(lmax: int) -> tuple:
 def m5_alg_bytes(neq: int, nmat: int) -> dict:
     """Algorithmic bytes per cell of each model-5 kernel (compulsory traffic, neighbour
     re-reads excluded).  FP32 form: the FP32 shadow state (4 neq), the 2 N critical slots in
-    FP64, face records of neq + N + 1 FP32 values."""
+    FP64, face records of neq + 2 FP32 values."""
     d = 8 * neq
-    rec = 4 * (neq + nmat + 1)
+    rec = 4 * (neq + 2)
     return {"m5_recon_slopes": d + 28 + 6 * d,
             "m5_relax_faces": 6 * d + 6 * 8 * (2 * nmat + 8),
-            "m5_face_flux": 6 * d + d + 28 + 6 * d + 6 * 3 * 8 + 6 * 8,
+            "m5_face_flux": 6 * d + d + 28 + 6 * d + 6 * 3 * 8 + 6,
             "m5_cell_update": d + 6 * d + 6 * 3 * 8 + d + 28 + d + d + 1,
             "m5_relax_cell": d + d + 1,
             "m5f_recon_face": 4 * neq + 8 * 2 * nmat + 28 + 6 * rec,
-            "m5f_face_flux": 6 * rec + 8 * 2 * nmat + 28 + 6 * 4 * neq + 6 * 3 * 4 + 6 * 8,
+            "m5f_face_flux": 6 * rec + 8 * 2 * nmat + 28 + 6 * 4 * neq + 6 * 3 * 4 + 6,
             "m5f_cell_update": d + 6 * 4 * neq + 6 * 3 * 4 + d + 28 + d + d + 1,
             "m5f_relax_cell": d + d + 1}
 

@@ -62,8 +62,8 @@ int ffv_m5_launches_per_stage(const M5Consts &k, int irk);
 
 // FP32-flux form (ffv_m5_fp32.cu): face states and face fluxes in FP32.
 //   Sf:  [neq][n] float copy of the state, made by ffv_m5f_shadow (scratch)
-//   SFf: [6][neq + nmat + 1][n] float -- the reconstructed, relaxed face state followed by
-//        each material's pressure, recovered in FP64, and the last volume fraction
+//   SFf: [6][neq + 2][n] float -- the reconstructed, relaxed face state followed by the last
+//        volume fraction and the relaxed pressure
 //   FFf: [6][neq][n] float face fluxes (area-weighted), UFf: [6][3][n] float face velocity
 void ffv_m5f_shadow(int64_t n, const M5Consts &k, const double *S, float *Sf, cudaStream_t st);
 void ffv_m5f_recon(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,

@@ -39,10 +39,11 @@
 
 namespace {
 
-// face record: [neq conserved | nmat pressures | last volume fraction]
+// face record: [neq conserved | last volume fraction | nmat pressures]; in memory one pressure, the
+// relaxed state's, which all materials share
 template <int N>
 struct RecL {
-  static constexpr int NEQ = K5<N>::NEQ, P = NEQ, AL = NEQ + N, SIZE = NEQ + N + 1;
+  static constexpr int NEQ = K5<N>::NEQ, AL = NEQ, P = NEQ + 1, SIZE = NEQ + 1 + N, STORED = NEQ + 2;
 };
 
 // ------------------------------------------------------------------ EOS in FP32
@@ -660,53 +661,84 @@ __device__ __forceinline__ void crit_load(const float *__restrict__ Sf, const fl
   for (int j = 0; j < 2 * N; j++) X[j] = df{Sf[(int64_t)crit_slot<N>(j) * n + o], Sflo[(int64_t)j * n + o]};
 }
 
+// Whether some volume fraction of avf[0..N-2] may lie outside [lo, top], by the high parts alone:
+// where none does, the clamps of the limits below change nothing (bounds inside the interval
+// are taken as outside).  The fractions of most states are far from the bounds (1e-8 and 1 - 1e-8
+// beside a floor of 1e-6), and a comparison of pairs takes four instructions.
+template <int N>
+__device__ __forceinline__ bool vf_near_bounds(const df *avf, df lo, df top) {
+  bool out = false;
+#pragma unroll
+  for (int j = 0; j < N - 1; ++j) out |= !(avf[j].hi > lo.hi && avf[j].hi < top.hi);
+  return out;
+}
+
+template <int N>
+__device__ __forceinline__ df vf_sum(const df *avf) {
+  df sum = avf[0];
+#pragma unroll
+  for (int j = 1; j < N - 1; ++j) sum = df_add(sum, avf[j]);
+  return sum;
+}
+
+// the fractions scaled so that their sum is the upper bound
+template <int N>
+__device__ __forceinline__ void vf_scale_df(const M5Consts &k, df *avf, df sum) {
+  const df dif = df_sub(sum, k.ahi_d);
+#pragma unroll
+  for (int j = 0; j < N - 1; ++j) avf[j] = df_sub(avf[j], df_mul(df_div(avf[j], sum), dif));
+}
+
 // avf_limit.c:3-21 on the double-float volume fractions X[0..N-2]
 template <int N>
 __device__ __forceinline__ void avf_limit_df(const M5Consts &k, df *X) {
-  df sum = df_make(0.0f);
+  if (vf_near_bounds<N>(X, k.alo_d, k.ahi_d)) {
 #pragma unroll
-  for (int j = 0; j < N - 1; ++j) {
-    df a = X[j];
-    if (df_le(a, k.alo_d)) a = k.alo_d;
-    else if (df_le(k.ahi_d, a)) a = k.ahi_d;
-    X[j] = a;
-    sum = df_add(sum, a);
+    for (int j = 0; j < N - 1; ++j) {
+      if (df_le(X[j], k.alo_d)) X[j] = k.alo_d;
+      else if (df_le(k.ahi_d, X[j])) X[j] = k.ahi_d;
+    }
   }
-  if (df_lt(k.ahi_d, sum)) {
-    const df dif = df_sub(sum, k.ahi_d);
-#pragma unroll
-    for (int j = 0; j < N - 1; ++j) X[j] = df_sub(X[j], df_mul(df_div(X[j], sum), dif));
-  }
+  const df sum = vf_sum<N>(X);
+  if (df_lt(k.ahi_d, sum)) vf_scale_df<N>(k, X, sum);
 }
 
-// the critical slots across face f (neighbour, mean of four finer, or the cell itself at
-// a boundary), volume fractions limited as avf_limit does: their slopes are differences of
-// nearly equal numbers (a liquid fraction 1 - 1e-6, an energy of 1e9), which the FP32 copy
-// alone cannot resolve
+// the slots whose slope needs more than FP32: the volume fractions and the total energy (the
+// internal energies keep the cell's value at its faces)
 template <int N>
-__device__ void crit_across_df(const M5Consts &k, const ffv_dmesh &m, const float *__restrict__ Sf,
-                               const float *__restrict__ Sflo, int64_t c, int f, uint32_t kind,
-                               const df *own, df *X) {
-  constexpr int NCR = 2 * N;
+__device__ __forceinline__ constexpr int steep_slot(int j) { return j < N - 1 ? j : 2 * N - 1; }
+
+// those slots across face f (neighbour, mean of four finer, or the cell itself at a boundary),
+// volume fractions limited as avf_limit does: their slopes are differences of nearly equal numbers
+// (a liquid fraction 1 - 1e-6, an energy of 1e9), which the FP32 copy alone cannot resolve
+template <int N>
+__device__ void steep_across_df(const M5Consts &k, const ffv_dmesh &m, const float *__restrict__ Sf,
+                                const float *__restrict__ Sflo, int64_t c, int f, uint32_t kind,
+                                const df *own, df *X) {
+  const auto load = [&](int64_t o, df *Y) {
+#pragma unroll
+    for (int j = 0; j < N; j++)
+      Y[j] = df{Sf[(int64_t)crit_slot<N>(steep_slot<N>(j)) * m.n + o], Sflo[(int64_t)steep_slot<N>(j) * m.n + o]};
+  };
   if (kind & FFV_FK_BC) {
 #pragma unroll
-    for (int j = 0; j < NCR; j++) X[j] = own[j];
+    for (int j = 0; j < N; j++) X[j] = own[steep_slot<N>(j)];
     return;
   }
   if (kind == FFV_FK_FINER) {
     const int32_t *sg = m.sub + 4 * (int64_t)m.nbr[(int64_t)f * m.n + c];
-    crit_load<N>(Sf, Sflo, m.n, sg[0], X);
+    load(sg[0], X);
 #pragma unroll 1
     for (int q = 1; q < 4; q++) {
-      df Y[NCR];
-      crit_load<N>(Sf, Sflo, m.n, sg[q], Y);
+      df Y[N];
+      load(sg[q], Y);
 #pragma unroll
-      for (int j = 0; j < NCR; j++) X[j] = df_add(X[j], Y[j]);
+      for (int j = 0; j < N; j++) X[j] = df_add(X[j], Y[j]);
     }
 #pragma unroll
-    for (int j = 0; j < NCR; j++) X[j] = df{X[j].hi * 0.25f, X[j].lo * 0.25f};
+    for (int j = 0; j < N; j++) X[j] = df{X[j].hi * 0.25f, X[j].lo * 0.25f};
   } else {
-    crit_load<N>(Sf, Sflo, m.n, m.nbr[(int64_t)f * m.n + c], X);
+    load(m.nbr[(int64_t)f * m.n + c], X);
   }
   avf_limit_df<N>(k, X);
 }
@@ -716,22 +748,21 @@ __device__ void crit_across_df(const M5Consts &k, const ffv_dmesh &m, const floa
 // their sum reaches 1 - lo, the last fraction 1 - sum
 template <int N>
 __device__ __forceinline__ void vf_limit_relax_df(const M5Consts &k, df *avf, bool elseif) {
-  df sum = df_make(0.0f);
+  if (vf_near_bounds<N>(avf, k.alo_d, k.ahi_d)) {
 #pragma unroll
-  for (int i = 0; i < N - 1; ++i) {
-    if (elseif) {
-      if (df_le(avf[i], k.alo_d)) avf[i] = k.alo_d;
-      else if (df_le(k.ahi_d, avf[i])) avf[i] = k.ahi_d;
-    } else {
-      if (df_le(avf[i], k.alo_d)) avf[i] = k.alo_d;
-      if (df_le(k.ahi_d, avf[i])) avf[i] = k.ahi_d;
+    for (int i = 0; i < N - 1; ++i) {
+      if (elseif) {
+        if (df_le(avf[i], k.alo_d)) avf[i] = k.alo_d;
+        else if (df_le(k.ahi_d, avf[i])) avf[i] = k.ahi_d;
+      } else {
+        if (df_le(avf[i], k.alo_d)) avf[i] = k.alo_d;
+        if (df_le(k.ahi_d, avf[i])) avf[i] = k.ahi_d;
+      }
     }
-    sum = df_add(sum, avf[i]);
   }
+  df sum = vf_sum<N>(avf);
   if (df_le(k.ahi_d, sum)) {
-    const df dif = df_sub(sum, k.ahi_d);
-#pragma unroll
-    for (int j = 0; j < N - 1; ++j) avf[j] = df_sub(avf[j], df_mul(df_div(avf[j], sum), dif));
+    vf_scale_df<N>(k, avf, sum);
     sum = k.ahi_d;
   }
   avf[N - 1] = df_sub(df_make(1.0f), sum);
@@ -894,10 +925,10 @@ __device__ unsigned relax_face_df(const M5Consts &k, float *v, df *cr, float &p_
     const int i_as = (df_lt(avf[0], avf[1]) && (k.mu[1] != 0.0)) ? 1 : 0;
     ratio = df_div(avf[i_as], avf0[i_as]);
   }
-  df num = df_make(0.0f), den = df_make(0.0f);
-  float sael = 0.0f;
+  df num = df_mul(avf[0], k.gpg_d[0]), den = df_mul(avf[0], k.ig1_d[0]);
+  float sael = ael[0];
 #pragma unroll
-  for (int iv = 0; iv < N; ++iv) {
+  for (int iv = 1; iv < N; ++iv) {
     num = df_add(num, df_mul(avf[iv], k.gpg_d[iv]));
     den = df_add(den, df_mul(avf[iv], k.ig1_d[iv]));
     sael += ael[iv];
@@ -980,111 +1011,107 @@ __global__ void __launch_bounds__(256) m5f_shadow(int64_t n, const double *__res
   }
 }
 
-// 7 blocks of 128 threads per SM (72 registers): the kernel is bound by latency and
-// instruction issue; measured on the wall configuration, 6 blocks (80 registers) 4.4 % and
-// 5 blocks (96 registers) 7 % slower
+// A block takes 32 cells, one warp per face.  A thread forms the differences across its own face
+// only and takes those across the opposite face, the other one-sided slope, from that face's warp
+// through shared memory: each neighbour is loaded, limited and subtracted once per cell and face
+// instead of twice.  Bound by instruction issue (74 % active) and latency; wall mesh of 10.1 M
+// cells 7.47 -> 5.37 ms per stage, 0.41 M 350 -> 253 us, bubble mesh of 2.3 M 1336 -> 954 us.  Six
+// blocks of 192 threads per SM (56 registers): 5.88 ms at four (80), 5.58 at five (64), 5.87 at
+// seven (48); on a mesh that does not fill the chip (15,968 cells) all take the same 36 us.
+constexpr int RF_CELLS = 32, RF_TPB = 6 * RF_CELLS;
 template <int N>
-__global__ void __launch_bounds__(128, 7) m5f_recon_face(ffv_dmesh m, ffv_geom g, M5Consts k,
-                                                      const float *__restrict__ Sf,
-                                                      const float *__restrict__ Sflo,
-                                                      float *__restrict__ SF,
-                                                      unsigned *__restrict__ status) {
+__global__ void __launch_bounds__(RF_TPB, 6) m5f_recon_face(ffv_dmesh m, ffv_geom g, M5Consts k,
+                                                            const float *__restrict__ Sf,
+                                                            const float *__restrict__ Sflo,
+                                                            float *__restrict__ SF,
+                                                            unsigned *__restrict__ status) {
   using C = K5<N>;
   using RL = RecL<N>;
-  constexpr int NCR = 2 * N;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 6 * m.n) return;
-  const int f = (int)(t / m.n);
-  const int64_t c = t - (int64_t)f * m.n;
+  constexpr int NCR = 2 * N, NS = C::NEQ - N;  // NS: all slots but the internal energies
+  __shared__ float diff[6][NS][RF_CELLS];
+  const int f = threadIdx.x / RF_CELLS, lane = threadIdx.x % RF_CELLS;
+  const int64_t c = (int64_t)blockIdx.x * RF_CELLS + lane;
+  const bool live = c < m.n;
   const int fo = fr_opp(f);
-  const uint32_t info = m.info[c];
+  uint32_t info = 0;
+  float sl[C::NEQ], d[C::NEQ];
+  df cr[NCR];
+  if (live) {
+    info = m.info[c];
+    const uint32_t kf = ffv_face_kind(info, f);
+#pragma unroll
+    for (int i = 0; i < C::NEQ; i++) sl[i] = Sf[(int64_t)i * m.n + c];
+    value_across_f<N>(k, m, Sf, c, f, kf, sl, d);
+    avf_limit_f<N>(k, sl);
+    // the critical slots of the cell (volume fractions limited as avf_limit does)
+    crit_load<N>(Sf, Sflo, m.n, c, cr);
+    avf_limit_df<N>(k, cr);
+    df x[N];
+    steep_across_df<N>(k, m, Sf, Sflo, c, f, kf, cr, x);
+#pragma unroll
+    for (int i = 0; i < C::NEQ; i++) d[i] -= sl[i];
+    // the steep slots' differences in double-float, rounded to FP32
+#pragma unroll
+    for (int j = 0; j < N; j++)
+      d[crit_slot<N>(steep_slot<N>(j))] = df_to_float(df_sub(x[j], cr[steep_slot<N>(j)]));
+#pragma unroll
+    for (int i = 0; i < NS; i++) diff[f][i][lane] = d[i < C::i4 ? i : i + N];
+  }
+  __syncthreads();
+  if (!live) return;
   const int l = ffv_info_level(info);
   const uint32_t kf = ffv_face_kind(info, f), ko = ffv_face_kind(info, fo);
-  float sl[C::NEQ], x[C::NEQ], df_[C::NEQ];
-#pragma unroll
-  for (int i = 0; i < C::NEQ; i++) sl[i] = Sf[(int64_t)i * m.n + c];
-  avf_limit_f<N>(k, sl);
-  // the critical slots of the cell (volume fractions limited as avf_limit does)
-  df cr[NCR];
-  crit_load<N>(Sf, Sflo, m.n, c, cr);
-  avf_limit_df<N>(k, cr);
-  // the differences across face f (side 0) and across the opposite face (side 1), unrolled:
-  // both neighbours' loads are in flight together, and with the two sides' arrays resolved
-  // at compile time the 80 registers spill less (measured: 11 % faster than one rolled copy)
-  float db_[C::NEQ];
-#pragma unroll
-  for (int side = 0; side < 2; side++) {
-    const int fs = side ? fo : f;
-    const uint32_t ks = side ? ko : kf;
-    value_across_f<N>(k, m, Sf, c, fs, ks, sl, x);
-    // the critical slots' differences in double-float, rounded to FP32
-    df xc[NCR];
-    crit_across_df<N>(k, m, Sf, Sflo, c, fs, ks, cr, xc);
-#pragma unroll
-    for (int i = 0; i < C::NEQ; i++) x[i] -= sl[i];
-#pragma unroll
-    for (int j = 0; j < NCR; j++) x[crit_slot<N>(j)] = df_to_float(df_sub(xc[j], cr[j]));
-#pragma unroll
-    for (int i = 0; i < C::NEQ; i++) {
-      if (side == 0) df_[i] = x[i];
-      else db_[i] = x[i];
-    }
-  }
   const float idp = g.idcc_f[l][face_class(kf)];
   const float idm = g.idcc_f[l][face_class(ko)];
   const float cf = g.dcf_f[l][face_class(kf)];
-  float corr[C::NEQ];
 #pragma unroll
-  for (int i = 0; i < C::NEQ; i++) {
-    const float db = db_[i];
+  for (int s = 0; s < NS; s++) {
+    const int i = s < C::i4 ? s : s + N;
+    const float db = diff[fo][s][lane];
     float grad = 0.0f;
-    if (!(kf & FFV_FK_BC) && fabsf(df_[i]) > 1e-10f && !(i >= C::i4 && i < C::i5)) {
-      const float sf = df_[i] * idp, sb = -db * idm;
+    if (!(kf & FFV_FK_BC) && fabsf(d[i]) > 1e-10f) {
+      const float sf = d[i] * idp, sb = -db * idm;
       if (sb * sf > 0.0f) grad = (fabsf(sb) > fabsf(sf)) ? sf : sb;
     }
-    corr[i] = cf * grad;
-    sl[i] += corr[i];  // the face value of the FP32 copy
+    d[i] = cf * grad;
+    sl[i] += d[i];  // the face value of the FP32 copy
   }
 #pragma unroll
-  for (int j = 0; j < NCR; j++) cr[j] = df_add_f(cr[j], corr[crit_slot<N>(j)]);
+  for (int j = 0; j < N; j++)
+    cr[steep_slot<N>(j)] = df_add_f(cr[steep_slot<N>(j)], d[crit_slot<N>(steep_slot<N>(j))]);
   // m5_reconctruct.c:144-179: volume-fraction limits of the face state
-  {
-    df sum = df_make(0.0f);
+  if (vf_near_bounds<N>(cr, k.alo_d, k.a2lo_d)) {
 #pragma unroll
     for (int iv = 0; iv < N - 1; ++iv) {
-      df a = cr[iv];
-      if (df_le(a, k.alo_d)) a = k.alo_d;
-      else if (df_le(k.a2lo_d, a)) a = k.a2lo_d;
-      cr[iv] = a;
-      sum = df_add(sum, a);
+      if (df_le(cr[iv], k.alo_d)) cr[iv] = k.alo_d;
+      else if (df_le(k.a2lo_d, cr[iv])) cr[iv] = k.a2lo_d;
     }
-    if (df_le(k.ahi_d, sum)) {
-      const df dif = df_sub(sum, k.ahi_d);
-#pragma unroll
-      for (int j = 0; j < N - 1; ++j) cr[j] = df_sub(cr[j], df_mul(df_div(cr[j], sum), dif));
-    }
+  }
+  {
+    const df sum = vf_sum<N>(cr);
+    if (df_le(k.ahi_d, sum)) vf_scale_df<N>(k, cr, sum);
   }
   float p_eq;
   const unsigned st = relax_face_df<N>(k, sl, cr, p_eq);
   // the face record: FP32 state with the critical slots rounded from their pairs, the
   // volume fractions as make_sol limits them, the equilibrium pressure for every material
   df at[N];
-  df sum = df_make(0.0f);
 #pragma unroll
-  for (int i = 0; i < N - 1; ++i) {
-    at[i] = cr[i];
-    if (df_le(at[i], k.alo_d)) at[i] = k.alo_d;
-    else if (df_le(k.ahi_d, at[i])) at[i] = k.ahi_d;
-    sum = df_add(sum, at[i]);
+  for (int i = 0; i < N - 1; ++i) at[i] = cr[i];
+  if (vf_near_bounds<N>(at, k.alo_d, k.ahi_d)) {
+#pragma unroll
+    for (int i = 0; i < N - 1; ++i) {
+      if (df_le(at[i], k.alo_d)) at[i] = k.alo_d;
+      else if (df_le(k.ahi_d, at[i])) at[i] = k.ahi_d;
+    }
   }
+  df sum = vf_sum<N>(at);
   if (df_lt(k.ahi_d, sum)) {
-    const df dif = df_sub(sum, k.ahi_d);
-#pragma unroll
-    for (int j = 0; j < N - 1; ++j) at[j] = df_sub(at[j], df_mul(df_div(at[j], sum), dif));
+    vf_scale_df<N>(k, at, sum);
     sum = k.ahi_d;
   }
   at[N - 1] = df_sub(df_make(1.0f), sum);
-  float *out = SF + (int64_t)f * RL::SIZE * m.n + c;
+  float *out = SF + (int64_t)f * RL::STORED * m.n + c;
 #pragma unroll
   for (int j = N - 1; j < NCR; j++) sl[crit_slot<N>(j)] = df_to_float(cr[j]);
 #pragma unroll
@@ -1092,8 +1119,7 @@ __global__ void __launch_bounds__(128, 7) m5f_recon_face(ffv_dmesh m, ffv_geom g
 #pragma unroll
   for (int i = 0; i < C::NEQ; i++) out[(int64_t)i * m.n] = sl[i];
   out[(int64_t)RL::AL * m.n] = df_to_float(at[N - 1]);
-#pragma unroll
-  for (int i = 0; i < N; ++i) out[(int64_t)(RL::P + i) * m.n] = p_eq;
+  out[(int64_t)RL::P * m.n] = p_eq;
   if (st) atomicOr(status, st);
 }
 
@@ -1102,7 +1128,9 @@ __device__ __forceinline__ void load_record(const float *__restrict__ SF, int64_
                                             int64_t c, float *U) {
   using RL = RecL<N>;
 #pragma unroll
-  for (int v = 0; v < RL::SIZE; v++) U[v] = SF[((int64_t)f * RL::SIZE + v) * n + c];
+  for (int v = 0; v < RL::STORED; v++) U[v] = SF[((int64_t)f * RL::STORED + v) * n + c];
+#pragma unroll
+  for (int v = RL::STORED; v < RL::SIZE; v++) U[v] = U[RL::P];
 }
 
 // order 1: the record of a cell state
@@ -1188,12 +1216,12 @@ __device__ __forceinline__ void owner_flux_f(const ffv_dmesh &m, const ffv_geom 
 }
 
 // The faces between cells of one level, each once: the positive face of one axis (blockIdx.y).
-// Bound by memory latency at 4 blocks of 128 threads per SM (118 registers).  Without the loop over
-// finer neighbours the kernel needs no spills (it took ~900 bytes per thread), and the listed
-// faces no longer run as single lanes of its warps: together 34.8 -> 30.9 ms per step on the wall
-// mesh of 10.1 M cells, 6.66 -> 5.85 ms on the bubble mesh of 2.3 M.
+// Bound by memory latency.  Without the loop over finer neighbours the kernel needs no spills (it
+// took ~900 bytes per thread), and the listed faces no longer run as single lanes of its warps:
+// 4.89 -> 2.62 + 0.34 ms per stage on the wall mesh of 10.1 M cells.  Six blocks of 128 threads per
+// SM: 2.55 ms (2.89 at four, 2.57 at five).
 template <int N>
-__global__ void __launch_bounds__(128, 4) m5f_face_flux(ffv_dmesh m, ffv_geom g, M5Consts k,
+__global__ void __launch_bounds__(128, 6) m5f_face_flux(ffv_dmesh m, ffv_geom g, M5Consts k,
                                                      const double *__restrict__ S,
                                                      const float *__restrict__ Sf,
                                                      const float *__restrict__ SF,
@@ -1293,7 +1321,8 @@ __device__ __forceinline__ void clamp_zerou_d(const M5Consts &k, double *s, cons
 // three fused multiply-adds per variable.  The RK stage, positivity, ZEROU and the stage-1
 // ghost-fluid trigger as in the FP64 form.  RHS receives the entries the ghost-fluid fix
 // reads (partial densities and momentum).
-// three blocks of 128 threads per SM (at most 170 registers)
+// three blocks of 128 threads per SM (at most 170 registers): 2.76 ms per stage on the wall mesh of
+// 10.1 M cells (4.15 at four, which spills, 3.29 at two)
 template <int N>
 __global__ void __launch_bounds__(128, 3) m5f_cell_update(ffv_dmesh m, ffv_geom g, M5Consts k,
                                                        const double *__restrict__ S,
@@ -1471,9 +1500,10 @@ __global__ void __launch_bounds__(128, 3) m5f_cell_update(ffv_dmesh m, ffv_geom 
   if (st) atomicOr(status, st);
 }
 
-// 6 blocks of 128 threads per SM (80 registers): 10 % faster than 4 blocks at 124 registers
+// 7 blocks of 128 threads per SM: wall mesh of 10.1 M cells 1.18 ms per stage (1.20 at six, 1.23 at
+// five), bubble mesh of 2.3 M 193 us (199 at six)
 template <int N>
-__global__ void __launch_bounds__(128, 6) m5f_relax_cell(int64_t n, M5Consts k,
+__global__ void __launch_bounds__(128, 7) m5f_relax_cell(int64_t n, M5Consts k,
                                                       const double *__restrict__ Sin,
                                                       double *__restrict__ Sout,
                                                       uint8_t *__restrict__ flag,
@@ -1567,9 +1597,9 @@ void ffv_m5f_recon(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, con
                    const float *Sf, float *SFf, unsigned *status, cudaStream_t st) {
   (void)S;
   const float *Sflo = Sf + (int64_t)ffv_m5_neq(k.nmat) * m.n;
-  const unsigned blocks = (unsigned)((6 * m.n + 127) / 128);
-  if (k.nmat == 2) m5f_recon_face<2><<<blocks, 128, 0, st>>>(m, g, k, Sf, Sflo, SFf, status);
-  else m5f_recon_face<3><<<blocks, 128, 0, st>>>(m, g, k, Sf, Sflo, SFf, status);
+  const unsigned blocks = (unsigned)((m.n + RF_CELLS - 1) / RF_CELLS);
+  if (k.nmat == 2) m5f_recon_face<2><<<blocks, RF_TPB, 0, st>>>(m, g, k, Sf, Sflo, SFf, status);
+  else m5f_recon_face<3><<<blocks, RF_TPB, 0, st>>>(m, g, k, Sf, Sflo, SFf, status);
 }
 
 void ffv_m5f_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
