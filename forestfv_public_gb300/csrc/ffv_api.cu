@@ -31,7 +31,7 @@ struct ffv_ctx {
   int32_t *d_flist, *d_flist_own;
   int64_t cap_flist_own;
   ffv_face_list flist;
-  int32_t *d_list, *d_bcount, *d_count;
+  int32_t *d_list;       // flagged cells: count, cells [n], and the face list's 12 cursors
   M5Consts m5;
   // refinement tags
   int32_t *d_SI, *d_SItmp, *d_split;
@@ -74,8 +74,6 @@ void free_mesh_buffers(ffv_ctx *c) {
   cudaFree(c->d_RHS);
   cudaFree(c->d_flag);
   cudaFree(c->d_list);
-  cudaFree(c->d_bcount);
-  cudaFree(c->d_count);
   cudaFree(c->d_flist_own);
   c->d_flist = c->d_flist_own = nullptr;
   c->cap_flist_own = 0;
@@ -90,7 +88,7 @@ void free_mesh_buffers(ffv_ctx *c) {
   c->d_S = c->d_SN = c->d_SF = nullptr;
   c->d_Snew = c->d_FF = c->d_UF = c->d_RHS = nullptr;
   c->d_GF = c->d_flag = nullptr;
-  c->d_list = c->d_bcount = c->d_count = nullptr;
+  c->d_list = nullptr;
   c->cap = c->cap_nsub = 0;
   if (c->graph_valid) cudaGraphExecDestroy(c->graph);
   c->graph_valid = 0;
@@ -111,16 +109,13 @@ int alloc_mesh_buffers(ffv_ctx *c) {
     return FFV_ERR_NOMEM;
   }
   if (c->p.model == 5) {
-    const int64_t nb = (n + 1023) / 1024;
     if (cudaMalloc(&c->d_Snew, sizeof(double) * c->neq * n) != cudaSuccess ||
         cudaMalloc(&c->d_FF, sizeof(double) * 6 * c->neq * n) != cudaSuccess ||
         cudaMalloc(&c->d_UF, sizeof(double) * 18 * n) != cudaSuccess ||
         cudaMalloc(&c->d_GF, (((6 * n + 3) & ~(int64_t)3) + 4 * n)) != cudaSuccess ||
         cudaMalloc(&c->d_RHS, sizeof(double) * c->neq * n) != cudaSuccess ||
         cudaMalloc(&c->d_flag, n) != cudaSuccess ||
-        cudaMalloc(&c->d_list, sizeof(int32_t) * n) != cudaSuccess ||
-        cudaMalloc(&c->d_bcount, sizeof(int32_t) * nb) != cudaSuccess ||
-        cudaMalloc(&c->d_count, sizeof(int32_t) * 16) != cudaSuccess) {  // count, 12 cursors
+        cudaMalloc(&c->d_list, sizeof(int32_t) * (n + 13)) != cudaSuccess) {
       free_mesh_buffers(c);
       return FFV_ERR_NOMEM;
     }
@@ -149,8 +144,8 @@ int launch_stage(ffv_ctx *c, int irk, cudaEvent_t *ev = nullptr) {
   }
   if (c->p.model == 5) {
     ffv_m5_bufs mb{c->d_S,   c->d_SN,   c->d_Snew, c->d_SF,     c->d_FF,    c->d_UF,
-                   c->d_RHS, c->d_dt,   c->d_GF,   c->d_flag,   c->d_list,  c->d_bcount,
-                   c->d_count, c->d_status, c->flist};
+                   c->d_RHS, c->d_dt,   c->d_GF,   c->d_flag,   c->d_list,  c->d_status,
+                   c->flist};
     ffv_m5_fp64_stage(c->dm, c->geom, c->m5, mb, irk, c->stream, ev, c->knames);
     return cuda_rc(cudaGetLastError());
   }
@@ -246,9 +241,11 @@ int build_face_list(ffv_ctx *c, const int64_t count[12]) {
   }
   l.cells = cells;
   CK(cudaMemsetAsync(c->d_GF, 0, 6 * c->n, c->stream));
+  CK(cudaMemsetAsync(c->d_list, 0, sizeof(int32_t), c->stream));  // no flagged cells
   if (total == 0) return FFV_OK;
-  CK(cudaMemcpyAsync(c->d_count + 1, l.off, sizeof(int32_t) * 12, cudaMemcpyHostToDevice, c->stream));
-  list_faces<<<(unsigned)((c->n + 255) / 256), 256, 0, c->stream>>>(c->n, c->d_info, c->d_count + 1, cells);
+  int32_t *cursor = c->d_list + 1 + c->cap;
+  CK(cudaMemcpyAsync(cursor, l.off, sizeof(int32_t) * 12, cudaMemcpyHostToDevice, c->stream));
+  list_faces<<<(unsigned)((c->n + 255) / 256), 256, 0, c->stream>>>(c->n, c->d_info, cursor, cells);
   return cuda_rc(cudaGetLastError());
 }
 

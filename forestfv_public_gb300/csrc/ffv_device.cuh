@@ -82,6 +82,21 @@ __device__ __forceinline__ int ffv_listed_face(const ffv_face_list &fl, int64_t 
   return g >> 1;
 }
 
+// a launch over all faces: the list's blocks, then three axes of FFV_LIST_TPB cells each
+static inline unsigned ffv_flux_blocks(const ffv_face_list &fl, int64_t n) {
+  return (unsigned)(fl.block[12] + 3 * ((n + FFV_LIST_TPB - 1) / FFV_LIST_TPB));
+}
+// whether this block is one of the latter, its axis and this thread's cell
+__device__ __forceinline__ bool ffv_owner_block(const ffv_face_list &fl, int64_t n, int &axis,
+                                                int64_t &c) {
+  const int b = (int)blockIdx.x - fl.block[12];
+  if (b < 0) return false;
+  const int per = (int)((n + FFV_LIST_TPB - 1) / FFV_LIST_TPB);
+  axis = b / per;
+  c = (int64_t)(b - axis * per) * FFV_LIST_TPB + threadIdx.x;
+  return true;
+}
+
 // The faces towards a neighbour of the same level that comes later in leaf order.  The order is
 // a Morton order, in which a neighbour one step along an axis comes later than the cell and one
 // step back earlier, so these are the faces of the three positive sides.

@@ -47,7 +47,7 @@ struct ffv_m5_bufs {
   double *S, *SN, *Snew, *SF, *FF, *UF, *RHS, *dt;
   uint8_t *GF, *flag;  // GF [6][n]: ghost-fluid faces, as the cell that evaluates the face sees them
 
-  int32_t *list, *bcount, *count;
+  int32_t *list;  // [1 + n]: the number of cells the last pass flagged, then the cells
   unsigned int *status;
   ffv_face_list list_faces;
 };
@@ -68,20 +68,16 @@ int ffv_m5_launches_per_stage(const M5Consts &k, int irk);
 void ffv_m5f_shadow(int64_t n, const M5Consts &k, const double *S, float *Sf, cudaStream_t st);
 void ffv_m5f_recon(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
                    const float *Sf, float *SFf, unsigned *status, cudaStream_t st);
-// the faces between cells of one level, and the listed others
 // Sf: the FP32 copy of the state (order 2), or nullptr (order 1: phi0 from S)
 void ffv_m5f_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
                   const float *Sf, const float *SFf, float *FFf, float *UFf, uint8_t *GF,
-                  unsigned *status, cudaStream_t st);
-void ffv_m5f_listed_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
-                         const float *Sf, const float *SFf, float *FFf, float *UFf, uint8_t *GF,
-                         const ffv_face_list &fl, unsigned *status, cudaStream_t st);
+                  const ffv_face_list &fl, unsigned *status, cudaStream_t st);
 // residual + RK stage of the FP32-flux form (the face fluxes of all but the deformation
 // summed in FP64)
 void ffv_m5f_cell_update(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
                          double *SN, const float *FFf, const float *UFf, double *RHS,
-                         double *Snew, uint8_t *flag, const double *dt, int irk, unsigned *status,
-                         cudaStream_t st);
+                         double *Snew, uint8_t *flag, int32_t *list, const double *dt, int irk,
+                         unsigned *status, cudaStream_t st);
 // the indicator's fields of a model-5 state, F [5][n] float (log rho, log p, alpha_0, |u|,
 // von Mises stress; FP32 with double-float pressure recovery; ffv_mlp.cu gathers them)
 void ffv_m5f_indicator_fields(int64_t n, const M5Consts &k, const double *S, float *F,
@@ -89,7 +85,7 @@ void ffv_m5f_indicator_fields(int64_t n, const M5Consts &k, const double *S, flo
 // cell pressure relaxation: the Newton iteration in FP32, the pressure recovery and the
 // energy-consistent pressure and internal energies in double-float
 void ffv_m5f_relax_cell(int64_t n, const M5Consts &k, const double *Sin, double *Sout,
-                        uint8_t *flag, unsigned *status, cudaStream_t st);
+                        uint8_t *flag, int32_t *list, unsigned *status, cudaStream_t st);
 void ffv_m5_cfl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
                 unsigned long long *d_out, cudaStream_t st);
 

@@ -1202,8 +1202,7 @@ __device__ __forceinline__ void owner_flux_f(const ffv_dmesh &m, const ffv_geom 
                                              const float *__restrict__ Sf,
                                              const float *__restrict__ SF, float *__restrict__ FF,
                                              float *__restrict__ UF, uint8_t *__restrict__ GF,
-                                             unsigned *status) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+                                             unsigned *status, int64_t c) {
   if (c >= m.n) return;
   const uint32_t info = m.info[c];
   // a 1:1 face is evaluated by its earlier cell (flux reuse, m5_residual.c:80-99)
@@ -1213,25 +1212,6 @@ __device__ __forceinline__ void owner_flux_f(const ffv_dmesh &m, const ffv_geom 
   const bool gfm = face_flux_f<N, F>(m, g, k, S, Sf, SF, c, info, 0, ff, un, st);
   store_flux_f<N>(m.n, F, c, ff, un, gfm, FF, UF, GF);
   if (st) atomicOr(status, st);
-}
-
-// The faces between cells of one level, each once: the positive face of one axis (blockIdx.y).
-// Bound by memory latency.  Without the loop over finer neighbours the kernel needs no spills (it
-// took ~900 bytes per thread), and the listed faces no longer run as single lanes of its warps:
-// 4.89 -> 2.62 + 0.34 ms per stage on the wall mesh of 10.1 M cells.  Six blocks of 128 threads per
-// SM: 2.55 ms (2.89 at four, 2.57 at five).
-template <int N>
-__global__ void __launch_bounds__(128, 6) m5f_face_flux(ffv_dmesh m, ffv_geom g, M5Consts k,
-                                                     const double *__restrict__ S,
-                                                     const float *__restrict__ Sf,
-                                                     const float *__restrict__ SF,
-                                                     float *__restrict__ FF,
-                                                     float *__restrict__ UF,
-                                                     uint8_t *__restrict__ GF,
-                                                     unsigned *__restrict__ status) {
-  if (blockIdx.y == 0) owner_flux_f<N, owner_face(0)>(m, g, k, S, Sf, SF, FF, UF, GF, status);
-  else if (blockIdx.y == 1) owner_flux_f<N, owner_face(1)>(m, g, k, S, Sf, SF, FF, UF, GF, status);
-  else owner_flux_f<N, owner_face(2)>(m, g, k, S, Sf, SF, FF, UF, GF, status);
 }
 
 template <int N, int F>
@@ -1268,13 +1248,26 @@ __device__ __forceinline__ void listed_flux_f(const ffv_dmesh &m, const ffv_geom
   if (st) atomicOr(status, st);
 }
 
-// the boundary, coarser and finer faces, from the mesh's list of them
+// All face fluxes in one launch, as the FP64 form's: the listed faces' blocks, then the faces
+// between cells of one level, each once.  Bound by memory latency.  Without a loop over finer
+// neighbours the kernel needs few spills (it took ~900 bytes per thread), and the listed faces no
+// longer run as single lanes of its warps: 4.89 -> 2.99 ms per stage on the wall mesh of 10.1 M
+// cells, 240 -> 168 us at 0.41 M, 33 -> 17 us at 15,968 (29 us as two launches, one after the
+// other; 2.91 ms and 166 us on the larger meshes).  Five blocks of 128 threads per SM (3.06 ms at
+// six, 3.40 at four).
 template <int N>
-__global__ void __launch_bounds__(FFV_LIST_TPB, 4) m5f_listed_flux(
+__global__ void __launch_bounds__(FFV_LIST_TPB, 5) m5f_face_flux(
     ffv_dmesh m, ffv_geom g, M5Consts k, ffv_face_list fl, const double *__restrict__ S,
     const float *__restrict__ Sf, const float *__restrict__ SF, float *__restrict__ FF,
     float *__restrict__ UF, uint8_t *__restrict__ GF, unsigned *__restrict__ status) {
+  int axis;
   int64_t c;
+  if (ffv_owner_block(fl, m.n, axis, c)) {
+    if (axis == 0) owner_flux_f<N, owner_face(0)>(m, g, k, S, Sf, SF, FF, UF, GF, status, c);
+    else if (axis == 1) owner_flux_f<N, owner_face(1)>(m, g, k, S, Sf, SF, FF, UF, GF, status, c);
+    else owner_flux_f<N, owner_face(2)>(m, g, k, S, Sf, SF, FF, UF, GF, status, c);
+    return;
+  }
   bool live, finer;
   const int f = ffv_listed_face(fl, c, live, finer);
   switch (f) {
@@ -1332,6 +1325,7 @@ __global__ void __launch_bounds__(128, 3) m5f_cell_update(ffv_dmesh m, ffv_geom 
                                                        double *__restrict__ RHS,
                                                        double *__restrict__ Snew,
                                                        uint8_t *__restrict__ flag,
+                                                       int32_t *__restrict__ list,
                                                        const double *__restrict__ dtp, int irk,
                                                        unsigned *__restrict__ status) {
   using C = K5<N>;
@@ -1497,6 +1491,7 @@ __global__ void __launch_bounds__(128, 3) m5f_cell_update(ffv_dmesh m, ffv_geom 
 #pragma unroll
   for (int e = 0; e < C::NEQ; e++) Snew[(int64_t)e * m.n + c] = s[e];
   flag[c] = gfm ? 1 : 0;
+  if (gfm) list[1 + atomicAdd(list, 1)] = (int32_t)c;
   if (st) atomicOr(status, st);
 }
 
@@ -1507,6 +1502,7 @@ __global__ void __launch_bounds__(128, 7) m5f_relax_cell(int64_t n, M5Consts k,
                                                       const double *__restrict__ Sin,
                                                       double *__restrict__ Sout,
                                                       uint8_t *__restrict__ flag,
+                                                      int32_t *__restrict__ list,
                                                       unsigned *__restrict__ status) {
   using C = K5<N>;
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1517,7 +1513,9 @@ __global__ void __launch_bounds__(128, 7) m5f_relax_cell(int64_t n, M5Consts k,
   const unsigned st = relax_cell_df<N>(k, s);
   if (k.plastic) plastic_return<N>(k, s);  // as the FP64 form: FP64 return after relaxation
   const double phi_new = (k.mu[0] != 0.0) ? s[C::i3] - k.avf_lim : phi_old;
-  flag[c] = (phi_old * phi_new < 0.0) ? 1 : 0;
+  const bool crossed = phi_old * phi_new < 0.0;
+  flag[c] = crossed ? 1 : 0;
+  if (crossed) list[1 + atomicAdd(list, 1)] = (int32_t)c;
 #pragma unroll
   for (int e = 0; e < C::NEQ; e++) Sout[(int64_t)e * n + c] = s[e];
   if (st) atomicOr(status, st);
@@ -1604,31 +1602,23 @@ void ffv_m5f_recon(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, con
 
 void ffv_m5f_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
                   const float *Sf, const float *SFf, float *FFf, float *UFf, uint8_t *GF,
-                  unsigned *status, cudaStream_t st) {
-  const dim3 blocks((unsigned)((m.n + 127) / 128), 3);
-  if (k.nmat == 2) m5f_face_flux<2><<<blocks, 128, 0, st>>>(m, g, k, S, Sf, SFf, FFf, UFf, GF, status);
-  else m5f_face_flux<3><<<blocks, 128, 0, st>>>(m, g, k, S, Sf, SFf, FFf, UFf, GF, status);
-}
-
-void ffv_m5f_listed_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
-                         const float *Sf, const float *SFf, float *FFf, float *UFf, uint8_t *GF,
-                         const ffv_face_list &fl, unsigned *status, cudaStream_t st) {
-  const unsigned blocks = (unsigned)fl.block[12];
+                  const ffv_face_list &fl, unsigned *status, cudaStream_t st) {
+  const unsigned blocks = ffv_flux_blocks(fl, m.n);
   if (k.nmat == 2)
-    m5f_listed_flux<2><<<blocks, FFV_LIST_TPB, 0, st>>>(m, g, k, fl, S, Sf, SFf, FFf, UFf, GF, status);
+    m5f_face_flux<2><<<blocks, FFV_LIST_TPB, 0, st>>>(m, g, k, fl, S, Sf, SFf, FFf, UFf, GF, status);
   else
-    m5f_listed_flux<3><<<blocks, FFV_LIST_TPB, 0, st>>>(m, g, k, fl, S, Sf, SFf, FFf, UFf, GF, status);
+    m5f_face_flux<3><<<blocks, FFV_LIST_TPB, 0, st>>>(m, g, k, fl, S, Sf, SFf, FFf, UFf, GF, status);
 }
 
 void ffv_m5f_cell_update(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
                          double *SN, const float *FFf, const float *UFf, double *RHS,
-                         double *Snew, uint8_t *flag, const double *dt, int irk, unsigned *status,
-                         cudaStream_t st) {
+                         double *Snew, uint8_t *flag, int32_t *list, const double *dt, int irk,
+                         unsigned *status, cudaStream_t st) {
   const unsigned blocks = (unsigned)((m.n + 127) / 128);
   if (k.nmat == 2)
-    m5f_cell_update<2><<<blocks, 128, 0, st>>>(m, g, k, S, SN, FFf, UFf, RHS, Snew, flag, dt, irk, status);
+    m5f_cell_update<2><<<blocks, 128, 0, st>>>(m, g, k, S, SN, FFf, UFf, RHS, Snew, flag, list, dt, irk, status);
   else
-    m5f_cell_update<3><<<blocks, 128, 0, st>>>(m, g, k, S, SN, FFf, UFf, RHS, Snew, flag, dt, irk, status);
+    m5f_cell_update<3><<<blocks, 128, 0, st>>>(m, g, k, S, SN, FFf, UFf, RHS, Snew, flag, list, dt, irk, status);
 }
 
 void ffv_m5f_indicator_fields(int64_t n, const M5Consts &k, const double *S, float *F,
@@ -1639,8 +1629,8 @@ void ffv_m5f_indicator_fields(int64_t n, const M5Consts &k, const double *S, flo
 }
 
 void ffv_m5f_relax_cell(int64_t n, const M5Consts &k, const double *Sin, double *Sout,
-                        uint8_t *flag, unsigned *status, cudaStream_t st) {
+                        uint8_t *flag, int32_t *list, unsigned *status, cudaStream_t st) {
   const unsigned blocks = (unsigned)((n + 127) / 128);
-  if (k.nmat == 2) m5f_relax_cell<2><<<blocks, 128, 0, st>>>(n, k, Sin, Sout, flag, status);
-  else m5f_relax_cell<3><<<blocks, 128, 0, st>>>(n, k, Sin, Sout, flag, status);
+  if (k.nmat == 2) m5f_relax_cell<2><<<blocks, 128, 0, st>>>(n, k, Sin, Sout, flag, list, status);
+  else m5f_relax_cell<3><<<blocks, 128, 0, st>>>(n, k, Sin, Sout, flag, list, status);
 }

@@ -23,10 +23,10 @@
 //                                  reuse, m5_residual.c:59-173)
 //   m5_cell_update  (cell)        residual sum + non-conservative terms (m5_residual.c:175-215),
 //                                  RK stage (m5_RK.c), positivity and ZEROU masks
-//   compaction + m5_gfm_seq       cells whose solid fraction crosses AVF_LIM in stage 1, in
+//   m5_gfm_seq                    cells whose solid fraction crosses AVF_LIM in stage 1, in
 //                                  leaf order (m5_gfm.c reads earlier neighbours' new state)
 //   m5_relax_cell   (cell)        cell pressure relaxation (m5_relaxation_solid.c)
-//   compaction + m5_gfm_rel_seq   relaxation-crossing cells in leaf order (m5_gfm_rel.c)
+//   m5_gfm_seq (relax)            relaxation-crossing cells in leaf order (m5_gfm_rel.c)
 #include <math.h>
 
 #include "ffv_device.cuh"
@@ -554,6 +554,12 @@ __device__ __forceinline__ double rcp_near(double x) {
   r = fma(fma(-x, r, 1.0), r, r);
   return fma(fma(-x, r, 1.0), r, r);
 }
+// y / x, the quotient from that reciprocal corrected by its remainder (Markstein): the rounded
+// quotient but where it lies within ~2^-100 of a midpoint
+__device__ __forceinline__ double div_near(double y, double x) {
+  const double r = rcp_near(x), q = y * r;
+  return fma(fma(-q, x, y), r, q);
+}
 
 // Newton on sum_k alpha_k(p) = 1 along each material's isentrope (m5_relaxationvec.c:456-490), to
 // |F| <= 1e-12 or the reference's cap of 500 iterations; alpha[k] receives the last iterate's
@@ -606,11 +612,11 @@ __device__ __forceinline__ bool newton_reference(const M5Consts &k, const double
 // ratio x = (p + p_inf) / (p_k + p_inf) is near 1 in all but the cells of an interface or a strong
 // shock: for |x - 1| <= 1/32 the power is 1 + t P(t), t = x - 1 (exact), P the binomial series to t^9
 // (the first omitted term is below 3e-18), rounded once -- an error of at most 0.53 ulp, below
-// pow's.  Reciprocals of the two other quotients' divisors take Newton-Raphson steps; the
-// fraction itself is corrected by its remainder.  31 FP64 instructions per material and iteration
-// against ~110 with pow and three divisions; the iterates differ from the reference's in the last
-// bit at most, so that the stopping test falls alike (a series in p - p_k, more exact still, moved
-// it in one state of 200,000, and with it a fraction by 1e-12).
+// pow's -- and the two other quotients start from Newton-Raphson reciprocals.  35 FP64 instructions
+// per material and iteration against ~110 with pow and three divisions.  The iterates are the
+// reference's but where the two powers round differently, so that the stopping test, |F| <= 1e-12,
+// falls alike: with derivatives good to an ulp only, or a series in p - p_k (more exact still), it
+// fell otherwise in one state of ~200,000 and moved a fraction by 1e-12.
 template <int N>
 __device__ __forceinline__ bool newton_series(const M5Consts &k, const double *avf,
                                               const double *ar, const bool *live,
@@ -648,10 +654,10 @@ __device__ __forceinline__ bool newton_series(const M5Consts &k, const double *a
         } else {
           pw = pow(x, k.igam[iv]);
         }
-        const double rho = rk[iv] * pw, r = rcp_near(rho), q = ar[iv] * r;
-        alpha[iv] = fma(fma(-q, rho, ar[iv]), r, q);
+        const double rho = rk[iv] * pw;
+        alpha[iv] = div_near(ar[iv], rho);
         F = F + alpha[iv];
-        dF = fma(-alpha[iv], rcp_near(k.gamma[iv] * pp), dF);
+        dF = dF - div_near(ar[iv], k.gamma[iv] * rho * pp);
       }
     }
     if (f64::is_nan(p) || f64::is_nan(F) || f64::is_nan(dF)) return true;
@@ -1006,8 +1012,7 @@ __device__ __forceinline__ void owner_flux(const ffv_dmesh &m, const ffv_geom &g
                                            const double *__restrict__ S,
                                            const double *__restrict__ SF, double *__restrict__ FF,
                                            double *__restrict__ UF, uint8_t *__restrict__ GF,
-                                           unsigned *status) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+                                           unsigned *status, int64_t c) {
   if (c >= m.n) return;
   const uint32_t info = m.info[c];
   // a 1:1 face is evaluated by its earlier cell, and m5_cell_update takes the negative for the
@@ -1018,22 +1023,6 @@ __device__ __forceinline__ void owner_flux(const ffv_dmesh &m, const ffv_geom &g
   const bool gfm = face_flux<N, ORDER, F>(m, g, k, S, SF, c, info, 0, ff, un, st);
   store_flux<N>(m.n, F, c, ff, un, gfm, FF, UF, GF);
   if (st) atomicOr(status, st);
-}
-
-// The faces between cells of one level, each once: the positive face of one axis (blockIdx.y).
-// FP64 pipe ~80 % busy; with the listed faces below 40.1 -> 19.5 ms per step on the wall mesh of
-// 0.41 M cells (21.3 before the list), 5.87 -> 3.83 ms on the bubble mesh of 51,584 (4.30).
-template <int N, int ORDER>
-__global__ void __launch_bounds__(128) m5_face_flux(ffv_dmesh m, ffv_geom g, M5Consts k,
-                                                    const double *__restrict__ S,
-                                                    const double *__restrict__ SF,
-                                                    double *__restrict__ FF,
-                                                    double *__restrict__ UF,
-                                                    uint8_t *__restrict__ GF,
-                                                    unsigned *__restrict__ status) {
-  if (blockIdx.y == 0) owner_flux<N, ORDER, owner_face(0)>(m, g, k, S, SF, FF, UF, GF, status);
-  else if (blockIdx.y == 1) owner_flux<N, ORDER, owner_face(1)>(m, g, k, S, SF, FF, UF, GF, status);
-  else owner_flux<N, ORDER, owner_face(2)>(m, g, k, S, SF, FF, UF, GF, status);
 }
 
 template <int N, int ORDER, int F>
@@ -1069,19 +1058,29 @@ __device__ __forceinline__ void listed_flux(const ffv_dmesh &m, const ffv_geom &
   if (st) atomicOr(status, st);
 }
 
-// The boundary, coarser and finer faces, from the mesh's list of them: on a refined mesh they are
-// 0.2 to 0.3 per cell, and as single lanes of the warps over all cells and faces they took a third
-// to a half of the kernel.
+// All face fluxes in one launch.  The first blocks take the boundary, coarser and finer faces from
+// the mesh's list of them (0.2 to 0.3 per cell on a refined mesh; as single lanes of the warps over
+// all cells and faces they took a third to a half of the kernel), the others the faces between
+// cells of one level, each once: the positive face of one axis of FFV_LIST_TPB cells.  FP64 pipe
+// ~80 % busy; with the list 40.1 -> 19.5 ms per step on the wall mesh of 0.41 M cells (21.3 before
+// it), 5.87 -> 3.83 ms on the bubble mesh of 51,584 (4.30).
 template <int N, int ORDER>
-__global__ void __launch_bounds__(FFV_LIST_TPB) m5_listed_flux(ffv_dmesh m, ffv_geom g, M5Consts k,
-                                                               ffv_face_list fl,
-                                                               const double *__restrict__ S,
-                                                               const double *__restrict__ SF,
-                                                               double *__restrict__ FF,
-                                                               double *__restrict__ UF,
-                                                               uint8_t *__restrict__ GF,
-                                                               unsigned *__restrict__ status) {
+__global__ void __launch_bounds__(FFV_LIST_TPB) m5_face_flux(ffv_dmesh m, ffv_geom g, M5Consts k,
+                                                             ffv_face_list fl,
+                                                             const double *__restrict__ S,
+                                                             const double *__restrict__ SF,
+                                                             double *__restrict__ FF,
+                                                             double *__restrict__ UF,
+                                                             uint8_t *__restrict__ GF,
+                                                             unsigned *__restrict__ status) {
+  int axis;
   int64_t c;
+  if (ffv_owner_block(fl, m.n, axis, c)) {
+    if (axis == 0) owner_flux<N, ORDER, owner_face(0)>(m, g, k, S, SF, FF, UF, GF, status, c);
+    else if (axis == 1) owner_flux<N, ORDER, owner_face(1)>(m, g, k, S, SF, FF, UF, GF, status, c);
+    else owner_flux<N, ORDER, owner_face(2)>(m, g, k, S, SF, FF, UF, GF, status, c);
+    return;
+  }
   bool live, finer;
   const int f = ffv_listed_face(fl, c, live, finer);
   switch (f) {
@@ -1163,6 +1162,7 @@ __global__ void __launch_bounds__(128) m5_cell_update(ffv_dmesh m, ffv_geom g, M
                                                       double *__restrict__ RHS,
                                                       double *__restrict__ Snew,
                                                       uint8_t *__restrict__ flag,
+                                                      int32_t *__restrict__ list,
                                                       const double *__restrict__ dtp, int irk,
                                                       unsigned *__restrict__ status) {
   using C = K5<N>;
@@ -1248,15 +1248,17 @@ __global__ void __launch_bounds__(128) m5_cell_update(ffv_dmesh m, ffv_geom g, M
 #pragma unroll
   for (int e = 0; e < C::NEQ; e++) Snew[(int64_t)e * m.n + c] = s[e];
   flag[c] = gfm ? 1 : 0;
+  if (gfm) list[1 + atomicAdd(list, 1)] = (int32_t)c;
   if (st) atomicOr(status, st);
 }
 
-// cell pressure relaxation (m5_relaxation_solid.c:16-32); flags solid-fraction crossings
+// cell pressure relaxation (m5_relaxation_solid.c:16-32); flags and lists solid-fraction crossings
 template <int N, bool FAST>
 __global__ void __launch_bounds__(128) m5_relax_cell(int64_t n, M5Consts k,
                                                      const double *__restrict__ Sin,
                                                      double *__restrict__ Sout,
                                                      uint8_t *__restrict__ flag,
+                                                     int32_t *__restrict__ list,
                                                      unsigned *__restrict__ status) {
   using C = K5<N>;
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1270,32 +1272,81 @@ __global__ void __launch_bounds__(128) m5_relax_cell(int64_t n, M5Consts k,
   if (k.plastic) plastic_return<N>(k, s);
   // phi_new[0] exists in the reference only for a solid material 0 (else no trigger)
   const double phi_new = (k.mu[0] != 0.0) ? s[C::i3] - k.avf_lim : phi_old;
-  flag[c] = (phi_old * phi_new < 0.0) ? 1 : 0;
+  const bool crossed = phi_old * phi_new < 0.0;
+  flag[c] = crossed ? 1 : 0;
+  if (crossed) list[1 + atomicAdd(list, 1)] = (int32_t)c;
 #pragma unroll
   for (int e = 0; e < C::NEQ; e++) Sout[(int64_t)e * n + c] = s[e];
   if (st) atomicOr(status, st);
 }
 
+// The flagged cells in leaf order, into sorted (up to GFM_SORT of them) or the list itself: the
+// kernels append them to list[1 ..], count list[0], as they come.  A few are ranked in shared
+// memory; many are collected anew from the flags, which are in leaf order (the fix below takes
+// microseconds per cell, far longer than that pass).
+constexpr int GFM_TPB = 256, GFM_SORT = 2048;
+__device__ const int32_t *flagged_in_order(int64_t n, const uint8_t *flag, int32_t *list, int cnt,
+                                           int32_t *found, int32_t *sorted) {
+  const int t = threadIdx.x;
+  if (cnt <= GFM_SORT) {
+    for (int i = t; i < cnt; i += GFM_TPB) found[i] = list[1 + i];
+    __syncthreads();
+    for (int i = t; i < cnt; i += GFM_TPB) {
+      const int32_t v = found[i];
+      int r = 0;
+      for (int j = 0; j < cnt; j++) r += found[j] < v;
+      sorted[r] = v;
+    }
+    __syncthreads();
+    return sorted;
+  }
+  int32_t at = 1;
+  for (int64_t c0 = 0; c0 < n; c0 += GFM_TPB * 8) {
+    const int64_t c = c0 + (int64_t)t * 8;
+    int mine = 0;
+    for (int i = 0; i < 8; i++) mine += c + i < n && flag[c + i];
+    found[t] = mine;
+    __syncthreads();
+    int before = 0, total = 0;
+    for (int j = 0; j < GFM_TPB; j++) {
+      if (j < t) before += found[j];
+      total += found[j];
+    }
+    for (int i = 0; i < 8; i++)
+      if (c + i < n && flag[c + i]) list[at + before++] = (int32_t)(c + i);
+    at += total;
+    __syncthreads();
+  }
+  return list + 1;
+}
+
 // m5_gfm.c (relax false) / m5_gfm_rel.c (relax true) for the flagged cells, one warp, in
 // leaf order.  A neighbour earlier in leaf order is read from Snew (its final state of this
-// pass), a later one from Sold, as the reference's in-place list walk sees them.
+// pass), a later one from Sold, as the reference's in-place list walk sees them.  One launch of
+// one block, which ends at once where no cell is flagged: a count, a scan and a scatter over all
+// cells before it took 12-15 us of every pass on meshes that the step itself crosses in 80 us.
 template <int N>
-__global__ void __launch_bounds__(32) m5_gfm_seq(ffv_dmesh m, ffv_geom g, M5Consts k,
-                                                 const int32_t *__restrict__ list,
-                                                 const int32_t *__restrict__ count,
-                                                 const double *__restrict__ Sold,
-                                                 double *__restrict__ Snew,
-                                                 const double *__restrict__ SN,
-                                                 const double *__restrict__ RHS,
-                                                 const uint8_t *__restrict__ GF,
-                                                 const double *__restrict__ dtp, int relax) {
+__global__ void __launch_bounds__(GFM_TPB) m5_gfm_seq(ffv_dmesh m, ffv_geom g, M5Consts k,
+                                                      const uint8_t *__restrict__ flag,
+                                                      int32_t *list,
+                                                      const double *__restrict__ Sold,
+                                                      double *__restrict__ Snew,
+                                                      const double *__restrict__ SN,
+                                                      const double *__restrict__ RHS,
+                                                      const uint8_t *__restrict__ GF,
+                                                      const double *__restrict__ dtp, int relax) {
   using C = K5<N>;
   __shared__ double s_phiR[6], s_vel[6][3], s_own[C::NEQ];
+  __shared__ int32_t found[GFM_SORT], sorted[GFM_SORT];
+  const int cnt = list[0];
+  if (cnt == 0) return;
+  const int32_t *cells = flagged_in_order(m.n, flag, list, cnt, found, sorted);
+  if (threadIdx.x == 0) list[0] = 0;  // for the next pass
+  if (threadIdx.x >= 32) return;
   const int lane = threadIdx.x;
-  const int cnt = *count;
   const double DT = *dtp;
   for (int idx = 0; idx < cnt; idx++) {
-    const int64_t c = list[idx];
+    const int64_t c = cells[idx];
     const uint32_t info = m.info[c];
     const int l = ffv_info_level(info);
     if (lane == 0)
@@ -1437,81 +1488,6 @@ __global__ void __launch_bounds__(32) m5_gfm_seq(ffv_dmesh m, ffv_geom g, M5Cons
       for (int e = 0; e < C::NEQ; e++) Snew[(int64_t)e * m.n + c] = s[e];
     }
     __syncwarp();
-  }
-}
-
-// ordered compaction of flag[] into list[] (leaf order kept): per-block counts, one-block
-// exclusive scan, per-block ordered scatter
-constexpr int CB = 1024;
-__global__ void __launch_bounds__(CB) flag_count(int64_t n, const uint8_t *__restrict__ flag,
-                                                 int32_t *__restrict__ bcount) {
-  __shared__ int warp_sum[CB / 32];
-  const int64_t c = (int64_t)blockIdx.x * CB + threadIdx.x;
-  const int f = (c < n) ? flag[c] : 0;
-  const unsigned b = __ballot_sync(0xffffffffu, f);
-  if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = __popc(b);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int s = 0;
-    for (int w = 0; w < CB / 32; w++) s += warp_sum[w];
-    bcount[blockIdx.x] = s;
-  }
-}
-__global__ void __launch_bounds__(CB) flag_scan(int nb, int32_t *__restrict__ bcount,
-                                                int32_t *__restrict__ total) {
-  // single block: sequential carry over chunks of CB, warp-level scans inside
-  __shared__ int warp_tot[CB / 32];
-  __shared__ int carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int base = 0; base < nb; base += CB) {
-    const int i = base + threadIdx.x;
-    const int v = i < nb ? bcount[i] : 0;
-    int x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, x, o);
-      if ((threadIdx.x & 31) >= o) x += y;
-    }
-    if ((threadIdx.x & 31) == 31) warp_tot[threadIdx.x >> 5] = x;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      int t = warp_tot[threadIdx.x];
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, t, o);
-        if (threadIdx.x >= o) t += y;
-      }
-      warp_tot[threadIdx.x] = t;
-    }
-    __syncthreads();
-    const int incl = x + ((threadIdx.x >> 5) ? warp_tot[(threadIdx.x >> 5) - 1] : 0);
-    if (i < nb) bcount[i] = carry + incl - v;
-    __syncthreads();
-    if (threadIdx.x == CB - 1) carry += incl;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *total = carry;
-}
-__global__ void __launch_bounds__(CB) flag_scatter(int64_t n, const uint8_t *__restrict__ flag,
-                                                   const int32_t *__restrict__ boff,
-                                                   int32_t *__restrict__ list) {
-  __shared__ int warp_off[CB / 32];
-  const int64_t c = (int64_t)blockIdx.x * CB + threadIdx.x;
-  const int f = (c < n) ? flag[c] : 0;
-  const unsigned b = __ballot_sync(0xffffffffu, f);
-  if ((threadIdx.x & 31) == 0) warp_off[threadIdx.x >> 5] = __popc(b);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int s = 0;
-    for (int w = 0; w < CB / 32; w++) {
-      const int t = warp_off[w];
-      warp_off[w] = s;
-      s += t;
-    }
-  }
-  __syncthreads();
-  if (f) {
-    const int r = __popc(b & ((1u << (threadIdx.x & 31)) - 1u));
-    list[boff[blockIdx.x] + warp_off[threadIdx.x >> 5] + r] = (int32_t)c;
   }
 }
 
@@ -1811,12 +1787,6 @@ void ffv_m5_cfl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const 
 
 int ffv_m5_neq(int nmat) { return 3 * nmat + 12; }
 
-// kernel names in launch order, for ffv_profile_stage
-static const char *k_names[] = {"m5_recon_slopes", "m5_face_flux",  "m5_cell_update",
-                                "flag_count",    "flag_scan",     "flag_scatter",
-                                "m5_gfm_seq",    "m5_relax_cell", "flag_count",
-                                "flag_scan",     "flag_scatter",  "m5_gfm_seq(relax)"};
-
 struct Rec {
   cudaEvent_t *ev;
   int i;
@@ -1836,7 +1806,6 @@ static void stage_impl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
                        const char **names) {
   const int tpb = 128;
   const unsigned gc = (unsigned)((m.n + tpb - 1) / tpb);
-  const unsigned nb = (unsigned)((m.n + CB - 1) / CB);
   Rec rec{ev, 0, names, st};
   if (ev) cudaEventRecord(ev[0], st);
   const bool f32 = k.precision == FFV_FP32_FLUX, fast = k.flux_form == FFV_FLUX_CONSISTENT;
@@ -1851,7 +1820,7 @@ static void stage_impl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
       rec("m5f_recon_face");
     } else {
       m5_recon_slopes<N><<<dim3(gc, 3), tpb, 0, st>>>(m, g, k, b.S, b.SF);
-      rec(k_names[0]);
+      rec("m5_recon_slopes");
       (fast ? m5_relax_faces<N, true> : m5_relax_faces<N, false>)<<<dim3(gc, 6), tpb, 0, st>>>(
           m.n, k, b.SF, b.status);
       rec("m5_relax_faces");
@@ -1859,54 +1828,33 @@ static void stage_impl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
   }
   if (f32)
     ffv_m5f_flux(m, g, k, b.S, k.order == 2 ? (const float *)b.RHS : nullptr, SFf, FFf, UFf, b.GF,
-                 b.status, st);
+                 b.list_faces, b.status, st);
   else
-    (k.order == 2 ? m5_face_flux<N, 2> : m5_face_flux<N, 1>)<<<dim3(gc, 3), tpb, 0, st>>>(
-        m, g, k, b.S, b.SF, b.FF, b.UF, b.GF, b.status);
-  rec(f32 ? "m5f_face_flux" : k_names[1]);
-  if (b.list_faces.block[12] > 0) {
-    if (f32)
-      ffv_m5f_listed_flux(m, g, k, b.S, k.order == 2 ? (const float *)b.RHS : nullptr, SFf, FFf, UFf,
-                          b.GF, b.list_faces, b.status, st);
-    else
-      (k.order == 2 ? m5_listed_flux<N, 2> : m5_listed_flux<N, 1>)
-          <<<b.list_faces.block[12], FFV_LIST_TPB, 0, st>>>(m, g, k, b.list_faces, b.S, b.SF, b.FF,
-                                                            b.UF, b.GF, b.status);
-  }
-  rec(f32 ? "m5f_listed_flux" : "m5_listed_flux");
+    (k.order == 2 ? m5_face_flux<N, 2> : m5_face_flux<N, 1>)
+        <<<ffv_flux_blocks(b.list_faces, m.n), FFV_LIST_TPB, 0, st>>>(
+            m, g, k, b.list_faces, b.S, b.SF, b.FF, b.UF, b.GF, b.status);
+  rec(f32 ? "m5f_face_flux" : "m5_face_flux");
   if (f32)
-    ffv_m5f_cell_update(m, g, k, b.S, b.SN, FFf, UFf, b.RHS, b.Snew, b.flag, b.dt, irk, b.status,
-                        st);
+    ffv_m5f_cell_update(m, g, k, b.S, b.SN, FFf, UFf, b.RHS, b.Snew, b.flag, b.list, b.dt, irk,
+                        b.status, st);
   else
     m5_cell_update<N><<<gc, tpb, 0, st>>>(m, g, k, b.S, b.SN, b.FF, b.UF, b.RHS, b.Snew,
-                                                  b.flag, b.dt, irk, b.status);
-  rec(f32 ? "m5f_cell_update" : k_names[2]);
+                                          b.flag, b.list, b.dt, irk, b.status);
+  rec(f32 ? "m5f_cell_update" : "m5_cell_update");
   if (irk == 1) {
-    flag_count<<<nb, CB, 0, st>>>(m.n, b.flag, b.bcount);
-    rec(k_names[3]);
-    flag_scan<<<1, CB, 0, st>>>((int)nb, b.bcount, b.count);
-    rec(k_names[4]);
-    flag_scatter<<<nb, CB, 0, st>>>(m.n, b.flag, b.bcount, b.list);
-    rec(k_names[5]);
-    m5_gfm_seq<N><<<1, 32, 0, st>>>(m, g, k, b.list, b.count, b.S, b.Snew, b.SN, b.RHS, b.GF,
-                                    b.dt, 0);
-    rec(k_names[6]);
+    m5_gfm_seq<N><<<1, GFM_TPB, 0, st>>>(m, g, k, b.flag, b.list, b.S, b.Snew, b.SN, b.RHS, b.GF,
+                                         b.dt, 0);
+    rec("m5_gfm_seq");
   }
-  if (f32) ffv_m5f_relax_cell(m.n, k, b.Snew, b.S, b.flag, b.status, st);
+  if (f32) ffv_m5f_relax_cell(m.n, k, b.Snew, b.S, b.flag, b.list, b.status, st);
   else
     (fast ? m5_relax_cell<N, true> : m5_relax_cell<N, false>)<<<gc, tpb, 0, st>>>(
-        m.n, k, b.Snew, b.S, b.flag, b.status);
-  rec(f32 ? "m5f_relax_cell" : k_names[7]);
-  flag_count<<<nb, CB, 0, st>>>(m.n, b.flag, b.bcount);
-  rec(k_names[8]);
-  flag_scan<<<1, CB, 0, st>>>((int)nb, b.bcount, b.count);
-  rec(k_names[9]);
-  flag_scatter<<<nb, CB, 0, st>>>(m.n, b.flag, b.bcount, b.list);
-  rec(k_names[10]);
+        m.n, k, b.Snew, b.S, b.flag, b.list, b.status);
+  rec(f32 ? "m5f_relax_cell" : "m5_relax_cell");
   // relaxed states are in S; a later neighbour is still unrelaxed (Snew)
-  m5_gfm_seq<N><<<1, 32, 0, st>>>(m, g, k, b.list, b.count, b.Snew, b.S, b.SN, b.RHS, b.GF,
-                                  b.dt, 1);
-  rec(k_names[11]);
+  m5_gfm_seq<N><<<1, GFM_TPB, 0, st>>>(m, g, k, b.flag, b.list, b.Snew, b.S, b.SN, b.RHS, b.GF, b.dt,
+                                       1);
+  rec("m5_gfm_seq(relax)");
 }
 
 void ffv_m5_fp64_stage(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
@@ -1918,5 +1866,5 @@ void ffv_m5_fp64_stage(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
 
 int ffv_m5_launches_per_stage(const M5Consts &k, int irk) {
   const int recon = k.order == 2 ? 2 : 0;
-  return recon + 3 + (irk == 1 ? 4 : 0) + 1 + 4;
+  return recon + 2 + (irk == 1 ? 1 : 0) + 2;
 }
