@@ -8,6 +8,7 @@
 #include <new>
 
 #include "ffv_device.cuh"
+#include "ffv_fp64.cuh"
 #include "ffv_m5.cuh"
 
 struct ffv_ctx {
@@ -31,11 +32,13 @@ struct ffv_ctx {
   int32_t *d_flist, *d_flist_own;
   int64_t cap_flist_own;
   ffv_face_list flist;
+  bool symmetric;        // every fine face's coarse neighbour has it among its four (no part mesh)
   int32_t *d_list;       // flagged cells: count, cells [n], and the face list's 12 cursors
   M5Consts m5;
   // refinement tags
-  int32_t *d_SI, *d_SItmp, *d_split;
-  double *d_tagpr;  // per-cell mixture pressure and density for the criterion [2][n]
+  uint32_t *d_SI;
+  int32_t *d_SItmp, *d_split;
+  double *d_tagpr;  // per-cell mixture pressure and density for the criterion, FP64 and FP32 [3][n]
   // cells and subface groups the mesh buffers are allocated for (a new mesh that fits reuses
   // them: a regrid then allocates nothing)
   int64_t cap, cap_nsub;
@@ -81,7 +84,8 @@ void free_mesh_buffers(ffv_ctx *c) {
   cudaFree(c->d_SItmp);
   cudaFree(c->d_split);
   cudaFree(c->d_tagpr);
-  c->d_SI = c->d_SItmp = c->d_split = nullptr;
+  c->d_SI = nullptr;
+  c->d_SItmp = c->d_split = nullptr;
   c->d_tagpr = nullptr;
   c->d_info = nullptr;
   c->d_nbr = c->d_sub = nullptr;
@@ -218,7 +222,7 @@ __global__ void __launch_bounds__(256) list_faces(int64_t n, const uint32_t *__r
 
 // the list of a mesh with count[g] pairs per group, on the context's stream (after its info
 // words are on the device); the ghost-fluid flags of faces nothing evaluates stay zero
-int build_face_list(ffv_ctx *c, const int64_t count[12]) {
+int build_face_list(ffv_ctx *c, const int64_t *count) {
   ffv_face_list &l = c->flist;
   l.off[0] = l.block[0] = 0;
   for (int g = 0; g < 12; g++) {
@@ -553,20 +557,25 @@ int ffv_set_mesh(ffv_ctx *c, const ffv_mesh *m) {
     return FFV_ERR_NOMEM;
   }
   // (and the listed faces per group, for model 5)
-  std::vector<std::array<int64_t, 12>> part((size_t)host_threads());
+  std::vector<std::array<int64_t, 13>> part((size_t)host_threads());
   parallel_chunks(n, host_threads(), [&](int t, int64_t a, int64_t b) {
-    std::array<int64_t, 12> k{};
+    std::array<int64_t, 13> k{};
+    int64_t fine_faces = 0;
     for (int64_t i = a; i < b; i++)
       for (int f = 0; f < 6; f++) {
         nbr_t[(int64_t)f * n + i] = m->nbr[6 * i + f];
         const uint32_t kind = ffv_face_kind(m->info[i], f);
         if (kind != FFV_FK_SAME) k[2 * f + (kind == FFV_FK_FINER)]++;
+        fine_faces += kind == FFV_FK_COARSER;
       }
+    k[12] = fine_faces;
     part[t] = k;
   });
-  int64_t listed[12] = {};
+  int64_t listed[13] = {}, finer = 0;
   for (const auto &k : part)
-    for (int g = 0; g < 12; g++) listed[g] += k[g];
+    for (int g = 0; g < 13; g++) listed[g] += k[g];
+  for (int g = 1; g < 12; g += 2) finer += listed[g];
+  c->symmetric = listed[12] == 4 * finer;
   cudaError_t e = cudaMemcpy(c->d_info, m->info, sizeof(uint32_t) * n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaMemcpy(c->d_nbr, nbr_t, sizeof(int32_t) * 6 * n, cudaMemcpyHostToDevice);
@@ -691,8 +700,13 @@ __global__ void __launch_bounds__(kSumThreads) sum_partials(ffv_dmesh m, ffv_geo
   for (int v = 0; v < neq; v++) {
     double acc = 0.0;
     for (int64_t c = (int64_t)blockIdx.x * kSumThreads + threadIdx.x; c < m.n;
-         c += (int64_t)gridDim.x * kSumThreads)
-      acc += fabs(g.vol[ffv_info_level(m.info[c])]) * S[(int64_t)v * m.n + c];
+         c += (int64_t)gridDim.x * kSumThreads) {
+      // one FP64 instruction per value (the product is exact where the volume is a power of two;
+      // an absolute value is one too, so its bit is cleared instead)
+      const int l = ffv_info_level(m.info[c]);
+      const double x = S[(int64_t)v * m.n + c];
+      acc = fma(f64::of_bits(f64::abs_bits(g.vol[l])), x, acc);
+    }
     red[threadIdx.x] = acc;
     __syncthreads();
     for (int o = kSumThreads / 2; o > 0; o >>= 1) {
@@ -800,6 +814,8 @@ int tags_device(ffv_ctx *c, const ffv_mesh *m, const ffv_tag_params *p, int32_t 
   t.si_max = 0;
   if (p->inter0 == 1 && p->inter1 == 1) t.si_max = t.lrs0 + t.lrs1;
   if (p->inter0 == 1 && p->inter1 == 0) t.si_max = t.lrs0;
+  // layers are kept in 16 bits: more than a forest of FFV_MAX_LEVEL levels is wide
+  if (t.si_max > 65536) t.si_max = 65536;
   // inputset.c:106, m5_input.c:53
   int32_t lmax = p->lvl_uniform;
   for (int32_t l : {p->lvl_prs, p->lvl_rho, p->lvl_vel, p->lvl_inter0, p->lvl_inter1})
@@ -809,24 +825,26 @@ int tags_device(ffv_ctx *c, const ffv_mesh *m, const ffv_tag_params *p, int32_t 
   const int64_t n = c->n;
   if (!c->d_split) {  // sized for the mesh buffers' capacity, kept while meshes fit
     const int64_t cap = c->cap;
-    if (cudaMalloc(&c->d_SI, sizeof(int32_t) * 2 * cap) != cudaSuccess ||
-        cudaMalloc(&c->d_SItmp, sizeof(int32_t) * 2 * cap) != cudaSuccess ||
+    if (cudaMalloc(&c->d_SI, sizeof(uint32_t) * cap) != cudaSuccess ||
+        cudaMalloc(&c->d_SItmp, sizeof(int32_t) * (2 * cap + 3)) != cudaSuccess ||
         cudaMalloc(&c->d_split, sizeof(int32_t) * cap) != cudaSuccess ||
-        cudaMalloc(&c->d_tagpr, sizeof(double) * 2 * cap) != cudaSuccess) {
+        cudaMalloc(&c->d_tagpr, sizeof(double) * 3 * cap) != cudaSuccess) {
       cudaFree(c->d_SI);
       cudaFree(c->d_SItmp);
       cudaFree(c->d_split);
       cudaFree(c->d_tagpr);
-      c->d_SI = c->d_SItmp = c->d_split = nullptr;
+      c->d_SI = nullptr;
+  c->d_SItmp = c->d_split = nullptr;
       c->d_tagpr = nullptr;
       return FFV_ERR_NOMEM;
     }
   }
   if (c->p.model == 5) {
-    ffv_m5_tags(c->dm, c->m5, t, c->d_S, c->d_SI, c->d_SItmp, c->d_split, c->d_tagpr, c->stream);
+    ffv_m5_tags(c->dm, c->m5, t, c->symmetric, c->d_S, c->d_SI, c->d_SItmp, c->d_split, c->d_tagpr,
+                c->stream);
   } else {
     ffv_m0_tags(c->dm, c->p.gamma[0], c->p.pinf[0], t, c->d_S, c->d_split, c->stream);
-    CK(cudaMemsetAsync(c->d_SI, 0, sizeof(int32_t) * 2 * n, c->stream));
+    CK(cudaMemsetAsync(c->d_SI, 0, sizeof(uint32_t) * n, c->stream));
   }
   CK(cudaGetLastError());
   return FFV_OK;
@@ -855,8 +873,12 @@ int ffv_tags(ffv_ctx *c, const ffv_mesh *m, const ffv_tag_params *p, int32_t *sp
   if (rc != FFV_OK) return rc;
   const int64_t n = c->n;
   CK(cudaMemcpyAsync(split, c->d_split, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, c->stream));
-  if (si)
-    CK(cudaMemcpyAsync(si, c->d_SI, sizeof(int32_t) * 2 * n, cudaMemcpyDeviceToHost, c->stream));
+  if (si) {
+    // the lists' space is free once the split levels are formed
+    ffv_m5_si_unpack(n, c->d_SI, c->d_SItmp, c->stream);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(si, c->d_SItmp, sizeof(int32_t) * 2 * n, cudaMemcpyDeviceToHost, c->stream));
+  }
   CK(cudaStreamSynchronize(c->stream));
   if (split_raw) memcpy(split_raw, split, sizeof(int32_t) * n);
   return ffv_tags_smooth(m, level_max, split);
@@ -884,8 +906,12 @@ int ffv_tags_raw(ffv_ctx *c, const ffv_mesh *m, const ffv_tag_params *p, int32_t
   const int64_t n = c->n;
   CK(cudaMemcpyAsync(split_raw, c->d_split, sizeof(int32_t) * n, cudaMemcpyDeviceToHost,
                      c->stream));
-  if (si)
-    CK(cudaMemcpyAsync(si, c->d_SI, sizeof(int32_t) * 2 * n, cudaMemcpyDeviceToHost, c->stream));
+  if (si) {
+    // the lists' space is free once the split levels are formed
+    ffv_m5_si_unpack(n, c->d_SI, c->d_SItmp, c->stream);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(si, c->d_SItmp, sizeof(int32_t) * 2 * n, cudaMemcpyDeviceToHost, c->stream));
+  }
   CK(cudaStreamSynchronize(c->stream));
   return FFV_OK;
 }

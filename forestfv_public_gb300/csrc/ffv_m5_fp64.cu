@@ -55,6 +55,26 @@ struct Elastic {
   bool solid;
 };
 
+// (1 + t)^a for |t| <= 1/32, a a unit fraction: 1 + t P(t), P the binomial series to t^9 (the first
+// omitted term is below 3e-18), rounded once
+template <int INV>
+__device__ __forceinline__ double root_near_one(double t) {
+  constexpr double a = 1.0 / INV;
+  constexpr double c1 = a, c2 = c1 * (a - 1) / 2, c3 = c2 * (a - 2) / 3, c4 = c3 * (a - 3) / 4,
+                   c5 = c4 * (a - 4) / 5, c6 = c5 * (a - 5) / 6, c7 = c6 * (a - 6) / 7,
+                   c8 = c7 * (a - 7) / 8, c9 = c8 * (a - 8) / 9, c10 = c9 * (a - 9) / 10;
+  double r = fma(c10, t, c9);
+  r = fma(r, t, c8);
+  r = fma(r, t, c7);
+  r = fma(r, t, c6);
+  r = fma(r, t, c5);
+  r = fma(r, t, c4);
+  r = fma(r, t, c3);
+  r = fma(r, t, c2);
+  r = fma(r, t, c1);
+  return fma(r, t, 1.0);
+}
+
 __device__ __forceinline__ void elastic_of(const M5Consts &k, const double A[9], Elastic &e) {
   e.solid = false;
   if (k.nsolids == 0 || no_deformation(A)) return;
@@ -73,8 +93,17 @@ __device__ __forceinline__ void elastic_of(const M5Consts &k, const double A[9],
   e.G[5] = G5;
   if (f64::abs_bits(Gmag) == 0) return;
   e.solid = true;
-  e.p13 = pow(fabs(Gmag), 1.0 / 3.0);
-  e.p16 = pow(fabs(Gmag), 1.0 / 6.0);
+  // a solid's determinant is within its volume strain of 1: the consistent flux form, which has no
+  // reference to equal bit for bit, takes the series instead of two powers of ~90 instructions
+  // each (wall mesh of 0.41 M cells, 45 % of them solid)
+  const double t = Gmag - 1.0;
+  if (k.flux_form == FFV_FLUX_CONSISTENT && f64::abs_bits(t) <= 0x3fa0000000000000ull) {
+    e.p13 = root_near_one<3>(t);
+    e.p16 = root_near_one<6>(t);
+  } else {
+    e.p13 = pow(fabs(Gmag), 1.0 / 3.0);
+    e.p16 = pow(fabs(Gmag), 1.0 / 6.0);
+  }
 }
 
 // state_equation.c:269-317 and :217-267
@@ -1491,20 +1520,73 @@ __global__ void __launch_bounds__(GFM_TPB) m5_gfm_seq(ffv_dmesh m, ffv_geom g, M
   }
 }
 
-// CFL (new, the reference has a fixed DT): dt = h / (max_a |u_a| + c), mixture sound
-// speed c = sqrt(sum_k c2Y_k) as m5_wave_speeds.c:43-50 forms it
+// CFL (new, the reference has a fixed DT): dt = h / (max_a |u_a| + c), mixture sound speed
+// c^2 = sum_k (alpha_k / rho) gamma_k (p_k + p_inf_k) as m5_wave_speeds.c:43-50 forms it.  With the
+// pressure put in, alpha_k (p_k + p_inf_k) = (gamma_k - 1) (alpha rho e_k - e_el - alpha_k p_inf_k)
+// needs no division by a fraction; at a power-of-two spacing the smallest dt is the reciprocal of
+// the largest speed over h.  A cell whose speed, formed in FP32 without the elastic energy (which
+// only lowers it), is below the thread's largest so far by more than FP32's error is passed over.
+// The rest are bound by the FP64 pipe: 360 -> 119 us at 0.61 M cells of the wall mesh.
 template <int N>
 __global__ void m5_cfl_kernel(ffv_dmesh m, ffv_geom g, M5Consts k, const double *__restrict__ S,
                               unsigned long long *out) {
+  using C = K5<N>;
   double best = INFINITY;
+  uint64_t fastest = 0;  // bits of the largest speed / h (NaN above all)
   for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < m.n;
        c += (int64_t)gridDim.x * blockDim.x) {
-    double s[K5<N>::NEQ];
+    double s[C::NEQ];
     load_state<N>(S, m.n, c, s);
-    Sol<N> q;
-    make_sol<N>(k, s, 0.0, false, q);
-    const double sp = fmax(fmax(fabs(q.u), fabs(q.v)), fabs(q.w)) + sqrt(q.c2);
-    const double dt = g.h[ffv_info_level(m.info[c])] / sp;
+    const int l = ffv_info_level(m.info[c]);
+    const bool scaled = (g.pow2 >> l) & 1u;
+    if (scaled && fastest) {
+      float rf = 0.0f, cf = 0.0f, uf = 0.0f, rest = 1.0f;
+      bool inside = true;  // no fraction that the limits below would move by more than rounding
+#pragma unroll
+      for (int i = 0; i < N; ++i) rf += f32_of_f64(s[i]);
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const float a = i < N - 1 ? f32_of_f64(s[C::i3 + (i < N - 1 ? i : 0)]) : rest;
+        inside &= a >= 0.0f && a <= 1.0f;
+        rest -= a;
+        cf += k.gamma_f[i] * (k.gamma_f[i] - 1.0f) * (f32_of_f64(s[C::i4 + i]) - a * k.pinf_f[i]);
+      }
+#pragma unroll
+      for (int d = 0; d < 3; d++) uf = fmaxf(uf, fabsf(f32_of_f64(s[C::i1 + d])));
+      // the last fraction is 1 - sum: next to 1 FP32 resolves it to 2e-7, against p_inf up to the
+      // energy's own size
+      const float bound = (uf / rf + sqrtf(cf / rf * 1.001f)) * g.idcc_f[l][0] * 1.001f;
+      if (inside && bound < f32_of_f64(f64::of_bits(fastest))) continue;  // (not where either is NaN)
+    }
+    double r = s[0];
+#pragma unroll
+    for (int i = 1; i < N; ++i) r += s[i];
+    const f64::Rcp rr = f64::rcp(r);
+    avf_limit<N>(k, s);
+    double last = 1.0 - s[C::i3];
+    if (N > 2) last = 1.0 - (s[C::i3] + s[C::i3 + 1]);
+    Elastic el;
+    elastic_of(k, s + C::i5, el);
+    double sum = 0.0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const double a = i < N - 1 ? s[C::i3 + (i < N - 1 ? i : 0)] : last;
+      sum += k.gamma[i] * k.gm1[i] * ((s[C::i4 + i] - elastic_energy(el, k.mu[i])) - a * k.pinf[i]);
+    }
+    uint64_t um = 0;
+#pragma unroll
+    for (int d = 0; d < 3; d++) um = um > f64::abs_bits(s[C::i1 + d]) ? um : f64::abs_bits(s[C::i1 + d]);
+    const double sp = f64::of_bits(f64::abs_bits(f64::div(f64::of_bits(um), rr))) + sqrt(f64::div(sum, rr));
+    if (scaled) {
+      const uint64_t v = f64::bits(sp * g.rdcc[l][0]);
+      fastest = v > fastest ? v : fastest;  // a speed is not negative; NaN sorts above infinity
+    } else {
+      const double dt = g.h[l] / sp;
+      best = (dt < best || isnan(dt)) ? dt : best;
+    }
+  }
+  if (fastest) {
+    const double dt = 1.0 / f64::of_bits(fastest);
     best = (dt < best || isnan(dt)) ? dt : best;
   }
   for (int o = 16; o > 0; o >>= 1) {
@@ -1519,27 +1601,6 @@ __global__ void m5_cfl_kernel(ffv_dmesh m, ffv_geom g, M5Consts k, const double 
 }
 
 // ------------------------------------------------------------------ refinement tags
-// phi[v] of a cell (m5_facevalues.c:83-99): the clamped volume fractions against AVF_LIM
-// (phi[0] the larger of two solids' fractions when there are two)
-template <int N>
-__device__ __forceinline__ void cell_phi(const M5Consts &k, const double *__restrict__ S,
-                                         int64_t n, int64_t c, double phi[2]) {
-  using C = K5<N>;
-  const double lo = k.amin / 100.0, hi = 1.0 - (k.amin / 100.0);
-  double ac[2] = {0.0, 0.0};
-#pragma unroll
-  for (int i = 0; i < N - 1; ++i) {
-    double a = S[(int64_t)(C::i3 + i) * n + c];
-    if (a <= lo) a = lo;
-    else if (a >= hi) a = hi;
-    ac[i] = a;
-  }
-  phi[0] = ac[0] - k.avf_lim;
-  phi[1] = ac[1] - k.avf_lim;
-  if (N > 2 && k.nsolids == 2 && k.mu[0] != 0.0)
-    phi[0] = ((ac[0] > ac[1]) ? ac[0] : ac[1]) - k.avf_lim;
-}
-
 // neighbour q (< count) of cell c across face f; count 0 for boundary faces
 __device__ __forceinline__ int face_neighbours(const ffv_dmesh &m, int64_t c, uint32_t info, int f,
                                                int64_t nb[4]) {
@@ -1555,59 +1616,181 @@ __device__ __forceinline__ int face_neighbours(const ffv_dmesh &m, int64_t c, ui
   return 1;
 }
 
-// interface_location.c:17-46: SI = 1 where phi changes sign across a face (the face loop
-// stops after the first face that shows a change)
+// the sign of phi[v], v = 0, 1 (m5_facevalues.c:83-99): the clamped volume fractions against AVF_LIM
+// (phi[0] the larger of two solids' fractions when there are two); two bits each: 0 below, 1 equal
+// (or NaN), 2 above
+__device__ __forceinline__ uint32_t phi_code(double a, double lim) {
+  const int64_t x = f64::order_key(a + 0.0), y = f64::order_key(lim + 0.0);  // (-0 as +0)
+  return f64::is_nan(a) || x == y ? 1u : (x < y ? 0u : 2u);
+}
+// What the criterion reads of every cell, made once: the signs of phi, the density and (where a
+// pressure criterion is on) the alpha-weighted pressure sum_k alpha_k p_k from the reference's cell
+// primitives (make_sol of the cell state), each also rounded to FP32 for the jumps' screen.
+struct TagCells {
+  double *pr, *rho;
+  float *pr_f, *rho_f;
+  uint8_t *phi;
+};
 template <int N>
-__global__ void __launch_bounds__(128) m5_si_first(ffv_dmesh m, M5Consts k,
-                                                   const double *__restrict__ S,
-                                                   int32_t *__restrict__ SI) {
+__global__ void __launch_bounds__(128) m5_tag_cells(int64_t n, M5Consts k, bool prs, bool rho,
+                                                    const double *__restrict__ S, TagCells t) {
+  using C = K5<N>;
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= m.n) return;
-  const uint32_t info = m.info[c];
-  double pl[2], pr[2];
-  cell_phi<N>(k, S, m.n, c, pl);
-  int si0 = 0, si1 = 0;
-  bool hit = false;
-  for (int f = 0; f < 6 && !hit; f++) {
-    int64_t nb[4];
-    const int cnt = face_neighbours(m, c, info, f, nb);
-    for (int q = 0; q < cnt; q++) {
-      cell_phi<N>(k, S, m.n, nb[q], pr);
-      for (int v = 0; v < N - 1; ++v)
-        if (pl[v] * pr[v] < 0.0) {
-          if (v == 0) si0 = 1;
-          else si1 = 1;
-          hit = true;
-        }
-    }
+  if (c >= n) return;
+  const double a0 = clamp_vf(k, S[(int64_t)C::i3 * n + c]);
+  uint32_t code;
+  if (N > 2) {
+    const double a1 = clamp_vf(k, S[(int64_t)(C::i3 + 1) * n + c]);
+    code = phi_code(k.nsolids == 2 && k.mu[0] != 0.0 && a0 <= a1 ? a1 : a0, k.avf_lim) |
+           phi_code(a1, k.avf_lim) << 2;
+  } else {
+    code = phi_code(a0, k.avf_lim) | 1u << 2;
   }
-  SI[c] = si0;
-  SI[m.n + c] = si1;
+  t.phi[c] = (uint8_t)code;
+  if (prs) {
+    double s[C::NEQ];
+    load_state<N>(S, n, c, s);
+    Sol<N> q;
+    make_sol<N>(k, s, 0.0, false, q);
+    double p = 0.0;
+#pragma unroll
+    for (int iv = 0; iv < N; ++iv) p += q.avf[iv] * q.p[iv];
+    t.pr[c] = p;
+    t.pr_f[c] = f32_of_f64(p);
+  }
+  if (rho) {
+    double r = S[c];
+#pragma unroll
+    for (int i = 1; i < N; ++i) r += S[(int64_t)i * n + c];
+    t.rho[c] = r;
+    t.rho_f[c] = f32_of_f64(r);
+  }
 }
 
-// interface_location.c:52-80: layer lvl next to layer lvl - 1.  The reference updates in
-// place in leaf order, but a cell only reads neighbours' lvl - 1 entries and only writes
-// lvl into entries that were 0, so reading the previous layer's copy gives the same result.
-__global__ void __launch_bounds__(128) m5_si_layer(ffv_dmesh m, int lvl,
-                                                   const int32_t *__restrict__ SIin,
-                                                   int32_t *__restrict__ SIout) {
+// Interface layers: one word per cell, SI[0] in its low half, SI[1] in the high one.
+
+// what the neighbours across a face show: hit(neighbour) of any of them, bit v for SI[v]
+template <typename Hit>
+__device__ __forceinline__ int face_shows(const ffv_dmesh &m, uint32_t kind, int32_t nb, Hit hit) {
+  if (kind & FFV_FK_BC) return 0;
+  if (kind != FFV_FK_FINER) return hit(nb);
+  const int4 s = *reinterpret_cast<const int4 *>(m.sub + 4 * (int64_t)nb);
+  return hit(s.x) | hit(s.y) | hit(s.z) | hit(s.w);
+}
+// the first face (in order) that shows any bit of `want`: its bits.  All six faces' loads are in
+// flight together.
+template <typename Hit>
+__device__ __forceinline__ int first_face(const ffv_dmesh &m, int64_t c, int want, Hit hit) {
+  const uint32_t info = m.info[c];
+  int32_t nb[6];
+#pragma unroll
+  for (int f = 0; f < 6; f++) nb[f] = m.nbr[(int64_t)f * m.n + c];
+  int shows[6];
+#pragma unroll
+  for (int f = 0; f < 6; f++) shows[f] = face_shows(m, ffv_face_kind(info, f), nb[f], hit);
+  int set = 0;
+#pragma unroll
+  for (int f = 0; f < 6; f++)
+    if (set == 0) set = shows[f] & want;
+  return set;
+}
+
+// interface_location.c:17-46: SI = 1 where phi changes sign across a face (the face loop
+// stops after the first face that shows a change); those cells are listed (list nullable)
+__global__ void __launch_bounds__(128) m5_si_first(ffv_dmesh m, const uint8_t *__restrict__ phi,
+                                                   uint32_t *__restrict__ SI,
+                                                   int32_t *__restrict__ list,
+                                                   int32_t *__restrict__ count) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  int set = 0;
+  if (c < m.n) {
+    const uint32_t own = phi[c];
+    set = first_face(m, c, 3, [&](int32_t o) {
+      const uint32_t x = own ^ phi[o];
+      return ((x & 3u) == 2u ? 1 : 0) | ((x >> 2) == 2u ? 2 : 0);
+    });
+    SI[c] = (set & 1) | (uint32_t)(set >> 1) << 16;
+  }
+  if (!list) return;
+  const unsigned b = __ballot_sync(0xffffffffu, set != 0);
+  if (b == 0) return;
+  const int lane = threadIdx.x & 31;
+  int at = 0;
+  if (lane == 0) at = atomicAdd(count, __popc(b));
+  at = __shfl_sync(0xffffffffu, at, 0);
+  if (set) list[at + __popc(b & ((1u << lane) - 1u))] = (int32_t)c;
+}
+
+// interface_location.c:52-80 for one cell: what layer lvl sets in it (bit v), from its
+// neighbours' layer lvl - 1.  The reference updates in place in leaf order, but a cell only reads
+// neighbours' lvl - 1 entries and only writes lvl into entries that were 0, so updating in place in
+// any order gives the same result (an entry that already is lvl was 0 before this layer).
+__device__ __forceinline__ int si_free(uint32_t w, int lvl) {
+  const int s0 = w & 0xffff, s1 = w >> 16;
+  return (s0 == 0 || s0 == lvl ? 1 : 0) | (s1 == 0 || s1 == lvl ? 2 : 0);
+}
+__device__ __forceinline__ int si_is(uint32_t w, int lvl) {
+  return ((int)(w & 0xffff) == lvl ? 1 : 0) | ((int)(w >> 16) == lvl ? 2 : 0);
+}
+__device__ __forceinline__ int si_set(const ffv_dmesh &m, int lvl, const uint32_t *SI, int64_t c,
+                                      int free) {
+  return first_face(m, c, free, [&](int32_t o) { return si_is(__ldcg(SI + o), lvl - 1); });
+}
+__device__ __forceinline__ uint32_t si_word(int set, int lvl) {
+  return (set & 1 ? (uint32_t)lvl : 0u) | (set & 2 ? (uint32_t)lvl << 16 : 0u);
+}
+
+// Layer lvl from the cells that layer lvl - 1 set: only their neighbours can be next to it.  A
+// neighbour of several is evaluated by each, with the same outcome; the one that sets its first
+// entry lists it for the next layer.  Bound by the latency of its chain of loads, so every SM is
+// filled.  The criterion's device part (cells, fourteen layers, split) took ~2.9 ms on the wall mesh
+// of 2.5 M cells with every layer over all cells and FP64 jumps and signs; now ~0.8 ms.
+__global__ void __launch_bounds__(128) m5_si_grow(ffv_dmesh m, int lvl, uint32_t *SI,
+                                                  const int32_t *__restrict__ from,
+                                                  int32_t *__restrict__ to, int32_t *count) {
+  const int n_from = count[(lvl - 1) % 3];
+  if (blockIdx.x == 0 && threadIdx.x == 0) count[(lvl + 1) % 3] = 0;  // the next layer's
+  // eight threads per cell: six faces
+  const int face = threadIdx.x & 7;
+  if (face >= 6) return;
+  for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3; i < n_from;
+       i += ((int64_t)gridDim.x * blockDim.x) >> 3) {
+    const int64_t b = from[i];
+    const int mine = si_is(__ldcg(SI + b), lvl - 1);
+    const auto visit = [&](int32_t c) {
+      const int free = si_free(__ldcg(SI + c), lvl);
+      if (!(free & mine)) return 0;
+      const int set = si_set(m, lvl, SI, c, free);
+      if (!set) return 0;
+      const uint32_t before = atomicOr(SI + c, si_word(set, lvl));
+      // the first of its visitors to set its first entry
+      if ((before & (set & 1 ? 0xffffu : 0xffff0000u)) == 0) to[atomicAdd(count + lvl % 3, 1)] = c;
+      return 0;
+    };
+    face_shows(m, ffv_face_kind(m.info[b], face), m.nbr[(int64_t)face * m.n + b], visit);
+  }
+}
+
+// layer lvl over all cells: meshes whose neighbour relation is not symmetric (a part of a forest:
+// a fine cell sees a coarser one whose own face towards it became a boundary)
+__global__ void __launch_bounds__(128) m5_si_layer(ffv_dmesh m, int lvl, uint32_t *SI) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.n) return;
-  const uint32_t info = m.info[c];
-  int s[2] = {SIin[c], SIin[m.n + c]};
-  bool hit = false;
-  for (int f = 0; f < 6 && !hit; f++) {
-    int64_t nb[4];
-    const int cnt = face_neighbours(m, c, info, f, nb);
-    for (int q = 0; q < cnt; q++)
-      for (int v = 0; v < 2; ++v)
-        if (SIin[(int64_t)v * m.n + nb[q]] == lvl - 1 && s[v] == 0) {
-          s[v] = lvl;
-          hit = true;
-        }
-  }
-  SIout[c] = s[0];
-  SIout[m.n + c] = s[1];
+  const uint32_t w = SI[c];
+  const int free = si_free(w, lvl);
+  if (free == 0) return;
+  const int set = si_set(m, lvl, SI, c, free);
+  if (set) SI[c] = w | si_word(set, lvl);
+}
+
+// the layers as two arrays
+__global__ void __launch_bounds__(256) m5_si_unpack(int64_t n, const uint32_t *__restrict__ SI,
+                                                    int32_t *__restrict__ out) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  const uint32_t w = SI[c];
+  out[c] = (int32_t)(w & 0xffff);
+  out[n + c] = (int32_t)(w >> 16);
 }
 
 // relative jump |x_nb - x| / max(|x_nb|, |x|) (criterionsplt.c:83-89), 0 below 1e-8
@@ -1620,32 +1803,25 @@ __device__ __forceinline__ double rel_jump(double x_cur, double x_nb) {
   return 0.0;
 }
 
-// each cell's alpha-weighted pressure sum_k alpha_k p_k and density, from the reference's cell
-// primitives (make_sol of the cell state): computed once per cell here, read by every
-// neighbour's criterion below (the same doubles the per-neighbour evaluation gave)
-template <int N>
-__global__ void __launch_bounds__(128) m5_tag_prims(int64_t n, M5Consts k,
-                                                    const double *__restrict__ S,
-                                                    double *__restrict__ pr) {
-  using C = K5<N>;
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  double s[C::NEQ];
-  load_state<N>(S, n, c, s);
-  Sol<N> q;
-  make_sol<N>(k, s, 0.0, false, q);
-  double p = 0.0;
-#pragma unroll
-  for (int iv = 0; iv < N; ++iv) p += q.avf[iv] * q.p[iv];
-  pr[c] = p;
-  pr[n + c] = q.r;
+// Whether a neighbour's jump reaches the threshold.  The FP32 values decide where the jump is not
+// within 1e-6 of it -- their rounding moves the ratio by less than 3e-7 -- and the magnitudes are
+// ordinary; the rest take the FP64 expression.
+__device__ __forceinline__ bool jump_reaches(double thr, float thr_f, const double *x,
+                                             const float *xf, int64_t c, int64_t o) {
+  const float a = xf[c], b = xf[o];
+  const float d = fabsf(b - a), big = fmaxf(fabsf(a), fabsf(b));
+  if (big > 1e-6f && big < 1e30f) {
+    if (d > (thr_f + 1e-6f) * big) return true;
+    if (d < (thr_f - 1e-6f) * big) return false;
+  }
+  return rel_jump(x[c], x[o]) >= thr;
 }
 
 // criterionsplt.c:3-140 per cell: the uniform level, the gradient criterion over every
-// sub-neighbour and the interface layers
-__global__ void __launch_bounds__(128) m5_tag_split(ffv_dmesh m, ffv_m5_tagc t,
-                                                    const double *__restrict__ pr,
-                                                    const int32_t *__restrict__ SI,
+// sub-neighbour (largest jump against the threshold: any neighbour's reaches it) and the interface
+// layers
+__global__ void __launch_bounds__(128) m5_tag_split(ffv_dmesh m, ffv_m5_tagc t, TagCells x,
+                                                    const uint32_t *__restrict__ SI,
                                                     int32_t *__restrict__ split) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.n) return;
@@ -1653,34 +1829,29 @@ __global__ void __launch_bounds__(128) m5_tag_split(ffv_dmesh m, ffv_m5_tagc t,
   if (t.uniform == 1) level = level > t.lvl_uniform ? level : t.lvl_uniform;
   if (t.prs == 1 || t.rho == 1 || t.vel == 1) {
     const uint32_t info = m.info[c];
-    const double pL = pr[c], rL = pr[m.n + c];
-    double gp = 0.0, gr = 0.0, gv = 0.0;
+    // (no neighbour jumps by less than zero: a threshold at or below it is always reached)
+    bool hp = 0.0 >= t.thr_prs, hr = 0.0 >= t.thr_rho, hv = 0.0 >= t.thr_vel;
+    const float fp = (float)t.thr_prs, fr = (float)t.thr_rho, fv = (float)t.thr_vel;
     for (int f = 0; f < 6; f++) {
       int64_t nb[4];
       const int cnt = face_neighbours(m, c, info, f, nb);
       for (int q = 0; q < cnt; q++) {
-        if (t.prs == 1) {
-          const double g = rel_jump(pL, pr[nb[q]]);
-          gp = (g > gp) ? g : gp;
-        }
-        double grho = 0.0;
-        if (t.rho == 1) {
-          grho = rel_jump(rL, pr[m.n + nb[q]]);
-          gr = (grho > gr) ? grho : gr;
-        }
-        // the reference's velocity criterion takes the density jump (criterionsplt.c:120)
-        if (t.vel == 1) gv = (grho > gv) ? grho : gv;
+        if (t.prs == 1 && !hp) hp = jump_reaches(t.thr_prs, fp, x.pr, x.pr_f, c, nb[q]);
+        if (t.rho == 1 && !hr) hr = jump_reaches(t.thr_rho, fr, x.rho, x.rho_f, c, nb[q]);
+        // the reference's velocity criterion takes the density jump (criterionsplt.c:120), which
+        // it has where the density criterion is on
+        if (t.vel == 1 && t.rho == 1 && !hv) hv = jump_reaches(t.thr_vel, fv, x.rho, x.rho_f, c, nb[q]);
       }
     }
     int lt = 1;
-    if (t.prs == 1 && fabs(gp) >= t.thr_prs) lt = t.lvl_prs;
-    if (t.rho == 1 && fabs(gr) >= t.thr_rho) lt = t.lvl_rho;
-    if (t.vel == 1 && fabs(gv) >= t.thr_vel) lt = t.lvl_vel;
+    if (t.prs == 1 && hp) lt = t.lvl_prs;
+    if (t.rho == 1 && hr) lt = t.lvl_rho;
+    if (t.vel == 1 && hv) lt = t.lvl_vel;
     level = level > lt ? level : lt;
   }
   if (t.inter0 != 0) {
     for (int v = 0; v < 2; ++v) {
-      const int si = SI[(int64_t)v * m.n + c];
+      const int si = (int)(v ? SI[c] >> 16 : SI[c] & 0xffff);
       if (si >= 1 && si < t.lrs0) level = level > t.lvl0 ? level : t.lvl0;
       if (si >= t.lrs0 && si < t.lrs1) level = level > t.lvl1 ? level : t.lvl1;
     }
@@ -1759,24 +1930,35 @@ void ffv_m5_export_fields(int64_t n, const M5Consts &k, const double *S, double 
   else m5_export_fields<3><<<gc, 128, 0, st>>>(n, k, S, F);
 }
 
-void ffv_m5_tags(const ffv_dmesh &m, const M5Consts &k, const ffv_m5_tagc &t, const double *S,
-                 int32_t *SI, int32_t *SItmp, int32_t *split, double *pr, cudaStream_t st) {
+void ffv_m5_tags(const ffv_dmesh &m, const M5Consts &k, const ffv_m5_tagc &t, bool symmetric,
+                 const double *S, uint32_t *SI, int32_t *lists, int32_t *split, double *pr,
+                 cudaStream_t st) {
   const unsigned gc = (unsigned)((m.n + 127) / 128);
+  // pr: pressure, density [n] doubles each, then both as floats; the phi codes wait in split
+  float *f = reinterpret_cast<float *>(pr + 2 * m.n);
+  const TagCells x{pr, pr + m.n, f, f + m.n, reinterpret_cast<uint8_t *>(split)};
+  const bool prs = t.prs == 1, rho = t.rho == 1 || t.vel == 1;
+  if (t.inter0 != 0 || prs || rho) {
+    if (k.nmat == 2) m5_tag_cells<2><<<gc, 128, 0, st>>>(m.n, k, prs, rho, S, x);
+    else m5_tag_cells<3><<<gc, 128, 0, st>>>(m.n, k, prs, rho, S, x);
+  }
   if (t.inter0 != 0) {
-    if (k.nmat == 2) m5_si_first<2><<<gc, 128, 0, st>>>(m, k, S, SI);
-    else m5_si_first<3><<<gc, 128, 0, st>>>(m, k, S, SI);
+    // two lists of at most n cells and the counts of three layers
+    int32_t *list[2] = {lists, lists + m.n}, *count = lists + 2 * m.n;
+    cudaMemsetAsync(count, 0, 3 * sizeof(int32_t), st);
+    m5_si_first<<<gc, 128, 0, st>>>(m, x.phi, SI, symmetric ? list[1] : nullptr, count + 1);
     for (int lvl = 2; lvl < t.si_max; lvl++) {
-      cudaMemcpyAsync(SItmp, SI, sizeof(int32_t) * 2 * m.n, cudaMemcpyDeviceToDevice, st);
-      m5_si_layer<<<gc, 128, 0, st>>>(m, lvl, SItmp, SI);
+      if (symmetric) m5_si_grow<<<152 * 16, 128, 0, st>>>(m, lvl, SI, list[(lvl - 1) & 1], list[lvl & 1], count);
+      else m5_si_layer<<<gc, 128, 0, st>>>(m, lvl, SI);
     }
   } else {
-    cudaMemsetAsync(SI, 0, sizeof(int32_t) * 2 * m.n, st);
+    cudaMemsetAsync(SI, 0, sizeof(uint32_t) * m.n, st);
   }
-  if (t.prs == 1 || t.rho == 1 || t.vel == 1) {
-    if (k.nmat == 2) m5_tag_prims<2><<<gc, 128, 0, st>>>(m.n, k, S, pr);
-    else m5_tag_prims<3><<<gc, 128, 0, st>>>(m.n, k, S, pr);
-  }
-  m5_tag_split<<<gc, 128, 0, st>>>(m, t, pr, SI, split);
+  m5_tag_split<<<gc, 128, 0, st>>>(m, t, x, SI, split);
+}
+
+void ffv_m5_si_unpack(int64_t n, const uint32_t *SI, int32_t *out, cudaStream_t st) {
+  m5_si_unpack<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, SI, out);
 }
 
 void ffv_m5_cfl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
