@@ -11,10 +11,9 @@
 // Arithmetic: BF16 operands, FP32 accumulation on the tensor cores.  Inference (features,
 // both layers and the marks in one kernel, mlp_infer_tc): a CTA builds the feature rows of
 // 128 cells in shared memory and one thread issues tcgen05.mma (M = 128, N = 64) for each
-// layer, the accumulators in tensor memory.  Training: warp-level mma.sync m16n8k16
-// (16 samples per warp); the backward pass recomputes the forward pass of its tile, forms
-// the weight gradients as (16-sample) tensor-core products into shared-memory FP32
-// accumulators and adds them to the global gradient once per block.
+// layer, the accumulators in tensor memory.  Training: warp-level mma.sync m16n8k16 over
+// 64-sample tiles, the weight gradients accumulated in registers and summed over blocks in a
+// fixed order.
 // Where a tensor-core product needs an operand the forward pass holds in FP32 (the hidden
 // activations, the pre-activation gradients) it is rounded to BF16; the CPU restatement
 // (oracle/mlp.py) rounds at the same points.
@@ -36,7 +35,6 @@ constexpr int OFF_W3 = OFF_B2 + NH, OFF_B3 = OFF_W3 + NH, NPARAM = OFF_B3 + 1;
 static_assert(NPARAM == FFV_MLP_NPARAM, "parameter count");
 constexpr int SX = 152;  // shared row stride (bf16) of 144-wide tiles: conflict-free fragments
 constexpr int SH = 72;   // shared row stride (bf16) of 64-wide tiles
-constexpr int WARPS = 4, TPB = 32 * WARPS;
 
 typedef __nv_bfloat16 bf16;
 
@@ -53,12 +51,8 @@ __device__ __forceinline__ void mma16816(float c[4], uint32_t a0, uint32_t a1, u
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// GELU (exact, erf form) and its derivative
+// GELU (exact, erf form)
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_grad(float x) {
-  return 0.5f * (1.0f + erff(x * 0.70710678118654752f)) +
-         x * 0.39894228040143268f * expf(-0.5f * x * x);
-}
 
 // ------------------------------------------------------------------------- features
 // the cells across faces fneg and fpos of cell e: a boundary face keeps the cell, a face
@@ -170,141 +164,6 @@ __global__ void mlp_pack(const float *__restrict__ P, bf16 *__restrict__ W1, bf1
     W2T[k * NH + r] = w;
   }
 }
-
-struct Smem {
-  bf16 *W1, *W2, *W2T, *X, *H1, *DA;
-  float *b1, *b2, *w3;
-};
-
-// stage the BF16 weights and the FP32 biases into shared memory (whole block)
-__device__ void stage_weights(const Smem &s, const bf16 *W1, const bf16 *W2, const bf16 *W2T,
-                              const float *P, bool with_t) {
-  for (int i = threadIdx.x; i < NH * (KIN / 8); i += blockDim.x) {
-    const int r = i / (KIN / 8), ch = i % (KIN / 8);
-    *reinterpret_cast<uint4 *>(s.W1 + r * SX + ch * 8) =
-        *reinterpret_cast<const uint4 *>(W1 + r * KIN + ch * 8);
-  }
-  for (int i = threadIdx.x; i < NH * (NH / 8); i += blockDim.x) {
-    const int r = i / (NH / 8), ch = i % (NH / 8);
-    *reinterpret_cast<uint4 *>(s.W2 + r * SH + ch * 8) =
-        *reinterpret_cast<const uint4 *>(W2 + r * NH + ch * 8);
-    if (with_t)
-      *reinterpret_cast<uint4 *>(s.W2T + r * SH + ch * 8) =
-          *reinterpret_cast<const uint4 *>(W2T + r * NH + ch * 8);
-  }
-  for (int i = threadIdx.x; i < NH; i += blockDim.x) {
-    s.b1[i] = P[OFF_B1 + i];
-    s.b2[i] = P[OFF_B2 + i];
-    s.w3[i] = P[OFF_W3 + i];
-  }
-}
-
-// load 16 sample rows (row index row_of(i), or zeros past `valid`) into the warp's X tile
-template <typename RowOf>
-__device__ __forceinline__ void load_tile(bf16 *Xs, const bf16 *__restrict__ X, int valid,
-                                          RowOf row_of) {
-  const int lane = threadIdx.x & 31;
-  for (int i = lane; i < 16 * (KIN / 8); i += 32) {
-    const int r = i / (KIN / 8), ch = i % (KIN / 8);
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (r < valid) v = *reinterpret_cast<const uint4 *>(X + row_of(r) * KIN + ch * 8);
-    *reinterpret_cast<uint4 *>(Xs + r * SX + ch * 8) = v;
-  }
-  __syncwarp();
-}
-
-// forward pass of one 16-sample tile: a1/a2 receive the pre-activations (C-fragment
-// layout: [n-tile][4], rows g, g, g+8, g+8 and columns nt*8 + 2q + {0,1}), H1s the first
-// hidden layer in BF16, z the logits of rows g and g+8 (every lane of the quad)
-__device__ __forceinline__ void tile_forward(const Smem &s, const bf16 *Xs, bf16 *H1s,
-                                             float a1[8][4], float a2[8][4], float &zg,
-                                             float &zg8) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-#pragma unroll
-  for (int nt = 0; nt < 8; nt++) a1[nt][0] = a1[nt][1] = a1[nt][2] = a1[nt][3] = 0.0f;
-#pragma unroll
-  for (int kk = 0; kk < KIN / 16; kk++) {
-    const int k0 = kk * 16 + 2 * q;
-    const uint32_t x0 = ld32(Xs + g * SX + k0), x1 = ld32(Xs + (g + 8) * SX + k0);
-    const uint32_t x2 = ld32(Xs + g * SX + k0 + 8), x3 = ld32(Xs + (g + 8) * SX + k0 + 8);
-#pragma unroll
-    for (int nt = 0; nt < 8; nt++) {
-      const bf16 *w = s.W1 + (nt * 8 + g) * SX + k0;
-      mma16816(a1[nt], x0, x1, x2, x3, ld32(w), ld32(w + 8));
-    }
-  }
-#pragma unroll
-  for (int nt = 0; nt < 8; nt++) {
-    const int col = nt * 8 + 2 * q;
-    a1[nt][0] += s.b1[col];
-    a1[nt][1] += s.b1[col + 1];
-    a1[nt][2] += s.b1[col];
-    a1[nt][3] += s.b1[col + 1];
-    *reinterpret_cast<__nv_bfloat162 *>(H1s + g * SH + col) =
-        __floats2bfloat162_rn(gelu(a1[nt][0]), gelu(a1[nt][1]));
-    *reinterpret_cast<__nv_bfloat162 *>(H1s + (g + 8) * SH + col) =
-        __floats2bfloat162_rn(gelu(a1[nt][2]), gelu(a1[nt][3]));
-  }
-  __syncwarp();
-#pragma unroll
-  for (int nt = 0; nt < 8; nt++) a2[nt][0] = a2[nt][1] = a2[nt][2] = a2[nt][3] = 0.0f;
-#pragma unroll
-  for (int kk = 0; kk < NH / 16; kk++) {
-    const int k0 = kk * 16 + 2 * q;
-    const uint32_t h0 = ld32(H1s + g * SH + k0), h1 = ld32(H1s + (g + 8) * SH + k0);
-    const uint32_t h2 = ld32(H1s + g * SH + k0 + 8), h3 = ld32(H1s + (g + 8) * SH + k0 + 8);
-#pragma unroll
-    for (int nt = 0; nt < 8; nt++) {
-      const bf16 *w = s.W2 + (nt * 8 + g) * SH + k0;
-      mma16816(a2[nt], h0, h1, h2, h3, ld32(w), ld32(w + 8));
-    }
-  }
-  zg = 0.0f;
-  zg8 = 0.0f;
-#pragma unroll
-  for (int nt = 0; nt < 8; nt++) {
-    const int col = nt * 8 + 2 * q;
-    a2[nt][0] += s.b2[col];
-    a2[nt][1] += s.b2[col + 1];
-    a2[nt][2] += s.b2[col];
-    a2[nt][3] += s.b2[col + 1];
-    zg += gelu(a2[nt][0]) * s.w3[col] + gelu(a2[nt][1]) * s.w3[col + 1];
-    zg8 += gelu(a2[nt][2]) * s.w3[col] + gelu(a2[nt][3]) * s.w3[col + 1];
-  }
-  zg += __shfl_xor_sync(0xffffffffu, zg, 1);
-  zg += __shfl_xor_sync(0xffffffffu, zg, 2);
-  zg8 += __shfl_xor_sync(0xffffffffu, zg8, 1);
-  zg8 += __shfl_xor_sync(0xffffffffu, zg8, 2);
-}
-
-__device__ __forceinline__ Smem carve(unsigned char *base, bool train) {
-  Smem s;
-  bf16 *p = reinterpret_cast<bf16 *>(base);
-  s.W1 = p;
-  p += NH * SX;
-  s.W2 = p;
-  p += NH * SH;
-  s.W2T = p;
-  if (train) p += NH * SH;
-  s.X = p;
-  p += WARPS * 16 * SX;
-  s.H1 = p;
-  p += WARPS * 16 * SH;
-  s.DA = p;
-  if (train) p += WARPS * 16 * SH;
-  float *f = reinterpret_cast<float *>(p);
-  s.b1 = f;
-  s.b2 = f + NH;
-  s.w3 = f + 2 * NH;
-  return s;
-}
-constexpr size_t smem_bytes(bool train) {
-  return sizeof(bf16) * (size_t)(NH * SX + NH * SH + (train ? NH * SH : 0) + WARPS * 16 * SX +
-                                 WARPS * 16 * SH + (train ? WARPS * 16 * SH : 0)) +
-         sizeof(float) * 3 * NH;
-}
-// FP32 gradient accumulators of a training block, after the operand area
-constexpr size_t ACC_FLOATS = NH * KIN + NH * NH + 3 * NH + 1 + 1;  // ... + b3 + loss
 
 // ------------------------------------------------------------------ inference (tcgen05)
 // One CTA of 128 threads per 128-cell tile (persistent over tiles), thread r owning cell
@@ -482,190 +341,317 @@ __device__ __forceinline__ float rows_sum(float v) {
   return v;
 }
 
-// weight gradient dW[m][j] += sum_s A[s][m] B[s][j] over the tile's 16 samples, A = DA
-// (16 x 64, stride SH), B = a 16 x (8 ntiles) BF16 tile of stride `sb`; columns j >= jmax
-// are dropped
+// ------------------------------------------------------------------ training (mma.sync)
+// The gradient of one batch, in two launches.
+//
+// mlp_grad_tiles: a block of eight warps takes 64 samples at a time.  Warp w holds rows 16 (w & 3) ..
+// of the tile and the output columns 32 (w >> 2) .. of either hidden layer, forms its activations
+// and their derivatives from one erf and one exponential each, and the pre-activation gradients;
+// the weight gradients are products over the tile's 64 samples (dW = dA^T X, both operands read
+// transposed by ldmatrix), accumulated in registers over the block's tiles: warp w owns rows
+// 16 (w & 3) .. and half of the columns of dW1 and dW2.  Every block then writes its own gradient.
+// mlp_update: the blocks' gradients summed in a fixed order (the result does not depend on the order
+// of execution), and AdamW and the BF16 copies of the weights in the same launch.
+//
+// What bounds it: at 8192 samples the grid is 128 blocks of one tile each, so the time is one
+// tile's chain of loads, products and activations.  With one warp per 16 samples, shared-memory
+// atomics for every outer product and global ones per block the gradient took 64 us and a step, with
+// its two clears, AdamW, packing and loss copy, 82 us; now 18 us of a step of 24, and 18 with each
+// kernel's launch overlapping the one before (the next batch's rows load during the update).
+constexpr int TG = 64, TG_TPB = 256;               // samples per tile, threads
+constexpr int PART = NPARAM + 1;                   // a block's gradient and loss
+struct TrainSmem {
+  bf16 W1[NH * SX], W2[NH * SH], W2T[NH * SH];
+  bf16 X[TG * SX], H1[TG * SH], DA2[TG * SH], DA1[TG * SH];
+  float b1[NH], b2[NH], w3[NH], y[TG], z[2][TG], cols[3][4][NH], last[2][4];
+  int64_t row[TG];
+};
+
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t r[4], const bf16 *p) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(a));
+}
+
+// GELU (exact, erf form) and its derivative from one erf
+__device__ __forceinline__ void gelu_both(float x, float &h, float &d) {
+  const float half_cdf = 0.5f * (1.0f + erff(x * 0.70710678118654752f));
+  h = x * half_cdf;
+  d = half_cdf + x * 0.39894228040143268f * expf(-0.5f * x * x);
+}
+
+// acc[nt] += A^T B over the tile's 64 samples for rows m0 .. m0 + 15 of A^T and NT column tiles from
+// n0 of B; A [64][SH], B [64][sb]
 template <int NT>
-__device__ __forceinline__ void grad_outer(const bf16 *DA, const bf16 *B, int sb, float *acc,
-                                           int acc_stride, int jmax) {
+__device__ __forceinline__ void outer_tile(const bf16 *A, int m0, const bf16 *B, int sb, int n0,
+                                           float acc[NT][4]) {
+  const int lane = threadIdx.x & 31, j = lane >> 3, r = lane & 7;
+#pragma unroll
+  for (int kk = 0; kk < TG / 16; kk++) {
+    uint32_t a[4];  // the 8 x 8 blocks (m, k): (0, 0), (8, 0), (0, 8), (8, 8)
+    ldmatrix_x4_trans(a, A + (kk * 16 + (j >> 1) * 8 + r) * SH + m0 + (j & 1) * 8);
+#pragma unroll
+    for (int nt = 0; nt < NT; nt += 2) {
+      // blocks (k, n): (0, 0), (8, 0) and the next column tile's; a last odd tile loads itself twice
+      const int n = n0 + 8 * (nt + 1 < NT ? nt + (j >> 1) : nt);
+      uint32_t b[4];
+      ldmatrix_x4_trans(b, B + (kk * 16 + (j & 1) * 8 + r) * sb + n);
+      mma16816(acc[nt], a[0], a[1], a[2], a[3], b[0], b[1]);
+      if (nt + 1 < NT) mma16816(acc[nt + 1], a[0], a[1], a[2], a[3], b[2], b[3]);
+    }
+  }
+}
+
+// c[nt] = A B^T for the 16 rows of A from row0 (stride sa) and four column tiles from n0 of B [n][k]
+// (stride sb), K the contraction length
+template <int K>
+__device__ __forceinline__ void rows_times(const bf16 *A, int row0, int sa, const bf16 *B, int n0,
+                                           int sb, float c[4][4]) {
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-#pragma unroll 1
-  for (int mt = 0; mt < NH / 16; mt++) {
-    const int m0 = mt * 16 + g;
-    const uint32_t a0 = pack2(DA[(2 * q) * SH + m0], DA[(2 * q + 1) * SH + m0]);
-    const uint32_t a1 = pack2(DA[(2 * q) * SH + m0 + 8], DA[(2 * q + 1) * SH + m0 + 8]);
-    const uint32_t a2 = pack2(DA[(2 * q + 8) * SH + m0], DA[(2 * q + 9) * SH + m0]);
-    const uint32_t a3 = pack2(DA[(2 * q + 8) * SH + m0 + 8], DA[(2 * q + 9) * SH + m0 + 8]);
-#pragma unroll 2
-    for (int nt = 0; nt < NT; nt++) {
-      const int j = nt * 8 + g;
-      const uint32_t b0 = pack2(B[(2 * q) * sb + j], B[(2 * q + 1) * sb + j]);
-      const uint32_t b1 = pack2(B[(2 * q + 8) * sb + j], B[(2 * q + 9) * sb + j]);
-      float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      mma16816(c, a0, a1, a2, a3, b0, b1);
-      const int col = nt * 8 + 2 * q;
-      if (col < jmax) {
-        atomicAdd(acc + m0 * acc_stride + col, c[0]);
-        atomicAdd(acc + (m0 + 8) * acc_stride + col, c[2]);
-      }
-      if (col + 1 < jmax) {
-        atomicAdd(acc + m0 * acc_stride + col + 1, c[1]);
-        atomicAdd(acc + (m0 + 8) * acc_stride + col + 1, c[3]);
-      }
+#pragma unroll
+  for (int nt = 0; nt < 4; nt++) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.0f;
+#pragma unroll
+  for (int kk = 0; kk < K / 16; kk++) {
+    const int k0 = kk * 16 + 2 * q;
+    const bf16 *x = A + (row0 + g) * sa + k0;
+    const uint32_t x0 = ld32(x), x1 = ld32(x + 8 * sa), x2 = ld32(x + 8), x3 = ld32(x + 8 * sa + 8);
+#pragma unroll
+    for (int nt = 0; nt < 4; nt++) {
+      const bf16 *w = B + (n0 + nt * 8 + g) * sb + k0;
+      mma16816(c[nt], x0, x1, x2, x3, ld32(w), ld32(w + 8));
     }
   }
 }
 
-// gradient of the mean binary cross-entropy over B samples (rows drawn by sample_row),
-// added to G (FP32, NPARAM, zeroed by the caller); loss sum added to *loss
-__global__ void __launch_bounds__(TPB) mlp_train_kernel(const bf16 *__restrict__ X,
-                                                        const float *__restrict__ y, int64_t N,
-                                                        int64_t B, uint64_t seed, int64_t step,
-                                                        const bf16 *__restrict__ W1,
-                                                        const bf16 *__restrict__ W2,
-                                                        const bf16 *__restrict__ W2T,
-                                                        const float *__restrict__ P,
-                                                        float *__restrict__ G,
-                                                        float *__restrict__ loss) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const Smem s = carve(smem, true);
-  float *acc = reinterpret_cast<float *>(smem + smem_bytes(true));
-  float *gW1 = acc, *gW2 = acc + NH * KIN, *gb1 = gW2 + NH * NH, *gb2 = gb1 + NH, *gw3 = gb2 + NH;
-  float *gb3 = gw3 + NH, *gl = gb3 + 1;
-  for (int i = threadIdx.x; i < (int)ACC_FLOATS; i += blockDim.x) acc[i] = 0.0f;
-  stage_weights(s, W1, W2, W2T, P, true);
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-  bf16 *Xs = s.X + warp * 16 * SX, *H1s = s.H1 + warp * 16 * SH, *DAs = s.DA + warp * 16 * SH;
+// gradient of the mean binary cross-entropy over B samples (rows drawn by sample_row): the
+// block's share and its sum of the loss into part[blockIdx.x]
+__global__ void __launch_bounds__(TG_TPB) mlp_grad_tiles(const bf16 *__restrict__ X,
+                                                         const float *__restrict__ y, int64_t N,
+                                                         int64_t B, uint64_t seed, int64_t step,
+                                                         const bf16 *W1, const bf16 *W2,
+                                                         const bf16 *W2T, const float *P, float *part) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  TrainSmem &s = *reinterpret_cast<TrainSmem *>(smem_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+  const int row0 = 16 * (warp & 3), n0 = 32 * (warp >> 2);
+  const int64_t ntiles = (B + TG - 1) / TG;
+  const auto load_tile = [&](int64_t t) {
+    const int64_t i0 = t * TG;
+    const int valid = (int)((B - i0) < TG ? (B - i0) : TG);
+    if (tid < TG) {
+      const int64_t r = tid < valid ? sample_row(seed, step, i0 + tid, N) : 0;
+      s.row[tid] = r;
+      s.y[tid] = tid < valid ? y[r] : 0.0f;
+    }
+    __syncthreads();
+    for (int i = tid; i < TG * (KIN / 8); i += TG_TPB) {
+      const int r = i / (KIN / 8), ch = i % (KIN / 8);
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (r < valid) v = *reinterpret_cast<const uint4 *>(X + s.row[r] * KIN + ch * 8);
+      *reinterpret_cast<uint4 *>(s.X + r * SX + ch * 8) = v;
+    }
+  };
+  // the samples do not depend on the step before: they load while its update still runs
+  cudaTriggerProgrammaticLaunchCompletion();
+  load_tile(blockIdx.x);
+  cudaGridDependencySynchronize();
+  for (int i = tid; i < NH * (KIN / 8); i += TG_TPB) {
+    const int r = i / (KIN / 8), ch = i % (KIN / 8);
+    *reinterpret_cast<uint4 *>(s.W1 + r * SX + ch * 8) = *reinterpret_cast<const uint4 *>(W1 + r * KIN + ch * 8);
+  }
+  for (int i = tid; i < NH * (NH / 8); i += TG_TPB) {
+    const int r = i / (NH / 8), ch = i % (NH / 8);
+    *reinterpret_cast<uint4 *>(s.W2 + r * SH + ch * 8) = *reinterpret_cast<const uint4 *>(W2 + r * NH + ch * 8);
+    *reinterpret_cast<uint4 *>(s.W2T + r * SH + ch * 8) = *reinterpret_cast<const uint4 *>(W2T + r * NH + ch * 8);
+  }
+  if (tid < NH) {
+    s.b1[tid] = P[OFF_B1 + tid];
+    s.b2[tid] = P[OFF_B2 + tid];
+    s.w3[tid] = P[OFF_W3 + tid];
+  }
   const float b3 = P[OFF_B3], invB = 1.0f / (float)B;
-  const int64_t ntiles = (B + 15) / 16;
-  for (int64_t t = (int64_t)blockIdx.x * WARPS + warp; t < ntiles; t += (int64_t)gridDim.x * WARPS) {
-    const int64_t i0 = t * 16;
-    const int valid = (int)((B - i0) < 16 ? (B - i0) : 16);
-    load_tile(Xs, X, valid, [&](int r) { return sample_row(seed, step, i0 + r, N); });
-    float a1[8][4], a2[8][4], zg, zg8;
-    tile_forward(s, Xs, H1s, a1, a2, zg, zg8);
+  float dW1[9][4], dW2[4][4], db1[4][2], db2[4][2], dw3[4][2], db3 = 0.0f, loss = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 9; i++) dW1[i][0] = dW1[i][1] = dW1[i][2] = dW1[i][3] = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    dW2[i][0] = dW2[i][1] = dW2[i][2] = dW2[i][3] = 0.0f;
+    db1[i][0] = db1[i][1] = db2[i][0] = db2[i][1] = dw3[i][0] = dw3[i][1] = 0.0f;
+  }
+  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const int valid = (int)((B - t * TG) < TG ? (B - t * TG) : TG);
+    __syncthreads();
+    // first hidden layer: H1 in BF16, the derivatives kept
+    float a[4][4], g1[4][4];
+    rows_times<KIN>(s.X, row0, SX, s.W1, n0, SX, a);
+#pragma unroll
+    for (int nt = 0; nt < 4; nt++) {
+      const int col = n0 + nt * 8 + 2 * q;
+      float h[4];
+#pragma unroll
+      for (int e = 0; e < 4; e++) gelu_both(a[nt][e] + s.b1[col + (e & 1)], h[e], g1[nt][e]);
+      *reinterpret_cast<__nv_bfloat162 *>(s.H1 + (row0 + g) * SH + col) = __floats2bfloat162_rn(h[0], h[1]);
+      *reinterpret_cast<__nv_bfloat162 *>(s.H1 + (row0 + g + 8) * SH + col) = __floats2bfloat162_rn(h[2], h[3]);
+    }
+    __syncthreads();
+    // second hidden layer and this warp's half of the logits
+    float h2[4][4], g2[4][4], zg = 0.0f, zg8 = 0.0f;
+    rows_times<NH>(s.H1, row0, SH, s.W2, n0, SH, a);
+#pragma unroll
+    for (int nt = 0; nt < 4; nt++) {
+      const int col = n0 + nt * 8 + 2 * q;
+#pragma unroll
+      for (int e = 0; e < 4; e++) gelu_both(a[nt][e] + s.b2[col + (e & 1)], h2[nt][e], g2[nt][e]);
+      zg += h2[nt][0] * s.w3[col] + h2[nt][1] * s.w3[col + 1];
+      zg8 += h2[nt][2] * s.w3[col] + h2[nt][3] * s.w3[col + 1];
+    }
+    zg += __shfl_xor_sync(0xffffffffu, zg, 1);
+    zg += __shfl_xor_sync(0xffffffffu, zg, 2);
+    zg8 += __shfl_xor_sync(0xffffffffu, zg8, 1);
+    zg8 += __shfl_xor_sync(0xffffffffu, zg8, 2);
+    if (q == 0) {
+      s.z[warp >> 2][row0 + g] = zg;
+      s.z[warp >> 2][row0 + g + 8] = zg8;
+    }
+    __syncthreads();
     // output layer: d loss / d z = (p - y) / B
-    float dzg = 0.0f, dzg8 = 0.0f;
-    if (g < valid) {
-      const float p = 1.0f / (1.0f + expf(-(zg + b3))), yy = y[sample_row(seed, step, i0 + g, N)];
-      dzg = (p - yy) * invB;
-      if (q == 0) atomicAdd(gl, -(yy * logf(fmaxf(p, 1e-12f)) + (1.0f - yy) * logf(fmaxf(1.0f - p, 1e-12f))));
-    }
-    if (g + 8 < valid) {
-      const float p = 1.0f / (1.0f + expf(-(zg8 + b3))),
-                  yy = y[sample_row(seed, step, i0 + g + 8, N)];
-      dzg8 = (p - yy) * invB;
-      if (q == 0)
-        atomicAdd(gl, -(yy * logf(fmaxf(p, 1e-12f)) + (1.0f - yy) * logf(fmaxf(1.0f - p, 1e-12f))));
-    }
-    {
-      float d3 = (q == 0) ? dzg + dzg8 : 0.0f;
-      d3 = rows_sum(d3);
-      if (lane == 0) atomicAdd(gb3, d3);
-    }
-    // second hidden layer
+    float dz[2];
 #pragma unroll
-    for (int nt = 0; nt < 8; nt++) {
-      const int col = nt * 8 + 2 * q;
-      float w3v[2] = {s.w3[col], s.w3[col + 1]};
-      float dw[2], db[2];
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const float h_g = gelu(a2[nt][e]), h_g8 = gelu(a2[nt][2 + e]);
-        dw[e] = rows_sum(dzg * h_g + dzg8 * h_g8);
-        const float d_g = dzg * w3v[e] * gelu_grad(a2[nt][e]);
-        const float d_g8 = dzg8 * w3v[e] * gelu_grad(a2[nt][2 + e]);
-        a2[nt][e] = d_g;
-        a2[nt][2 + e] = d_g8;
-        db[e] = rows_sum(d_g + d_g8);
-      }
-      if (g == 0) {
-        atomicAdd(gw3 + col, dw[0]);
-        atomicAdd(gw3 + col + 1, dw[1]);
-        atomicAdd(gb2 + col, db[0]);
-        atomicAdd(gb2 + col + 1, db[1]);
-      }
-      *reinterpret_cast<__nv_bfloat162 *>(DAs + g * SH + col) = __floats2bfloat162_rn(a2[nt][0], a2[nt][1]);
-      *reinterpret_cast<__nv_bfloat162 *>(DAs + (g + 8) * SH + col) =
-          __floats2bfloat162_rn(a2[nt][2], a2[nt][3]);
-    }
-    __syncwarp();
-    // dW2 = da2^T h1
-    grad_outer<8>(DAs, H1s, SH, gW2, NH, NH);
-    // dh1 = da2 W2, then da1 = dh1 * gelu'(a1)
-    float dh[8][4];
-#pragma unroll
-    for (int nt = 0; nt < 8; nt++) dh[nt][0] = dh[nt][1] = dh[nt][2] = dh[nt][3] = 0.0f;
-#pragma unroll
-    for (int kk = 0; kk < NH / 16; kk++) {
-      const int k0 = kk * 16 + 2 * q;
-      const uint32_t d0 = ld32(DAs + g * SH + k0), d1 = ld32(DAs + (g + 8) * SH + k0);
-      const uint32_t d2 = ld32(DAs + g * SH + k0 + 8), d3 = ld32(DAs + (g + 8) * SH + k0 + 8);
-#pragma unroll
-      for (int nt = 0; nt < 8; nt++) {
-        const bf16 *w = s.W2T + (nt * 8 + g) * SH + k0;
-        mma16816(dh[nt], d0, d1, d2, d3, ld32(w), ld32(w + 8));
+    for (int e = 0; e < 2; e++) {
+      const int r = row0 + g + 8 * e;
+      dz[e] = 0.0f;
+      if (r < valid) {
+        const float p = 1.0f / (1.0f + expf(-(s.z[0][r] + s.z[1][r] + b3))), yy = s.y[r];
+        dz[e] = (p - yy) * invB;
+        if (q == 0 && n0 == 0) {
+          db3 += dz[e];
+          loss -= yy * logf(fmaxf(p, 1e-12f)) + (1.0f - yy) * logf(fmaxf(1.0f - p, 1e-12f));
+        }
       }
     }
-    __syncwarp();
 #pragma unroll
-    for (int nt = 0; nt < 8; nt++) {
-      const int col = nt * 8 + 2 * q;
-      float db[2];
+    for (int nt = 0; nt < 4; nt++) {
+      const int col = n0 + nt * 8 + 2 * q;
+      float d[4];
 #pragma unroll
-      for (int e = 0; e < 2; e++) {
-        dh[nt][e] *= gelu_grad(a1[nt][e]);
-        dh[nt][2 + e] *= gelu_grad(a1[nt][2 + e]);
-        db[e] = rows_sum(dh[nt][e] + dh[nt][2 + e]);
+      for (int e = 0; e < 4; e++) {
+        dw3[nt][e & 1] += dz[e >> 1] * h2[nt][e];
+        d[e] = dz[e >> 1] * s.w3[col + (e & 1)] * g2[nt][e];
+        db2[nt][e & 1] += d[e];
       }
-      if (g == 0) {
-        atomicAdd(gb1 + col, db[0]);
-        atomicAdd(gb1 + col + 1, db[1]);
-      }
-      *reinterpret_cast<__nv_bfloat162 *>(DAs + g * SH + col) = __floats2bfloat162_rn(dh[nt][0], dh[nt][1]);
-      *reinterpret_cast<__nv_bfloat162 *>(DAs + (g + 8) * SH + col) =
-          __floats2bfloat162_rn(dh[nt][2], dh[nt][3]);
+      *reinterpret_cast<__nv_bfloat162 *>(s.DA2 + (row0 + g) * SH + col) = __floats2bfloat162_rn(d[0], d[1]);
+      *reinterpret_cast<__nv_bfloat162 *>(s.DA2 + (row0 + g + 8) * SH + col) = __floats2bfloat162_rn(d[2], d[3]);
     }
-    __syncwarp();
-    // dW1 = da1^T x
-    grad_outer<KIN / 8>(DAs, Xs, SX, gW1, KIN, NIN);
-    __syncwarp();
+    __syncthreads();
+    // dh1 = da2 W2, da1 = dh1 gelu'(a1)
+    rows_times<NH>(s.DA2, row0, SH, s.W2T, n0, SH, a);
+#pragma unroll
+    for (int nt = 0; nt < 4; nt++) {
+      const int col = n0 + nt * 8 + 2 * q;
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        a[nt][e] *= g1[nt][e];
+        db1[nt][e & 1] += a[nt][e];
+      }
+      *reinterpret_cast<__nv_bfloat162 *>(s.DA1 + (row0 + g) * SH + col) = __floats2bfloat162_rn(a[nt][0], a[nt][1]);
+      *reinterpret_cast<__nv_bfloat162 *>(s.DA1 + (row0 + g + 8) * SH + col) = __floats2bfloat162_rn(a[nt][2], a[nt][3]);
+    }
+    outer_tile<4>(s.DA2, row0, s.H1, SH, n0, dW2);
+    __syncthreads();
+    outer_tile<9>(s.DA1, row0, s.X, SX, 72 * (warp >> 2), dW1);
+    if (t + gridDim.x < ntiles) {
+      __syncthreads();  // the next tile overwrites what these read
+      load_tile(t + gridDim.x);
+    }
+  }
+  // the block's gradient
+  float *G = part + (size_t)blockIdx.x * PART;
+#pragma unroll
+  for (int nt = 0; nt < 9; nt++) {
+    const int col = 72 * (warp >> 2) + nt * 8 + 2 * q;
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+      if (col + (e & 1) < NIN) G[OFF_W1 + (row0 + g + 8 * (e >> 1)) * NIN + col + (e & 1)] = dW1[nt][e];
+  }
+#pragma unroll
+  for (int nt = 0; nt < 4; nt++) {
+    const int col = n0 + nt * 8 + 2 * q;
+#pragma unroll
+    for (int e = 0; e < 4; e++) G[OFF_W2 + (row0 + g + 8 * (e >> 1)) * NH + col + (e & 1)] = dW2[nt][e];
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const float v[3] = {db1[nt][e], db2[nt][e], dw3[nt][e]};
+#pragma unroll
+      for (int j = 0; j < 3; j++) {
+        const float sum = rows_sum(v[j]);
+        if (g == 0) s.cols[j][warp & 3][col + e] = sum;
+      }
+    }
+  }
+  db3 = rows_sum(db3);
+  loss = rows_sum(loss);
+  if (lane == 0 && n0 == 0) {
+    s.last[0][warp] = db3;
+    s.last[1][warp] = loss;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < NH * NIN; i += blockDim.x) {
-    const int r = i / NIN, k = i % NIN;
-    const float v = gW1[r * KIN + k];
-    if (v != 0.0f) atomicAdd(G + OFF_W1 + i, v);
-  }
-  for (int i = threadIdx.x; i < NH * NH; i += blockDim.x)
-    if (gW2[i] != 0.0f) atomicAdd(G + OFF_W2 + i, gW2[i]);
-  for (int i = threadIdx.x; i < NH; i += blockDim.x) {
-    atomicAdd(G + OFF_B1 + i, gb1[i]);
-    atomicAdd(G + OFF_B2 + i, gb2[i]);
-    atomicAdd(G + OFF_W3 + i, gw3[i]);
-  }
-  if (threadIdx.x == 0) {
-    atomicAdd(G + OFF_B3, *gb3);
-    atomicAdd(loss, *gl);
+  if (tid < 3 * NH) {
+    const int j = tid / NH, c = tid % NH;
+    const float v = (s.cols[j][0][c] + s.cols[j][1][c]) + (s.cols[j][2][c] + s.cols[j][3][c]);
+    G[(j == 0 ? OFF_B1 : j == 1 ? OFF_B2 : OFF_W3) + c] = v;
+  } else if (tid < 3 * NH + 2) {
+    const int j = tid - 3 * NH;
+    G[j == 0 ? OFF_B3 : NPARAM] = (s.last[j][0] + s.last[j][1]) + (s.last[j][2] + s.last[j][3]);
   }
 }
 
-// AdamW (decoupled weight decay on W1, W2, w3; none on the biases)
-__global__ void mlp_adamw(float *__restrict__ P, const float *__restrict__ G, float *__restrict__ M,
-                          float *__restrict__ V, float lr, float wd, float b1, float b2, float eps,
-                          float c1, float c2) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NPARAM; i += gridDim.x * blockDim.x) {
-    const float gr = G[i];
-    const float m = b1 * M[i] + (1.0f - b1) * gr;
-    const float v = b2 * V[i] + (1.0f - b2) * gr * gr;
-    M[i] = m;
-    V[i] = v;
-    const bool decay = (i < OFF_B1) || (i >= OFF_W2 && i < OFF_B2) || (i >= OFF_W3 && i < OFF_B3);
-    float p = P[i];
-    if (decay) p -= lr * wd * p;
-    p -= lr * (m / c1) / (sqrtf(v / c2) + eps);
-    P[i] = p;
+// the sum of the blocks' gradients (four lanes per entry, each every fourth block), into G and the
+// loss sum into *loss; with STEP then AdamW (decoupled weight decay on W1, W2, w3; none on the
+// biases) and the weights' BF16 copies
+template <bool STEP>
+__global__ void __launch_bounds__(256) mlp_update(const float *part, int nblocks,
+                                                  float *__restrict__ G, float *__restrict__ loss,
+                                                  float *__restrict__ P, float *__restrict__ M,
+                                                  float *__restrict__ V, bf16 *__restrict__ W1,
+                                                  bf16 *__restrict__ W2, bf16 *__restrict__ W2T,
+                                                  float lr, float wd, float b1, float b2, float eps,
+                                                  float c1, float c2) {
+  const int i = (int)(blockIdx.x * 256 + threadIdx.x) >> 2, j = threadIdx.x & 3;
+  float gr = 0.0f;
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+  if (i < PART) {
+#pragma unroll 8
+    for (int b = j; b < nblocks; b += 4) gr += part[(size_t)b * PART + i];
+  }
+  gr += __shfl_xor_sync(0xffffffffu, gr, 1);
+  gr += __shfl_xor_sync(0xffffffffu, gr, 2);
+  if (i >= PART || j) return;
+  if (i == NPARAM) {
+    *loss = gr;
+    return;
+  }
+  if (!STEP) {
+    G[i] = gr;
+    return;
+  }
+  const float m = b1 * M[i] + (1.0f - b1) * gr;
+  const float v = b2 * V[i] + (1.0f - b2) * gr * gr;
+  M[i] = m;
+  V[i] = v;
+  const bool decay = (i < OFF_B1) || (i >= OFF_W2 && i < OFF_B2) || (i >= OFF_W3 && i < OFF_B3);
+  float p = P[i];
+  if (decay) p -= lr * wd * p;
+  p -= lr * (m / c1) / (sqrtf(v / c2) + eps);
+  P[i] = p;
+  if (i < OFF_B1) {
+    W1[(i / NIN) * KIN + i % NIN] = __float2bfloat16_rn(p);
+  } else if (i >= OFF_W2 && i < OFF_B2) {
+    const int r = (i - OFF_W2) / NH, k = (i - OFF_W2) % NH;
+    const bf16 w = __float2bfloat16_rn(p);
+    W2[i - OFF_W2] = w;
+    W2T[k * NH + r] = w;
   }
 }
 
@@ -677,6 +663,9 @@ struct ffv_mlp {
   float *d_P, *d_G, *d_M, *d_V, *d_norm, *d_loss;
   bf16 *d_W1, *d_W2, *d_W2T;
   int64_t t;  // AdamW step count
+  // training: the blocks' gradients [nsm][PART] and the steps' losses, made by the first call
+  float *d_part, *d_losses;
+  int64_t cap_losses;
   // predict buffers
   int64_t cap;
   float *d_F, *d_prob;
@@ -738,20 +727,39 @@ int take_timeout(ffv_mlp *m) {
   return FFV_ERR_TIMEOUT;
 }
 
-int grad(ffv_mlp *m, const bf16 *X, const float *y, int64_t N, int64_t B, uint64_t seed,
-         int64_t step) {
-  MCK(cudaMemsetAsync(m->d_G, 0, sizeof(float) * NPARAM, m->stream));
-  MCK(cudaMemsetAsync(m->d_loss, 0, sizeof(float), m->stream));
-  const size_t sb = smem_bytes(true) + sizeof(float) * ACC_FLOATS;
-  MCK(cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb));
-  const int64_t tiles = (B + 15) / 16;
-  int64_t blocks = (tiles + WARPS - 1) / WARPS;
-  if (blocks > 152) blocks = 152;
-  mlp_train_kernel<<<(unsigned)blocks, TPB, sb, m->stream>>>(X, y, N, B, seed, step, m->d_W1,
-                                                             m->d_W2, m->d_W2T, m->d_P, m->d_G,
-                                                             m->d_loss);
-  return mlp_cuda(cudaGetLastError());
+// a launch that may begin before the stream's previous kernel has ended: the kernel itself waits
+// for it (cudaGridDependencySynchronize) before it reads or writes what the two share
+template <typename... Params, typename... Args>
+int launch_early(ffv_mlp *m, void (*kernel)(Params...), unsigned blocks, unsigned threads, size_t smem,
+                 Args... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = m->stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return mlp_cuda(cudaLaunchKernelEx(&cfg, kernel, Params(args)...));
 }
+
+// the blocks' gradients of one batch into d_part; *blocks receives their number
+int grad(ffv_mlp *m, const bf16 *X, const float *y, int64_t N, int64_t B, uint64_t seed,
+         int64_t step, int *blocks) {
+  if (!m->d_part && cudaMalloc(&m->d_part, sizeof(float) * PART * (size_t)m->nsm) != cudaSuccess) {
+    m->d_part = nullptr;
+    return FFV_ERR_NOMEM;
+  }
+  MCK(cudaFuncSetAttribute(mlp_grad_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainSmem)));
+  const int64_t tiles = (B + TG - 1) / TG;
+  *blocks = (int)(tiles < m->nsm ? tiles : m->nsm);
+  return launch_early(m, mlp_grad_tiles, (unsigned)*blocks, TG_TPB, sizeof(TrainSmem), X, y, N, B, seed, step,
+                      (const bf16 *)m->d_W1, (const bf16 *)m->d_W2, (const bf16 *)m->d_W2T,
+                      (const float *)m->d_P, m->d_part);
+}
+constexpr unsigned UPDATE_BLOCKS = (4 * PART + 255) / 256;
 
 // seeded host initialisation: weights uniform in +-1/sqrt(fan_in), biases zero
 void init_params(float *P, uint64_t seed) {
@@ -859,6 +867,8 @@ int ffv_mlp_destroy(ffv_mlp *m) {
   cudaFree(m->d_W2T);
   cudaFree(m->d_F);
   cudaFree(m->d_prob);
+  cudaFree(m->d_part);
+  cudaFree(m->d_losses);
   cudaFreeHost(m->h_err);
   if (m->stream) cudaStreamDestroy(m->stream);
   free(m);
@@ -978,7 +988,11 @@ int ffv_mlp_grad(ffv_mlp *m, const void *X_dev, const float *y_dev, int64_t B, f
                  float *loss_host) {
   if (!m || !X_dev || !y_dev || !grad_host || B < 1) return FFV_ERR_ARG;
   MCK(cudaSetDevice(m->device));
-  int rc = grad(m, (const bf16 *)X_dev, y_dev, B, B, 0, 0);
+  int blocks;
+  int rc = grad(m, (const bf16 *)X_dev, y_dev, B, B, 0, 0, &blocks);
+  if (rc != FFV_OK) return rc;
+  rc = launch_early(m, mlp_update<false>, UPDATE_BLOCKS, 256, 0, m->d_part, blocks, m->d_G, m->d_loss, m->d_P,
+                    m->d_M, m->d_V, m->d_W1, m->d_W2, m->d_W2T, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 1.0f, 1.0f);
   if (rc != FFV_OK) return rc;
   MCK(cudaMemcpyAsync(grad_host, m->d_G, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost, m->stream));
   float l = 0.0f;
@@ -993,23 +1007,28 @@ int ffv_mlp_train(ffv_mlp *m, const void *X_dev, const float *y_dev, int64_t N, 
   if (!m || !X_dev || !y_dev || N < 1 || batch < 1 || steps < 0 || seed == 0) return FFV_ERR_ARG;
   MCK(cudaSetDevice(m->device));
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  if (steps > m->cap_losses) {
+    cudaFree(m->d_losses);
+    m->d_losses = nullptr;
+    m->cap_losses = 0;
+    if (cudaMalloc(&m->d_losses, sizeof(float) * (size_t)steps) != cudaSuccess) return FFV_ERR_NOMEM;
+    m->cap_losses = steps;
+  }
   for (int32_t i = 0; i < steps; i++) {
-    int rc = grad(m, (const bf16 *)X_dev, y_dev, N, batch, seed, m->t);
+    int blocks;
+    int rc = grad(m, (const bf16 *)X_dev, y_dev, N, batch, seed, m->t, &blocks);
     if (rc != FFV_OK) return rc;
     m->t++;
     const float c1 = 1.0f - powf(b1, (float)m->t), c2 = 1.0f - powf(b2, (float)m->t);
-    mlp_adamw<<<(NPARAM + 255) / 256, 256, 0, m->stream>>>(m->d_P, m->d_G, m->d_M, m->d_V, lr, wd,
-                                                           b1, b2, eps, c1, c2);
-    rc = repack(m);
+    rc = launch_early(m, mlp_update<true>, UPDATE_BLOCKS, 256, 0, m->d_part, blocks, m->d_G, m->d_losses + i,
+                      m->d_P, m->d_M, m->d_V, m->d_W1, m->d_W2, m->d_W2T, lr, wd, b1, b2, eps, c1, c2);
     if (rc != FFV_OK) return rc;
-    if (loss_host) {
-      float l = 0.0f;
-      MCK(cudaMemcpyAsync(&l, m->d_loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-      MCK(cudaStreamSynchronize(m->stream));
-      loss_host[i] = l / (float)batch;
-    }
   }
+  if (loss_host && steps > 0)
+    MCK(cudaMemcpyAsync(loss_host, m->d_losses, sizeof(float) * (size_t)steps, cudaMemcpyDeviceToHost, m->stream));
   MCK(cudaStreamSynchronize(m->stream));
+  if (loss_host)
+    for (int32_t i = 0; i < steps; i++) loss_host[i] /= (float)batch;
   return FFV_OK;
 }
 
