@@ -118,7 +118,7 @@ int alloc_mesh_buffers(ffv_ctx *c) {
         cudaMalloc(&c->d_UF, sizeof(double) * 18 * n) != cudaSuccess ||
         cudaMalloc(&c->d_GF, (((6 * n + 3) & ~(int64_t)3) + 4 * n)) != cudaSuccess ||
         cudaMalloc(&c->d_RHS, sizeof(double) * c->neq * n) != cudaSuccess ||
-        cudaMalloc(&c->d_flag, n) != cudaSuccess ||
+        cudaMalloc(&c->d_flag, 10 * n) != cudaSuccess ||  // flags, and the FP32-flux form's marks
         cudaMalloc(&c->d_list, sizeof(int32_t) * (n + 13)) != cudaSuccess) {
       free_mesh_buffers(c);
       return FFV_ERR_NOMEM;
@@ -138,19 +138,32 @@ unsigned status_to_err(unsigned st) {
 
 int neq_of(const ffv_params &p) { return p.model == 0 ? 5 : ffv_m5_neq(p.nmaterials); }
 
-int launch_stage(ffv_ctx *c, int irk, cudaEvent_t *ev = nullptr) {
+// the marks of flat cells behind the flags
+FlatMarks flat_marks(const ffv_ctx *c) {
+  uint8_t *p = c->d_flag + c->cap;
+  return FlatMarks{p, p + c->cap, p + 2 * c->cap, p + 3 * c->cap};
+}
+
+// SN holds a whole state (not one of a stage 1 that left out flat cells' deformation)
+cudaError_t whole_base(ffv_ctx *c) {
+  return c->p.model == 5 ? cudaMemsetAsync(flat_marks(c).base, 0, c->n, c->stream) : cudaSuccess;
+}
+
+// follows: nothing but the stage before has touched the state
+int launch_stage(ffv_ctx *c, int irk, bool follows, cudaEvent_t *ev = nullptr) {
   ffv_m0_bufs b{c->d_S, c->d_SN, c->d_SF, c->d_dt, c->d_status};
   ffv_m0_consts k{c->p.gamma[0], c->p.pinf[0], c->p.order};
   if (irk == 0) {
     CK(cudaMemcpyAsync(c->d_SN, c->d_S, sizeof(double) * c->neq * c->n, cudaMemcpyDeviceToDevice,
                        c->stream));
+    CK(whole_base(c));
     return FFV_OK;
   }
   if (c->p.model == 5) {
     ffv_m5_bufs mb{c->d_S,   c->d_SN,   c->d_Snew, c->d_SF,     c->d_FF,    c->d_UF,
-                   c->d_RHS, c->d_dt,   c->d_GF,   c->d_flag,   c->d_list,  c->d_status,
-                   c->flist};
-    ffv_m5_fp64_stage(c->dm, c->geom, c->m5, mb, irk, c->stream, ev, c->knames);
+                   c->d_RHS, c->d_dt,   c->d_GF,   c->d_flag,   flat_marks(c), c->d_list,
+                   c->d_status, c->flist};
+    ffv_m5_fp64_stage(c->dm, c->geom, c->m5, mb, irk, follows, c->stream, ev, c->knames);
     return cuda_rc(cudaGetLastError());
   }
   ffv_m0_fp64_stage(c->dm, c->geom, b, k, irk, c->stream, ev);
@@ -169,7 +182,7 @@ int build_graph(ffv_ctx *c) {
   cudaGraph_t g;
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   int rc = FFV_OK;
-  for (int irk = 1; irk <= c->p.rk_steps && rc == FFV_OK; irk++) rc = launch_stage(c, irk);
+  for (int irk = 1; irk <= c->p.rk_steps && rc == FFV_OK; irk++) rc = launch_stage(c, irk, irk > 1);
   cudaError_t e = cudaStreamEndCapture(c->stream, &g);
   if (rc != FFV_OK) return rc;
   CK(e);
@@ -246,6 +259,7 @@ int build_face_list(ffv_ctx *c, const int64_t *count) {
   l.cells = cells;
   CK(cudaMemsetAsync(c->d_GF, 0, 6 * c->n, c->stream));
   CK(cudaMemsetAsync(c->d_list, 0, sizeof(int32_t), c->stream));  // no flagged cells
+  CK(whole_base(c));
   if (total == 0) return FFV_OK;
   int32_t *cursor = c->d_list + 1 + c->cap;
   CK(cudaMemcpyAsync(cursor, l.off, sizeof(int32_t) * 12, cudaMemcpyHostToDevice, c->stream));
@@ -609,6 +623,7 @@ int ffv_upload_state(ffv_ctx *c, const double *S, int64_t ncells, int32_t neq) {
                      c->stream));
   CK(cudaMemcpyAsync(c->d_SN, c->d_S, sizeof(double) * neq * ncells, cudaMemcpyDeviceToDevice,
                      c->stream));
+  CK(whole_base(c));
   CK(cudaStreamSynchronize(c->stream));
   c->have_state = 1;
   return FFV_OK;
@@ -632,7 +647,7 @@ int ffv_stage(ffv_ctx *c, int32_t irk, double dt) {
   CK(cudaSetDevice(c->device));
   int rc = queue_dt(c, dt);
   if (rc != FFV_OK) return rc;
-  return launch_stage(c, irk);
+  return launch_stage(c, irk, false);
 }
 
 int ffv_sync(ffv_ctx *c) {
@@ -772,7 +787,7 @@ int ffv_profile_stage(ffv_ctx *c, int32_t irk, double dt, float *ms, int32_t max
   cudaEvent_t ev[17];
   for (int i = 0; i <= nk; i++) CK(cudaEventCreate(&ev[i]));
   int rc = queue_dt(c, dt);
-  if (rc == FFV_OK) rc = launch_stage(c, irk, ev);
+  if (rc == FFV_OK) rc = launch_stage(c, irk, false, ev);
   if (rc == FFV_OK && cudaEventSynchronize(ev[nk]) != cudaSuccess) rc = FFV_ERR_CUDA;
   for (int i = 0; i < nk && rc == FFV_OK; i++)
     if (cudaEventElapsedTime(&ms[i], ev[i], ev[i + 1]) != cudaSuccess) rc = FFV_ERR_CUDA;

@@ -43,9 +43,22 @@ struct M5Consts {
   df alo_d, ahi_d, a2lo_d, eps_d, oneeps_d;
 };
 
+// bits of a face's mark (GF): a ghost-fluid face; its deformation flux is stored (FP32-flux form)
+#define FFV_FACE_GFM 1
+#define FFV_FACE_DEFORMS 2
+
+// FP32-flux form: flat cells and face states, whose deformation is zero and kept nowhere but in S
+struct FlatMarks {
+  uint8_t *cell;  // [n]: the stage's input state
+  uint8_t *next;  // [n]: the state the cell update made (before it: this one's calm cells)
+  uint8_t *base;  // [n]: SN (its deformation is then not stored)
+  uint8_t *face;  // [6][n]: face states
+};
+
 struct ffv_m5_bufs {
   double *S, *SN, *Snew, *SF, *FF, *UF, *RHS, *dt;
-  uint8_t *GF, *flag;  // GF [6][n]: ghost-fluid faces, as the cell that evaluates the face sees them
+  uint8_t *GF, *flag;  // GF [6][n]: marks of faces, as the cell that evaluates the face sees them
+  FlatMarks flat;
 
   int32_t *list;  // [1 + n]: the number of cells the last pass flagged, then the cells
   unsigned int *status;
@@ -54,10 +67,10 @@ struct ffv_m5_bufs {
 
 int ffv_m5_neq(int nmat);
 // ev (nullable): an event before the first and after every kernel; names[i] receives
-// kernel i's name
+// kernel i's name.  follows: the stage before ran on this state and nothing else has touched it.
 void ffv_m5_fp64_stage(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
-                       const ffv_m5_bufs &b, int irk, cudaStream_t st, cudaEvent_t *ev,
-                       const char **names);
+                       const ffv_m5_bufs &b, int irk, bool follows, cudaStream_t st,
+                       cudaEvent_t *ev, const char **names);
 int ffv_m5_launches_per_stage(const M5Consts &k, int irk);
 
 // FP32-flux form (ffv_m5_fp32.cu): face states and face fluxes in FP32.
@@ -65,27 +78,31 @@ int ffv_m5_launches_per_stage(const M5Consts &k, int irk);
 //   SFf: [6][neq + 2][n] float -- the reconstructed, relaxed face state followed by the last
 //        volume fraction and the relaxed pressure
 //   FFf: [6][neq][n] float face fluxes (area-weighted), UFf: [6][3][n] float face velocity
-void ffv_m5f_shadow(int64_t n, const M5Consts &k, const double *S, float *Sf, cudaStream_t st);
-void ffv_m5f_recon(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
-                   const float *Sf, float *SFf, unsigned *status, cudaStream_t st);
+// known: the marks of the previous stage's cell update hold for S
+void ffv_m5f_shadow(int64_t n, const M5Consts &k, const double *S, float *Sf, const FlatMarks &fm,
+                    bool known, cudaStream_t st);
+void ffv_m5f_recon(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const float *Sf,
+                   const FlatMarks &fm, float *SFf, unsigned *status, cudaStream_t st);
 // Sf: the FP32 copy of the state (order 2), or nullptr (order 1: phi0 from S)
 void ffv_m5f_flux(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
-                  const float *Sf, const float *SFf, float *FFf, float *UFf, uint8_t *GF,
-                  const ffv_face_list &fl, unsigned *status, cudaStream_t st);
-// residual + RK stage of the FP32-flux form (the face fluxes of all but the deformation
-// summed in FP64)
+                  const float *Sf, const float *SFf, const FlatMarks &fm, float *FFf, float *UFf,
+                  uint8_t *GF, const ffv_face_list &fl, unsigned *status, cudaStream_t st);
+// residual + RK stage of the FP32-flux form (the face fluxes of all but the deformation summed as
+// double-float pairs)
 void ffv_m5f_cell_update(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
-                         double *SN, const float *FFf, const float *UFf, double *RHS,
-                         double *Snew, uint8_t *flag, int32_t *list, const double *dt, int irk,
-                         unsigned *status, cudaStream_t st);
+                         double *SN, const float *FFf, const float *UFf, const uint8_t *GF,
+                         const FlatMarks &fm, double *RHS, double *Snew, uint8_t *flag,
+                         int32_t *list, const double *dt, int irk, unsigned *status,
+                         cudaStream_t st);
 // the indicator's fields of a model-5 state, F [5][n] float (log rho, log p, alpha_0, |u|,
 // von Mises stress; FP32 with double-float pressure recovery; ffv_mlp.cu gathers them)
 void ffv_m5f_indicator_fields(int64_t n, const M5Consts &k, const double *S, float *F,
                               cudaStream_t st);
 // cell pressure relaxation: the Newton iteration in FP32, the pressure recovery and the
 // energy-consistent pressure and internal energies in double-float
-void ffv_m5f_relax_cell(int64_t n, const M5Consts &k, const double *Sin, double *Sout,
-                        uint8_t *flag, int32_t *list, unsigned *status, cudaStream_t st);
+void ffv_m5f_relax_cell(int64_t n, const M5Consts &k, const double *Sin, const FlatMarks &fm,
+                        double *Sout, uint8_t *flag, int32_t *list, unsigned *status,
+                        cudaStream_t st);
 void ffv_m5_cfl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
                 unsigned long long *d_out, cudaStream_t st);
 

@@ -1033,7 +1033,7 @@ __device__ __forceinline__ void store_flux(int64_t n, int f, int64_t c, const do
   for (int iv = 0; iv < C::NEQ; iv++) FF[((int64_t)f * C::NEQ + iv) * n + c] = ff[iv];
 #pragma unroll
   for (int d = 0; d < 3; d++) UF[((int64_t)f * 3 + d) * n + c] = un[d];
-  GF[(int64_t)f * n + c] = gfm ? 1 : 0;
+  GF[(int64_t)f * n + c] = gfm ? FFV_FACE_GFM : 0;
 }
 
 template <int N, int ORDER, int F>
@@ -1390,7 +1390,7 @@ __global__ void __launch_bounds__(GFM_TPB) m5_gfm_seq(ffv_dmesh m, ffv_geom g, M
       const int f = lane;
       const uint32_t kind = ffv_face_kind(info, f);
       double phiR = 0.0, vr[3] = {0.0, 0.0, 0.0};
-      if (GF[(int64_t)f * m.n + c]) {
+      if (GF[(int64_t)f * m.n + c] & FFV_FACE_GFM) {
         Sol<N> R;
         if (kind & FFV_FK_BC) {
           const int bc = (int)(kind & 7u);
@@ -1446,7 +1446,7 @@ __global__ void __launch_bounds__(GFM_TPB) m5_gfm_seq(ffv_dmesh m, ffv_geom g, M
       double nxi = 0.0, nyi = 0.0, nzi = 0.0, total = 0.0, ug[6], vg[6], wg[6];
       int nint = 0;
       for (int f = 0; f < 6; f++) {
-        if (GF[(int64_t)f * m.n + c]) {
+        if (GF[(int64_t)f * m.n + c] & FFV_FACE_GFM) {
           const double phi = (L.phi0 + s_phiR[f]) / 2.0;
           const double A = g.area[ffv_face_kind(info, f) == FFV_FK_FINER ? l + 1 : l];
           const int ax = fr_n_axis(f), sg = fr_n_sign(f);
@@ -1489,7 +1489,7 @@ __global__ void __launch_bounds__(GFM_TPB) m5_gfm_seq(ffv_dmesh m, ffv_geom g, M
         double vnl = 0.0, wnl = 0.0;
         int ft = 0;
         for (int f = 0; f < 6; f++) {
-          if (GF[(int64_t)f * m.n + c]) {
+          if (GF[(int64_t)f * m.n + c] & FFV_FACE_GFM) {
             const double A = g.area[ffv_face_kind(info, f) == FFV_FK_FINER ? l + 1 : l];
             const double vl = ug[ft] * n1x + vg[ft] * n1y + wg[ft] * n1z;
             const double wl = ug[ft] * n2x + vg[ft] * n2y + wg[ft] * n2z;
@@ -1984,8 +1984,8 @@ struct Rec {
 
 template <int N>
 static void stage_impl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
-                       const ffv_m5_bufs &b, int irk, cudaStream_t st, cudaEvent_t *ev,
-                       const char **names) {
+                       const ffv_m5_bufs &b, int irk, bool follows, cudaStream_t st,
+                       cudaEvent_t *ev, const char **names) {
   const int tpb = 128;
   const unsigned gc = (unsigned)((m.n + tpb - 1) / tpb);
   Rec rec{ev, 0, names, st};
@@ -1996,9 +1996,9 @@ static void stage_impl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
   if (k.order == 2) {
     if (f32) {
       // the FP32 copy of the state lives in RHS, which m5_cell_update writes later
-      ffv_m5f_shadow(m.n, k, b.S, (float *)b.RHS, st);
+      ffv_m5f_shadow(m.n, k, b.S, (float *)b.RHS, b.flat, follows, st);
       rec("m5f_shadow");
-      ffv_m5f_recon(m, g, k, b.S, (float *)b.RHS, SFf, b.status, st);
+      ffv_m5f_recon(m, g, k, (float *)b.RHS, b.flat, SFf, b.status, st);
       rec("m5f_recon_face");
     } else {
       m5_recon_slopes<N><<<dim3(gc, 3), tpb, 0, st>>>(m, g, k, b.S, b.SF);
@@ -2009,16 +2009,16 @@ static void stage_impl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
     }
   }
   if (f32)
-    ffv_m5f_flux(m, g, k, b.S, k.order == 2 ? (const float *)b.RHS : nullptr, SFf, FFf, UFf, b.GF,
-                 b.list_faces, b.status, st);
+    ffv_m5f_flux(m, g, k, b.S, k.order == 2 ? (const float *)b.RHS : nullptr, SFf, b.flat, FFf, UFf,
+                 b.GF, b.list_faces, b.status, st);
   else
     (k.order == 2 ? m5_face_flux<N, 2> : m5_face_flux<N, 1>)
         <<<ffv_flux_blocks(b.list_faces, m.n), FFV_LIST_TPB, 0, st>>>(
             m, g, k, b.list_faces, b.S, b.SF, b.FF, b.UF, b.GF, b.status);
   rec(f32 ? "m5f_face_flux" : "m5_face_flux");
   if (f32)
-    ffv_m5f_cell_update(m, g, k, b.S, b.SN, FFf, UFf, b.RHS, b.Snew, b.flag, b.list, b.dt, irk,
-                        b.status, st);
+    ffv_m5f_cell_update(m, g, k, b.S, b.SN, FFf, UFf, b.GF, b.flat, b.RHS, b.Snew, b.flag, b.list,
+                        b.dt, irk, b.status, st);
   else
     m5_cell_update<N><<<gc, tpb, 0, st>>>(m, g, k, b.S, b.SN, b.FF, b.UF, b.RHS, b.Snew,
                                           b.flag, b.list, b.dt, irk, b.status);
@@ -2028,7 +2028,7 @@ static void stage_impl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
                                          b.dt, 0);
     rec("m5_gfm_seq");
   }
-  if (f32) ffv_m5f_relax_cell(m.n, k, b.Snew, b.S, b.flag, b.list, b.status, st);
+  if (f32) ffv_m5f_relax_cell(m.n, k, b.Snew, b.flat, b.S, b.flag, b.list, b.status, st);
   else
     (fast ? m5_relax_cell<N, true> : m5_relax_cell<N, false>)<<<gc, tpb, 0, st>>>(
         m.n, k, b.Snew, b.S, b.flag, b.list, b.status);
@@ -2040,10 +2040,10 @@ static void stage_impl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
 }
 
 void ffv_m5_fp64_stage(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k,
-                       const ffv_m5_bufs &b, int irk, cudaStream_t st, cudaEvent_t *ev,
-                       const char **names) {
-  if (k.nmat == 2) stage_impl<2>(m, g, k, b, irk, st, ev, names);
-  else stage_impl<3>(m, g, k, b, irk, st, ev, names);
+                       const ffv_m5_bufs &b, int irk, bool follows, cudaStream_t st,
+                       cudaEvent_t *ev, const char **names) {
+  if (k.nmat == 2) stage_impl<2>(m, g, k, b, irk, follows, st, ev, names);
+  else stage_impl<3>(m, g, k, b, irk, follows, st, ev, names);
 }
 
 int ffv_m5_launches_per_stage(const M5Consts &k, int irk) {
