@@ -68,16 +68,13 @@ __global__ void __launch_bounds__(128) m0_tag_split(ffv_dmesh m, double gamma, d
 
 __global__ void __launch_bounds__(128) m0_indicator_fields(int64_t n, double gamma, double pinf,
                                                            const double *__restrict__ S,
-                                                           float *__restrict__ F) {
+                                                           ffv_field_out out) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   double r, p, um;
   m0_prim(S, n, c, gamma, pinf, r, p, um);
-  F[c] = (float)log(r > 1e-300 ? r : 1e-300);
-  F[n + c] = (float)log(p > 1e-30 ? p : 1e-30);
-  F[2 * n + c] = 1.0f;
-  F[3 * n + c] = (float)um;
-  F[4 * n + c] = 0.0f;
+  const float f[5] = {(float)log(r > 1e-300 ? r : 1e-300), (float)log(p > 1e-30 ? p : 1e-30), 1.0f, (float)um, 0.0f};
+  out.put(n, c, f);
 }
 
 __global__ void __launch_bounds__(128) m0_export_fields(int64_t n, double gamma, double pinf,
@@ -106,7 +103,7 @@ void ffv_m0_tags(const ffv_dmesh &m, double gamma, double pinf, const ffv_m5_tag
   m0_tag_split<<<(unsigned)((m.n + 127) / 128), 128, 0, st>>>(m, gamma, pinf, t, S, split);
 }
 
-void ffv_m0_indicator_fields(int64_t n, double gamma, double pinf, const double *S, float *F,
-                             cudaStream_t st) {
-  m0_indicator_fields<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(n, gamma, pinf, S, F);
+void ffv_m0_indicator_fields(int64_t n, double gamma, double pinf, const double *S,
+                             const ffv_field_out &out, cudaStream_t st) {
+  m0_indicator_fields<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(n, gamma, pinf, S, out);
 }

@@ -1,5 +1,6 @@
 // Model-5 launch interface (ffv_m5_fp64.cu).
 #pragma once
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -94,9 +95,28 @@ void ffv_m5f_cell_update(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &
                          const FlatMarks &fm, double *RHS, double *Snew, uint8_t *flag,
                          int32_t *list, const double *dt, int irk, unsigned *status,
                          cudaStream_t st);
-// the indicator's fields of a model-5 state, F [5][n] float (log rho, log p, alpha_0, |u|,
-// von Mises stress; FP32 with double-float pressure recovery; ffv_mlp.cu gathers them)
-void ffv_m5f_indicator_fields(int64_t n, const M5Consts &k, const double *S, float *F,
+// where the indicator's fields of a cell go: F [5][n], or, with R, one 16-byte record [n] of the five
+// normalised by norm (means, standard deviations) and rounded to BF16, as the perceptron takes them
+struct ffv_field_out {
+  float *F;
+  uint4 *R;
+  const float *norm;
+  __device__ __forceinline__ void put(int64_t n, int64_t c, const float f[5]) const {
+    if (!R) {
+#pragma unroll
+      for (int q = 0; q < 5; q++) F[q * n + c] = f[q];
+      return;
+    }
+    uint32_t h[5];
+#pragma unroll
+    for (int q = 0; q < 5; q++)
+      h[q] = __bfloat16_as_ushort(__float2bfloat16_rn((f[q] - norm[q]) * (1.0f / norm[5 + q])));
+    R[c] = make_uint4(h[0] | h[1] << 16, h[2] | h[3] << 16, h[4], 0u);
+  }
+};
+// the indicator's fields of a model-5 state (log rho, log p, alpha_0, |u|, von Mises stress; FP32
+// with double-float pressure recovery; ffv_mlp.cu gathers them)
+void ffv_m5f_indicator_fields(int64_t n, const M5Consts &k, const double *S, const ffv_field_out &out,
                               cudaStream_t st);
 // cell pressure relaxation: the Newton iteration in FP32, the pressure recovery and the
 // energy-consistent pressure and internal energies in double-float
@@ -133,8 +153,8 @@ void ffv_m0_export_fields(int64_t n, double gamma, double pinf, const double *S,
 // fields (log rho, log p, 1, |u|, 0)
 void ffv_m0_tags(const ffv_dmesh &m, double gamma, double pinf, const ffv_m5_tagc &t,
                  const double *S, int32_t *split, cudaStream_t st);
-void ffv_m0_indicator_fields(int64_t n, double gamma, double pinf, const double *S, float *F,
-                             cudaStream_t st);
+void ffv_m0_indicator_fields(int64_t n, double gamma, double pinf, const double *S,
+                             const ffv_field_out &out, cudaStream_t st);
 
 // the reference's FP64 relaxation of the cells a mesh adaptation merged (map < 0)
 void ffv_m5_relax_merged(int64_t n, const M5Consts &k, const int64_t *map, double *S,

@@ -1803,18 +1803,20 @@ __global__ void __launch_bounds__(128, 7) m5f_relax_cell(int64_t n, M5Consts k,
 template <int N>
 __global__ void __launch_bounds__(128) m5f_indicator_fields(int64_t n, M5Consts k,
                                                             const double *__restrict__ S,
-                                                            float *__restrict__ F) {
+                                                            ffv_field_out out) {
   using C = K5<N>;
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
+  // all loads ahead of the conversions, whose branches they do not pass
+  double s[C::NEQ];
+  load_state<N>(S, n, c, s);
   float r = 0.0f;
 #pragma unroll
-  for (int iv = 0; iv < N; ++iv) r += f32_of_f64(S[(int64_t)(C::i0 + iv) * n + c]);
-  const float mx = f32_of_f64(S[(int64_t)C::i1 * n + c]), my = f32_of_f64(S[(int64_t)(C::i1 + 1) * n + c]),
-              mz = f32_of_f64(S[(int64_t)(C::i1 + 2) * n + c]);
+  for (int iv = 0; iv < N; ++iv) r += f32_of_f64(s[C::i0 + iv]);
+  const float mx = f32_of_f64(s[C::i1]), my = f32_of_f64(s[C::i1 + 1]), mz = f32_of_f64(s[C::i1 + 2]);
   df at[N];
 #pragma unroll
-  for (int i = 0; i < N - 1; ++i) at[i] = df_from_double(S[(int64_t)(C::i3 + i) * n + c]);
+  for (int i = 0; i < N - 1; ++i) at[i] = df_from_double(s[C::i3 + i]);
   avf_limit_df<N>(k, at);
   df sum = df_make(0.0f);
 #pragma unroll
@@ -1822,8 +1824,7 @@ __global__ void __launch_bounds__(128) m5f_indicator_fields(int64_t n, M5Consts 
   at[N - 1] = df_sub(df_make(1.0f), sum);
   float D[9];
 #pragma unroll
-  for (int q = 0; q < 9; q++)
-    D[q] = f32_of_f64(S[(int64_t)(C::i5 + q) * n + c] - ((q == 0 || q == 4 || q == 8) ? 1.0 : 0.0));
+  for (int q = 0; q < 9; q++) D[q] = dev_of(s + C::i5, q);
   StrainF sE;
   strain_f(D, sE);
   stress_deviator_f(sE);
@@ -1832,8 +1833,7 @@ __global__ void __launch_bounds__(128) m5f_indicator_fields(int64_t n, M5Consts 
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     const float ael = elastic_energy_f(sE, k.mu_f[i]);
-    const df pk = df_sub(df_div(df_mul(k.gm1_d[i], df_add_f(df_from_double(S[(int64_t)(C::i4 + i) * n + c]), -ael)),
-                                at[i]),
+    const df pk = df_sub(df_div(df_mul(k.gm1_d[i], df_add_f(df_from_double(s[C::i4 + i]), -ael)), at[i]),
                          k.gpi_d[i]);
     p = df_add(p, df_mul(at[i], pk));
     // the von Mises stress depends on the deviator only, to which -alpha_k p_k I adds
@@ -1851,11 +1851,9 @@ __global__ void __launch_bounds__(128) m5f_indicator_fields(int64_t n, M5Consts 
       j2 += d * d;
     }
   const float pf = df_to_float(p);
-  F[c] = logf(fmaxf(r, 1e-30f));
-  F[n + c] = logf(fmaxf(pf, 1.0f));
-  F[2 * n + c] = df_to_float(at[0]);
-  F[3 * n + c] = sqrtf(mx * mx + my * my + mz * mz) / r;
-  F[4 * n + c] = sqrtf(1.5f * j2);
+  const float f[5] = {logf(fmaxf(r, 1e-30f)), logf(fmaxf(pf, 1.0f)), df_to_float(at[0]),
+                      sqrtf(mx * mx + my * my + mz * mz) / r, sqrtf(1.5f * j2)};
+  out.put(n, c, f);
 }
 
 }  // namespace
@@ -1900,11 +1898,11 @@ void ffv_m5f_cell_update(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &
   kernel<<<blocks, 128, 0, st>>>(m, g, k, S, SN, FFf, UFf, GF, fm, RHS, Snew, flag, list, dt, irk, status);
 }
 
-void ffv_m5f_indicator_fields(int64_t n, const M5Consts &k, const double *S, float *F,
+void ffv_m5f_indicator_fields(int64_t n, const M5Consts &k, const double *S, const ffv_field_out &out,
                               cudaStream_t st) {
   const unsigned blocks = (unsigned)((n + 127) / 128);
-  if (k.nmat == 2) m5f_indicator_fields<2><<<blocks, 128, 0, st>>>(n, k, S, F);
-  else m5f_indicator_fields<3><<<blocks, 128, 0, st>>>(n, k, S, F);
+  if (k.nmat == 2) m5f_indicator_fields<2><<<blocks, 128, 0, st>>>(n, k, S, out);
+  else m5f_indicator_fields<3><<<blocks, 128, 0, st>>>(n, k, S, out);
 }
 
 void ffv_m5f_relax_cell(int64_t n, const M5Consts &k, const double *Sin, const FlatMarks &fm,

@@ -93,25 +93,28 @@ __device__ __forceinline__ void stencil27(const ffv_dmesh &m, int32_t c, int32_t
 }
 
 // the 135 normalised features of a cell as BF16, eight per 16-byte chunk (chunk 16 holds
-// features 128-134 and a zero, chunk 17 zeros), handed to put(chunk, uint4)
+// features 128-134 and a zero, chunk 17 zeros), handed to put(chunk, uint4).  A stencil cell's five
+// come as one record: a value is normalised and rounded once, where its cell's fields are formed,
+// and not by each of the 27 rows that take it, and a row's gather is 27 loads instead of 135.
 template <typename Put>
-__device__ __forceinline__ void cell_features(const ffv_dmesh &m, const float *__restrict__ F,
-                                              const float mean[5], const float istd[5], int32_t c,
-                                              Put put) {
+__device__ __forceinline__ void cell_features(const ffv_dmesh &m, const uint4 *__restrict__ R,
+                                              int32_t c, Put put) {
   int32_t e[27];
   stencil27(m, c, e);
   uint32_t w[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-  for (int o = 0; o < 27; o++)
+  for (int o = 0; o < 27; o++) {
+    const uint4 r = R[e[o]];
 #pragma unroll
     for (int q = 0; q < 5; q++) {
       const int k = 5 * o + q;
-      const bf16 v = __float2bfloat16_rn((F[(int64_t)q * m.n + e[o]] - mean[q]) * istd[q]);
-      const uint32_t u = __bfloat16_as_ushort(v);
+      const uint32_t pair = q < 2 ? r.x : (q < 4 ? r.y : r.z);
+      const uint32_t u = (q & 1) ? pair >> 16 : pair & 0xFFFFu;
       if ((k & 1) == 0) w[(k & 7) >> 1] = u;
       else w[(k & 7) >> 1] |= u << 16;
       if ((k & 7) == 7) put(k >> 3, make_uint4(w[0], w[1], w[2], w[3]));
     }
+  }
   put(NIN >> 3, make_uint4(w[0], w[1], w[2], w[3] & 0xFFFFu));
   put(KIN / 8 - 1, make_uint4(0u, 0u, 0u, 0u));
 }
@@ -121,21 +124,14 @@ __device__ __forceinline__ void cell_features(const ffv_dmesh &m, const float *_
 // then writes them out as one contiguous run of 4-byte words: a thread writing its own
 // 288-byte row directly would touch 32 cache lines per warp store.
 constexpr int GATHER_TPB = 128, GATHER_SW = 73;  // shared words per row (KIN / 2 = 72, +1)
-__global__ void __launch_bounds__(GATHER_TPB) mlp_gather(ffv_dmesh m, const float *__restrict__ F,
-                                                         const float *__restrict__ norm,
+__global__ void __launch_bounds__(GATHER_TPB) mlp_gather(ffv_dmesh m, const uint4 *__restrict__ R,
                                                          bf16 *__restrict__ X) {
   __shared__ uint32_t tile[GATHER_TPB * GATHER_SW];
   const int64_t c0 = (int64_t)blockIdx.x * GATHER_TPB;
   const int64_t c = c0 + threadIdx.x;
   if (c < m.n) {
-    float mean[5], istd[5];
-#pragma unroll
-    for (int q = 0; q < 5; q++) {
-      mean[q] = norm[q];
-      istd[q] = 1.0f / norm[5 + q];
-    }
     uint32_t *row = tile + threadIdx.x * GATHER_SW;
-    cell_features(m, F, mean, istd, (int32_t)c, [&](int ch, uint4 v) {
+    cell_features(m, R, (int32_t)c, [&](int ch, uint4 v) {
       row[4 * ch] = v.x;
       row[4 * ch + 1] = v.y;
       row[4 * ch + 2] = v.z;
@@ -188,8 +184,7 @@ static_assert(TC_TMEM_COLS * TC_CTAS_PER_SM <= 512, "tensor memory of three CTAs
 
 template <bool GATHER>
 __global__ void __launch_bounds__(TC_ROWS, TC_CTAS_PER_SM)
-    mlp_infer_tc(ffv_dmesh m, const float *__restrict__ F, const float *__restrict__ norm,
-                 const bf16 *__restrict__ X, int64_t n, const bf16 *__restrict__ W1,
+    mlp_infer_tc(ffv_dmesh m, const uint4 *__restrict__ R, const bf16 *__restrict__ X, int64_t n, const bf16 *__restrict__ W1,
                  const bf16 *__restrict__ W2, const float *__restrict__ P, float *__restrict__ prob,
                  uint8_t *__restrict__ marks, float threshold, int accumulate,
                  unsigned *__restrict__ err) {
@@ -224,12 +219,6 @@ __global__ void __launch_bounds__(TC_ROWS, TC_CTAS_PER_SM)
                  w2s = tc::smem_addr(sm + TC_W2);
   constexpr uint32_t idesc = tc::idesc_bf16_f32(TC_ROWS, NH);
   const float b3 = P[OFF_B3];
-  float mean[5], istd[5];
-#pragma unroll
-  for (int q = 0; q < 5; q++) {
-    mean[q] = GATHER ? norm[q] : 0.0f;
-    istd[q] = GATHER ? 1.0f / norm[5 + q] : 1.0f;
-  }
   const int64_t ntiles = (n + TC_ROWS - 1) / TC_ROWS;
   int failed_parity = -1;
   for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -242,7 +231,7 @@ __global__ void __launch_bounds__(TC_ROWS, TC_CTAS_PER_SM)
 #pragma unroll 1
       for (int ch = 0; ch < KIN / 8; ch++) put(ch, make_uint4(0u, 0u, 0u, 0u));
     } else if (GATHER) {
-      cell_features(m, F, mean, istd, (int32_t)c, put);
+      cell_features(m, R, (int32_t)c, put);
     } else {
 #pragma unroll
       for (int ch = 0; ch < KIN / 8; ch++) put(ch, *reinterpret_cast<const uint4 *>(X + c * KIN + 8 * ch));
@@ -264,7 +253,9 @@ __global__ void __launch_bounds__(TC_ROWS, TC_CTAS_PER_SM)
       break;
     }
     tc::fence_after_sync();
-#pragma unroll
+    // rolled, like the loop of layer 2: 128 erff in line are 80 KB of code, which every warp then
+    // waited for (1.7 M cells: 696 -> 531 us)
+#pragma unroll 1
     for (int c0 = 0; c0 < NH; c0 += 16) {
       float a[16];
       tc::tmem_ld16(row_tmem + c0, a);
@@ -294,7 +285,7 @@ __global__ void __launch_bounds__(TC_ROWS, TC_CTAS_PER_SM)
     }
     tc::fence_after_sync();
     float z = 0.0f;
-#pragma unroll
+#pragma unroll 1
     for (int c0 = 0; c0 < NH; c0 += 16) {
       float a[16];
       tc::tmem_ld16(row_tmem + c0, a);
@@ -668,7 +659,8 @@ struct ffv_mlp {
   int64_t cap_losses;
   // predict buffers
   int64_t cap;
-  float *d_F, *d_prob;
+  uint4 *d_R;  // records of the mesh's cells
+  float *d_prob;
   // inference wait timeouts: mapped pinned word, set by the device, read by the host
   unsigned *h_err, *d_err;
 };
@@ -688,11 +680,12 @@ int repack(ffv_mlp *m) {
 
 int ensure_cap(ffv_mlp *m, int64_t n) {
   if (m->cap >= n) return FFV_OK;
-  cudaFree(m->d_F);
+  cudaFree(m->d_R);
   cudaFree(m->d_prob);
-  m->d_F = m->d_prob = nullptr;
+  m->d_R = nullptr;
+  m->d_prob = nullptr;
   m->cap = 0;
-  if (cudaMalloc(&m->d_F, sizeof(float) * 5 * n) != cudaSuccess ||
+  if (cudaMalloc(&m->d_R, sizeof(uint4) * n) != cudaSuccess ||
       cudaMalloc(&m->d_prob, sizeof(float) * n) != cudaSuccess)
     return FFV_ERR_NOMEM;
   m->cap = n;
@@ -700,8 +693,8 @@ int ensure_cap(ffv_mlp *m, int64_t n) {
 }
 
 // the fused inference kernel over n rows: feature rows X (dm unused), or the stencil gather
-// of the fields F on mesh dm (X unused); probabilities and/or marks out
-int infer(ffv_mlp *m, bool gather, const ffv_dmesh &dm, const float *F, const bf16 *X, int64_t n,
+// of the cells' records R on mesh dm (X unused); probabilities and/or marks out
+int infer(ffv_mlp *m, bool gather, const ffv_dmesh &dm, const uint4 *R, const bf16 *X, int64_t n,
           float *prob, uint8_t *marks, float threshold, int accumulate, cudaStream_t st) {
   if (n <= 0) return FFV_OK;
   const int64_t tiles = (n + TC_ROWS - 1) / TC_ROWS;
@@ -710,11 +703,11 @@ int infer(ffv_mlp *m, bool gather, const ffv_dmesh &dm, const float *F, const bf
   if (gather) {
     MCK(cudaFuncSetAttribute(mlp_infer_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
     mlp_infer_tc<true><<<(unsigned)blocks, TC_ROWS, TC_SMEM, st>>>(
-        dm, F, m->d_norm, nullptr, n, m->d_W1, m->d_W2, m->d_P, prob, marks, threshold, accumulate, m->d_err);
+        dm, R, nullptr, n, m->d_W1, m->d_W2, m->d_P, prob, marks, threshold, accumulate, m->d_err);
   } else {
     MCK(cudaFuncSetAttribute(mlp_infer_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
     mlp_infer_tc<false><<<(unsigned)blocks, TC_ROWS, TC_SMEM, st>>>(
-        dm, nullptr, nullptr, X, n, m->d_W1, m->d_W2, m->d_P, prob, marks, threshold, accumulate, m->d_err);
+        dm, nullptr, X, n, m->d_W1, m->d_W2, m->d_P, prob, marks, threshold, accumulate, m->d_err);
   }
   return mlp_cuda(cudaGetLastError());
 }
@@ -795,10 +788,11 @@ struct CtxView {
 int view(ffv_ctx *ctx, CtxView &v) {
   return ffv_ctx_view(ctx, &v.device, &v.st, &v.dm, &v.S, &v.k, &v.model, &v.gamma0, &v.pinf0);
 }
-void launch_fields(const CtxView &v, float *F) {
-  if (v.model == 5) ffv_m5f_indicator_fields(v.dm.n, *v.k, v.S, F, v.st);
-  else ffv_m0_indicator_fields(v.dm.n, v.gamma0, v.pinf0, v.S, F, v.st);
+void launch_fields(const CtxView &v, const ffv_field_out &out) {
+  if (v.model == 5) ffv_m5f_indicator_fields(v.dm.n, *v.k, v.S, out, v.st);
+  else ffv_m0_indicator_fields(v.dm.n, v.gamma0, v.pinf0, v.S, out, v.st);
 }
+void launch_records(const CtxView &v, ffv_mlp *m) { launch_fields(v, {nullptr, m->d_R, m->d_norm}); }
 }  // namespace
 
 extern "C" {
@@ -865,7 +859,7 @@ int ffv_mlp_destroy(ffv_mlp *m) {
   cudaFree(m->d_W1);
   cudaFree(m->d_W2);
   cudaFree(m->d_W2T);
-  cudaFree(m->d_F);
+  cudaFree(m->d_R);
   cudaFree(m->d_prob);
   cudaFree(m->d_part);
   cudaFree(m->d_losses);
@@ -916,7 +910,7 @@ int ffv_mlp_fields(ffv_ctx *ctx, float *F_dev) {
   if (rc != FFV_OK) return rc;
   if (!F_dev) return FFV_ERR_ARG;
   MCK(cudaSetDevice(v.device));
-  launch_fields(v, F_dev);
+  launch_fields(v, {F_dev, nullptr, nullptr});
   MCK(cudaGetLastError());
   MCK(cudaStreamSynchronize(v.st));
   return FFV_OK;
@@ -931,9 +925,8 @@ int ffv_mlp_features(ffv_ctx *ctx, ffv_mlp *m, void *X_dev) {
   MCK(cudaSetDevice(v.device));
   rc = ensure_cap(m, v.dm.n);
   if (rc != FFV_OK) return rc;
-  launch_fields(v, m->d_F);
-  mlp_gather<<<(unsigned)((v.dm.n + 127) / 128), 128, 0, v.st>>>(v.dm, m->d_F, m->d_norm,
-                                                                  (bf16 *)X_dev);
+  launch_records(v, m);
+  mlp_gather<<<(unsigned)((v.dm.n + 127) / 128), 128, 0, v.st>>>(v.dm, m->d_R, (bf16 *)X_dev);
   MCK(cudaGetLastError());
   MCK(cudaStreamSynchronize(v.st));
   return FFV_OK;
@@ -959,8 +952,8 @@ int ffv_mlp_predict(ffv_ctx *ctx, ffv_mlp *m, float *prob_host) {
   MCK(cudaSetDevice(v.device));
   rc = ensure_cap(m, v.dm.n);
   if (rc != FFV_OK) return rc;
-  launch_fields(v, m->d_F);
-  rc = infer(m, true, v.dm, m->d_F, nullptr, v.dm.n, m->d_prob, nullptr, 0.0f, 0, v.st);
+  launch_records(v, m);
+  rc = infer(m, true, v.dm, m->d_R, nullptr, v.dm.n, m->d_prob, nullptr, 0.0f, 0, v.st);
   if (rc != FFV_OK) return rc;
   MCK(cudaMemcpyAsync(prob_host, m->d_prob, sizeof(float) * v.dm.n, cudaMemcpyDeviceToHost, v.st));
   MCK(cudaStreamSynchronize(v.st));
@@ -980,8 +973,8 @@ int ffv_mlp_mark(ffv_ctx *ctx, ffv_mlp *m, float threshold, uint8_t *marks_dev,
   // a timeout of an earlier call (this call is not waited for)
   rc = take_timeout(m);
   if (rc != FFV_OK) return rc;
-  launch_fields(v, m->d_F);
-  return infer(m, true, v.dm, m->d_F, nullptr, v.dm.n, nullptr, marks_dev, threshold, accumulate, v.st);
+  launch_records(v, m);
+  return infer(m, true, v.dm, m->d_R, nullptr, v.dm.n, nullptr, marks_dev, threshold, accumulate, v.st);
 }
 
 int ffv_mlp_grad(ffv_mlp *m, const void *X_dev, const float *y_dev, int64_t B, float *grad_host,
