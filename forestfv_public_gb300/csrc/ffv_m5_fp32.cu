@@ -991,7 +991,7 @@ __device__ unsigned relax_face_df(const M5Consts &k, float *v, df *cr, bool flat
               pf = c > 0.0f ? exp2f(k.gamma_f[iv] * log2f(a0[iv] / c)) / b0[iv] - pif[iv] : preset[iv];
             }
         } else {
-          const float step = F / dF;
+          const float step = __fdividef(F, dF);  // dF is no better than that
           if (iter > 0 && !(fabsf(step) > 1.0e-7f * fabsf(pf))) break;
           if (iter > 7 && fabsf(step) >= last && fabsf(step) <= 1.0e-4f * fabsf(pf)) break;
           last = fabsf(step);
