@@ -313,7 +313,9 @@ __device__ unsigned star_region_f(const M5Consts &k, const SolF<N> &s, float rL,
   } else {
     SK = SR; uK = uR; vK = vR; wK = wR; s11K = sR[0]; s12K = sR[1]; s13K = sR[2];
   }
-  const float q = (SK - uK) / (SK - u_S);
+  // the quotients by u* - S_K share its reciprocal, each rounded as a division
+  const float w = u_S - SK, ius = __frcp_rn(w);
+  const float q = quotient(uK - SK, w, ius);
   float ar_S[N], r_S = 0.0f;
 #pragma unroll
   for (int v = 0; v < N; ++v) {
@@ -344,7 +346,6 @@ __device__ unsigned star_region_f(const M5Consts &k, const SolF<N> &s, float rL,
   //   A*_0j = (A_0j (uK - SK) - A_1j (vK - v*) + A_2j (wK - w*)) / (u* - SK),
   // rows 1 and 2 unchanged; on D = A - I the identity's share of row 0 is the jump
   // (uK - u*) / (u* - SK), formed as that difference
-  const float ius = 1.0f / (u_S - SK);
   StrainF sE;
   sE.solid = false;
   if (s.flat) {
@@ -381,16 +382,15 @@ __device__ unsigned star_region_f(const M5Consts &k, const SolF<N> &s, float rL,
     const float p_S = (-s.p[v] + pi) * (((ga - 1.0f) * rm + (ga + 1.0f) * rm_S) /
                                        ((ga - 1.0f) * rm_S + (ga + 1.0f) * rm)) - pi;
     const float ael = elastic_energy_f(sE, k.mu_f[v]);
-    const float eel = ael / (s.avf[v] * rm_S);
+    const float eel = ael != 0.0f ? ael / (s.avf[v] * rm_S) : 0.0f;
     const float e_S = (p_S + ga * pi) / (rm_S * (ga + 1.0f)) + eel;
     nc.are[v] = ar_S[v] * e_S;
   }
   if (k.flux_form == FFV_FLUX_CONSISTENT) {
-    const float iw = 1.0f / (SK - u_S);
 #pragma unroll
-    for (int v = 0; v < N; ++v) dU[C::i0 + v] = s.ra[v] * (u_S - uK) * iw;
-    dU[C::i2] = (re * (uK - u_S) - s11K * uK - s12K * vK - s13K * wK + s11_S * u_S + s12_S * v_S +
-                 s13_S * w_S) / (u_S - SK);
+    for (int v = 0; v < N; ++v) dU[C::i0 + v] = s.ra[v] * (u_S - uK) * -ius;
+    dU[C::i2] = quotient(re * (uK - u_S) - s11K * uK - s12K * vK - s13K * wK + s11_S * u_S + s12_S * v_S +
+                             s13_S * w_S, w, ius);
   } else {
 #pragma unroll
     for (int v = 0; v < N; ++v) dU[C::i0 + v] = ar_S[v] - s.vec[C::i0 + v];
@@ -1164,7 +1164,9 @@ __global__ void __launch_bounds__(256) m5f_shadow(int64_t n, const double *__res
 // instead of twice.  Bound by instruction issue (74 % active) and latency; wall mesh of 10.1 M
 // cells 7.47 -> 5.37 ms per stage, 0.41 M 350 -> 253 us, bubble mesh of 2.3 M 1336 -> 954 us.  Six
 // blocks of 192 threads per SM (56 registers): 5.88 ms at four (80), 5.58 at five (64), 5.87 at
-// seven (48); on a mesh that does not fill the chip (15,968 cells) all take the same 36 us.
+// seven (48); on a mesh that does not fill the chip (15,968 cells) all took the same 36 us, with the
+// relaxation's slow starts.  Without those, the deformation of fluid cells and two divisions of
+// three: 5.00 ms, 234 us, 710 us and 25 us; stalls on instruction fetches are now the largest.
 constexpr int RF_CELLS = 32, RF_TPB = 6 * RF_CELLS;
 template <int N>
 __global__ void __launch_bounds__(RF_TPB, 6) m5f_recon_face(ffv_dmesh m, ffv_geom g, M5Consts k,
@@ -1458,8 +1460,9 @@ __device__ __forceinline__ void listed_flux_f(const ffv_dmesh &m, const ffv_geom
 // neighbours the kernel needs few spills (it took ~900 bytes per thread), and the listed faces no
 // longer run as single lanes of its warps: 4.89 -> 2.99 ms per stage on the wall mesh of 10.1 M
 // cells, 240 -> 168 us at 0.41 M, 33 -> 17 us at 15,968 (29 us as two launches, one after the
-// other; 2.91 ms and 166 us on the larger meshes).  Five blocks of 128 threads per SM (3.06 ms at
-// six, 3.40 at four).
+// other; 2.91 ms and 166 us on the larger meshes).  Without the deformation of fluid states 2.89 ms
+// (2.88 at six blocks of 128 threads per SM, 3.12 at four), with the star state's quotients from one
+// reciprocal 2.71 ms.
 template <int N>
 __global__ void __launch_bounds__(FFV_LIST_TPB, 5) m5f_face_flux(
     ffv_dmesh m, ffv_geom g, M5Consts k, ffv_face_list fl, const double *__restrict__ S,
@@ -1760,7 +1763,8 @@ __global__ void __launch_bounds__(128, 3) m5f_cell_update(ffv_dmesh m, ffv_geom 
 }
 
 // 7 blocks of 128 threads per SM: wall mesh of 10.1 M cells 1.18 ms per stage (1.20 at six, 1.23 at
-// five), bubble mesh of 2.3 M 193 us (199 at six)
+// five), bubble mesh of 2.3 M 193 us (199 at six).  Without the deformation of fluid cells and with
+// the Newton's better start 1.08 ms and 133 us, 15,968 cells 53 -> 18 us.
 template <int N>
 __global__ void __launch_bounds__(128, 7) m5f_relax_cell(int64_t n, M5Consts k,
                                                       const double *__restrict__ Sin,
