@@ -354,7 +354,8 @@ constexpr int PART = NPARAM + 1;                   // a block's gradient and los
 struct TrainSmem {
   bf16 W1[NH * SX], W2[NH * SH], W2T[NH * SH];
   bf16 X[TG * SX], H1[TG * SH], DA2[TG * SH], DA1[TG * SH];
-  float b1[NH], b2[NH], w3[NH], y[TG], z[2][TG], cols[3][4][NH], last[2][4];
+  float b1[NH], b2[NH], w3[NH], y[TG], cols[3][4][NH], last[2][4];
+  float logit[NH / 8][TG][4];  // the logits' terms: column tile, sample, lane of its quad
   int64_t row[TG];
 };
 
@@ -365,20 +366,27 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t r[4], const bf16 *p) 
                : "r"(a));
 }
 
-// GELU (exact, erf form) and its derivative from one erf
+// GELU (exact, erf form) and its derivative from one erf.  Every product and sum that BF16 rounding or
+// AdamW's m / sqrt(v) could carry on is rounded as in the kernel that took one warp per 16 samples
+// (explicit forms here, in the logits' terms and in the column sums): the gradient of one 16-sample tile
+// has that kernel's bits.
 __device__ __forceinline__ void gelu_both(float x, float &h, float &d) {
   const float half_cdf = 0.5f * (1.0f + erff(x * 0.70710678118654752f));
   h = x * half_cdf;
-  d = half_cdf + x * 0.39894228040143268f * expf(-0.5f * x * x);
+  d = __fadd_rn(half_cdf, __fmul_rn(__fmul_rn(x, 0.39894228040143268f), expf(-0.5f * x * x)));
 }
 
 // acc[nt] += A^T B over the tile's 64 samples for rows m0 .. m0 + 15 of A^T and NT column tiles from
-// n0 of B; A [64][SH], B [64][sb]
+// n0 of B; A [64][SH], B [64][sb].  Sixteen samples at a time from zero, the products added in FP32:
+// the tensor core's accumulator does not round to nearest, and a chain of products through it grows
+// with the batch (a million samples: entries off by up to 230 * 2^-24 of their terms' magnitudes with
+// the chain, 26 now).  Rolled: four copies of the loop cost more in instruction fetches (40 steps of
+// 8192: 762 us unrolled, 693 rolled, 671 with the chain).
 template <int NT>
 __device__ __forceinline__ void outer_tile(const bf16 *A, int m0, const bf16 *B, int sb, int n0,
                                            float acc[NT][4]) {
   const int lane = threadIdx.x & 31, j = lane >> 3, r = lane & 7;
-#pragma unroll
+#pragma unroll 1
   for (int kk = 0; kk < TG / 16; kk++) {
     uint32_t a[4];  // the 8 x 8 blocks (m, k): (0, 0), (8, 0), (0, 8), (8, 8)
     ldmatrix_x4_trans(a, A + (kk * 16 + (j >> 1) * 8 + r) * SH + m0 + (j & 1) * 8);
@@ -388,8 +396,13 @@ __device__ __forceinline__ void outer_tile(const bf16 *A, int m0, const bf16 *B,
       const int n = n0 + 8 * (nt + 1 < NT ? nt + (j >> 1) : nt);
       uint32_t b[4];
       ldmatrix_x4_trans(b, B + (kk * 16 + (j & 1) * 8 + r) * sb + n);
-      mma16816(acc[nt], a[0], a[1], a[2], a[3], b[0], b[1]);
-      if (nt + 1 < NT) mma16816(acc[nt + 1], a[0], a[1], a[2], a[3], b[2], b[3]);
+#pragma unroll
+      for (int t = 0; t < (nt + 1 < NT ? 2 : 1); t++) {
+        float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        mma16816(c, a[0], a[1], a[2], a[3], b[2 * t], b[2 * t + 1]);
+#pragma unroll
+        for (int e = 0; e < 4; e++) acc[nt + t][e] += c[e];
+      }
     }
   }
 }
@@ -486,26 +499,29 @@ __global__ void __launch_bounds__(TG_TPB) mlp_grad_tiles(const bf16 *__restrict_
       *reinterpret_cast<__nv_bfloat162 *>(s.H1 + (row0 + g + 8) * SH + col) = __floats2bfloat162_rn(h[2], h[3]);
     }
     __syncthreads();
-    // second hidden layer and this warp's half of the logits
-    float h2[4][4], g2[4][4], zg = 0.0f, zg8 = 0.0f;
+    // second hidden layer and this warp's terms of the logits
+    float h2[4][4], g2[4][4];
     rows_times<NH>(s.H1, row0, SH, s.W2, n0, SH, a);
 #pragma unroll
     for (int nt = 0; nt < 4; nt++) {
       const int col = n0 + nt * 8 + 2 * q;
 #pragma unroll
       for (int e = 0; e < 4; e++) gelu_both(a[nt][e] + s.b2[col + (e & 1)], h2[nt][e], g2[nt][e]);
-      zg += h2[nt][0] * s.w3[col] + h2[nt][1] * s.w3[col + 1];
-      zg8 += h2[nt][2] * s.w3[col] + h2[nt][3] * s.w3[col + 1];
-    }
-    zg += __shfl_xor_sync(0xffffffffu, zg, 1);
-    zg += __shfl_xor_sync(0xffffffffu, zg, 2);
-    zg8 += __shfl_xor_sync(0xffffffffu, zg8, 1);
-    zg8 += __shfl_xor_sync(0xffffffffu, zg8, 2);
-    if (q == 0) {
-      s.z[warp >> 2][row0 + g] = zg;
-      s.z[warp >> 2][row0 + g + 8] = zg8;
+      s.logit[(n0 >> 3) + nt][row0 + g][q] =
+          __fmaf_rn(h2[nt][0], s.w3[col], __fmul_rn(h2[nt][1], s.w3[col + 1]));
+      s.logit[(n0 >> 3) + nt][row0 + g + 8][q] =
+          __fmaf_rn(h2[nt][3], s.w3[col + 1], __fmul_rn(h2[nt][2], s.w3[col]));
     }
     __syncthreads();
+    // the logits, formed alike by both warps of a row: a chain over the column tiles, then the quad
+    float z[2] = {0.0f, 0.0f};
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+#pragma unroll
+      for (int nt = 0; nt < NH / 8; nt++) z[e] += s.logit[nt][row0 + g + 8 * e][q];
+      z[e] += __shfl_xor_sync(0xffffffffu, z[e], 1);
+      z[e] += __shfl_xor_sync(0xffffffffu, z[e], 2);
+    }
     // output layer: d loss / d z = (p - y) / B
     float dz[2];
 #pragma unroll
@@ -513,7 +529,7 @@ __global__ void __launch_bounds__(TG_TPB) mlp_grad_tiles(const bf16 *__restrict_
       const int r = row0 + g + 8 * e;
       dz[e] = 0.0f;
       if (r < valid) {
-        const float p = 1.0f / (1.0f + expf(-(s.z[0][r] + s.z[1][r] + b3))), yy = s.y[r];
+        const float p = 1.0f / (1.0f + expf(-(z[e] + b3))), yy = s.y[r];
         dz[e] = (p - yy) * invB;
         if (q == 0 && n0 == 0) {
           db3 += dz[e];
@@ -526,10 +542,11 @@ __global__ void __launch_bounds__(TG_TPB) mlp_grad_tiles(const bf16 *__restrict_
       const int col = n0 + nt * 8 + 2 * q;
       float d[4];
 #pragma unroll
-      for (int e = 0; e < 4; e++) {
-        dw3[nt][e & 1] += dz[e >> 1] * h2[nt][e];
-        d[e] = dz[e >> 1] * s.w3[col + (e & 1)] * g2[nt][e];
-        db2[nt][e & 1] += d[e];
+      for (int e = 0; e < 4; e++) d[e] = __fmul_rn(dz[e >> 1] * s.w3[col + (e & 1)], g2[nt][e]);
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        dw3[nt][e] += __fmaf_rn(dz[0], h2[nt][e], __fmul_rn(dz[1], h2[nt][e + 2]));
+        db2[nt][e] += __fadd_rn(d[e], d[e + 2]);
       }
       *reinterpret_cast<__nv_bfloat162 *>(s.DA2 + (row0 + g) * SH + col) = __floats2bfloat162_rn(d[0], d[1]);
       *reinterpret_cast<__nv_bfloat162 *>(s.DA2 + (row0 + g + 8) * SH + col) = __floats2bfloat162_rn(d[2], d[3]);
@@ -541,10 +558,9 @@ __global__ void __launch_bounds__(TG_TPB) mlp_grad_tiles(const bf16 *__restrict_
     for (int nt = 0; nt < 4; nt++) {
       const int col = n0 + nt * 8 + 2 * q;
 #pragma unroll
-      for (int e = 0; e < 4; e++) {
-        a[nt][e] *= g1[nt][e];
-        db1[nt][e & 1] += a[nt][e];
-      }
+      for (int e = 0; e < 4; e++) a[nt][e] = __fmul_rn(a[nt][e], g1[nt][e]);
+#pragma unroll
+      for (int e = 0; e < 2; e++) db1[nt][e] += __fadd_rn(a[nt][e], a[nt][e + 2]);
       *reinterpret_cast<__nv_bfloat162 *>(s.DA1 + (row0 + g) * SH + col) = __floats2bfloat162_rn(a[nt][0], a[nt][1]);
       *reinterpret_cast<__nv_bfloat162 *>(s.DA1 + (row0 + g + 8) * SH + col) = __floats2bfloat162_rn(a[nt][2], a[nt][3]);
     }
