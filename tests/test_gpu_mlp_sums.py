@@ -1,6 +1,6 @@
 """How the training gradient is summed.  Its rounding points: the gradients of two batches of 16
 samples (one tile of every product, nothing added up between tiles) against recorded ones of the
-kernel that took one warp per 16 samples (tests/golden/indicator_gradient16.npz, recorded on a GB300
+kernel that took one warp per 16 samples (tests/golden/indicator/gradient16.npz, recorded on a GB300
 from its C entry ffv_mlp_grad), to the bit.
 
 And the sum over many tiles: a batch of a million samples that repeats 1024 in order, against the mean
@@ -22,7 +22,7 @@ pytestmark = pytest.mark.gpu
 
 
 def test_gradient_of_one_product_tile(built_lib):
-    g = load_golden("indicator_gradient16")
+    g = load_golden("indicator/gradient16")
     ind = Indicator(seed=5)
     for i, seed in enumerate(g["seeds"]):
         rng = np.random.default_rng(int(seed))
