@@ -1520,13 +1520,83 @@ __global__ void __launch_bounds__(GFM_TPB) m5_gfm_seq(ffv_dmesh m, ffv_geom g, M
   }
 }
 
+// Whether a cell's speed over h is certainly below `fastest` and the cell certainly has one: an upper
+// bound of m5_cfl_kernel's speed in FP32.  c^2 cancels -- a nearly absent stiff material's energy
+// against its p_inf, the liquid's against its own -- so the bound is raised by the rounding of the terms
+// and not of their sum: nine roundings of 6e-8 in all, taken as 1e-6.  The last fraction is formed as a
+// double-float difference (1 - alpha in FP32 is off by 3e-8, of which p_inf = 3.2e10 beside a gas makes
+// 3 % of c^2), and the fractions are within what the exact form leaves alone but for 1e-4 of the limit.
+// The elastic energy only lowers c^2.  It is left out, but where it, or a value that is not finite,
+// could leave a cell without a speed, the cell is not passed over: with eps^2 = |A A^T - I|^2 <= 0.01 it
+// is below 2 mu eps^2 (eigenvalues 1 + l of G, |l| <= eps, sum (l - g)^2 <= (1 + sqrt 3)^2 eps^2 and
+// |G|^(1/6) >= 0.948).
+template <int N>
+__device__ __forceinline__ bool certainly_slower(const M5Consts &k, const double *s, float ih,
+                                                 float fastest) {
+  using C = K5<N>;
+  bool sure = true;
+  float rf = 0.0f, uf = 0.0f, cf = 0.0f, err = 0.0f, softer = 0.0f;
+  df rest = df_make(1.0f);
+  float deformed = 0.0f;  // eps^2, rounding included
+  if (k.nsolids != 0) {
+    float A[9];
+    bool any = false;
+#pragma unroll
+    for (int q = 0; q < 9; q++) {
+      A[q] = f32_of_f64(s[C::i5 + q]);
+      any |= f64::abs_bits(s[C::i5 + q]) != 0;
+    }
+    if (any) {
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = i; j < 3; j++) {
+          const float e = (A[3 * i] * A[3 * j] + A[3 * i + 1] * A[3 * j + 1] + A[3 * i + 2] * A[3 * j + 2]) -
+                          (i == j ? 1.0f : 0.0f);
+          deformed += (i == j ? 1.0f : 2.0f) * e * e;
+        }
+      sure = deformed <= 0.01f;  // (not where it is NaN)
+      deformed = deformed * 1.02f + 1.0e-10f;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const float r = f32_of_f64(s[i]);
+    sure &= r >= 0.0f;
+    rf += r;
+    float a;
+    if (i < N - 1) {
+      const df x = df_from_double(s[C::i3 + (i < N - 1 ? i : 0)]);
+      a = x.hi;
+      sure &= a >= k.alo_f && a <= k.ahi_f;
+      rest = df_sub(rest, x);
+    } else {
+      a = rest.hi;
+      sure &= a >= 0.9999f * k.alo_f;
+    }
+    const float w = k.gamma_f[i] * (k.gamma_f[i] - 1.0f), e = f32_of_f64(s[C::i4 + i]);
+    cf += w * (e - a * k.pinf_f[i]);
+    err += w * (1.0e-6f * (fabsf(e) + a * k.pinf_f[i]) + 1.0e-4f * k.alo_f * k.pinf_f[i]);
+    softer += w * 2.0f * k.mu_f[i] * deformed;
+  }
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const float u = fabsf(f32_of_f64(s[C::i1 + d]));
+    sure &= u <= 3.0e38f;
+    uf = fmaxf(uf, u);
+  }
+  sure &= rf > 1.0e-20f && rf < 1.0e30f && cf > 1.0e-20f && cf > 1.01f * (err + softer);
+  return sure && (uf / rf + sqrtf((cf + err) / rf)) * ih * 1.001f < fastest;
+}
+
 // CFL (new, the reference has a fixed DT): dt = h / (max_a |u_a| + c), mixture sound speed
 // c^2 = sum_k (alpha_k / rho) gamma_k (p_k + p_inf_k) as m5_wave_speeds.c:43-50 forms it.  With the
 // pressure put in, alpha_k (p_k + p_inf_k) = (gamma_k - 1) (alpha rho e_k - e_el - alpha_k p_inf_k)
 // needs no division by a fraction; at a power-of-two spacing the smallest dt is the reciprocal of
-// the largest speed over h.  A cell whose speed, formed in FP32 without the elastic energy (which
-// only lowers it), is below the thread's largest so far by more than FP32's error is passed over.
-// The rest are bound by the FP64 pipe: 360 -> 119 us at 0.61 M cells of the wall mesh.
+// the largest speed over h.  A cell certainly slower than the thread's largest so far is passed
+// over.  The rest are bound by the FP64 pipe: ffv_cfl_dt took 298 / 1404 / 6186 us on wall meshes of
+// 0.41, 2.5 and 10.1 M cells with all cells in FP64, now 150 / 433 / 1773 us (a bound that left out the
+// deformation and the rounding of the terms 112 / 409 / 1331 us).
 template <int N>
 __global__ void m5_cfl_kernel(ffv_dmesh m, ffv_geom g, M5Consts k, const double *__restrict__ S,
                               unsigned long long *out) {
@@ -1539,25 +1609,7 @@ __global__ void m5_cfl_kernel(ffv_dmesh m, ffv_geom g, M5Consts k, const double 
     load_state<N>(S, m.n, c, s);
     const int l = ffv_info_level(m.info[c]);
     const bool scaled = (g.pow2 >> l) & 1u;
-    if (scaled && fastest) {
-      float rf = 0.0f, cf = 0.0f, uf = 0.0f, rest = 1.0f;
-      bool inside = true;  // no fraction that the limits below would move by more than rounding
-#pragma unroll
-      for (int i = 0; i < N; ++i) rf += f32_of_f64(s[i]);
-#pragma unroll
-      for (int i = 0; i < N; ++i) {
-        const float a = i < N - 1 ? f32_of_f64(s[C::i3 + (i < N - 1 ? i : 0)]) : rest;
-        inside &= a >= 0.0f && a <= 1.0f;
-        rest -= a;
-        cf += k.gamma_f[i] * (k.gamma_f[i] - 1.0f) * (f32_of_f64(s[C::i4 + i]) - a * k.pinf_f[i]);
-      }
-#pragma unroll
-      for (int d = 0; d < 3; d++) uf = fmaxf(uf, fabsf(f32_of_f64(s[C::i1 + d])));
-      // the last fraction is 1 - sum: next to 1 FP32 resolves it to 2e-7, against p_inf up to the
-      // energy's own size
-      const float bound = (uf / rf + sqrtf(cf / rf * 1.001f)) * g.idcc_f[l][0] * 1.001f;
-      if (inside && bound < f32_of_f64(f64::of_bits(fastest))) continue;  // (not where either is NaN)
-    }
+    if (scaled && fastest && certainly_slower<N>(k, s, g.idcc_f[l][0], f32_of_f64(f64::of_bits(fastest)))) continue;
     double r = s[0];
 #pragma unroll
     for (int i = 1; i < N; ++i) r += s[i];
@@ -1594,9 +1646,9 @@ __global__ void m5_cfl_kernel(ffv_dmesh m, ffv_geom g, M5Consts k, const double 
     best = (other < best || isnan(other)) ? other : best;
   }
   if ((threadIdx.x & 31) == 0) {
-    const unsigned long long bits =
-        isnan(best) ? 0x7ff8000000000000ULL : (unsigned long long)__double_as_longlong(best);
-    atomicMin(out, best >= 0.0 || isnan(best) ? bits : 0ULL);
+    // a cell without a speed leaves no stable step: 0 (as NaN it would lose to every other warp's
+    // step, and its own warp's cells with it)
+    atomicMin(out, best >= 0.0 ? (unsigned long long)__double_as_longlong(best) : 0ULL);
   }
 }
 
