@@ -584,8 +584,10 @@ __device__ __forceinline__ double rcp_near(double x) {
   return fma(fma(-x, r, 1.0), r, r);
 }
 // y / x, the quotient from that reciprocal corrected by its remainder (Markstein): the rounded
-// quotient but where it lies within ~2^-100 of a midpoint
+// quotient but where it lies within ~2^-100 of a midpoint.  Divisors beyond the reciprocal's range (a
+// material thinned out to 1e-38 kg/m^3) take the division.
 __device__ __forceinline__ double div_near(double y, double x) {
+  if (((uint32_t)(f64::bits(x) >> 52) & 0x7FFu) - 901u > 244u) return f64::div_plain(y, x);
   const double r = rcp_near(x), q = y * r;
   return fma(fma(-q, x, y), r, q);
 }
