@@ -71,21 +71,38 @@ __device__ __forceinline__ df df_mul_f(df x, float b) {
   return fast_two_sum(p.hi, p.lo);
 }
 
-// a / y from r, the correctly rounded reciprocal of y: one correction by the remainder rounds the
-// quotient correctly (Markstein, IBM J. Res. Dev. 34 (1990) 111)
+// a / y from q = a r, r the correctly rounded reciprocal of y: one correction by the remainder rounds
+// the quotient correctly (Markstein, IBM J. Res. Dev. 34 (1990) 111) where the remainder is exact and
+// neither r nor q is subnormal or infinite
+__device__ __forceinline__ float corrected(float a, float y, float r, float q) {
+  return __fmaf_rn(__fmaf_rn(-q, y, a), r, q);
+}
+
+// 2^lo <= |x| < 2^hi (false for infinities and NaN)
+__device__ __forceinline__ bool within(float x, int lo, int hi) {
+  return (cvt_bits(x) & 0x7FFFFFFFu) - ((uint32_t)(127 + lo) << 23) < ((uint32_t)(hi - lo) << 23);
+}
+
+static __device__ __noinline__ float quotient_plain(float a, float y) { return __fdiv_rn(a, y); }
+
+// a / y from r, as the division gives it: operands for which the correction is not exact (zero,
+// infinite and subnormal divisors among them) take the division
 __device__ __forceinline__ float quotient(float a, float y, float r) {
   const float q = __fmul_rn(a, r);
-  return __fmaf_rn(__fmaf_rn(-q, y, a), r, q);
+  if (within(y, -60, 60) && (within(q, -40, 60) || a == 0.0f)) return corrected(a, y, r, q);
+  return quotient_plain(a, y);
 }
 
 // x / y: a quotient from the leading parts, corrected once by the remainder x - q y.  Both quotients
 // share one reciprocal: two divisions, each with its test for the extremes of the range, were a
-// tenth of the reconstruction's time.
+// tenth of the reconstruction's time.  No test is needed here: where the reciprocal is subnormal the
+// second quotient makes up for the first (error below 2^-45 over the whole range, as with two
+// divisions), and a zero or infinite divisor gives NaN either way, from the remainder.
 __device__ __forceinline__ df df_div(df x, df y) {
   const float rc = __frcp_rn(y.hi);
-  const float q1 = quotient(x.hi, y.hi, rc);
+  const float q1 = corrected(x.hi, y.hi, rc, __fmul_rn(x.hi, rc));
   const df r = df_sub(x, df_mul_f(y, q1));
-  return fast_two_sum(q1, quotient(r.hi, y.hi, rc));
+  return fast_two_sum(q1, corrected(r.hi, y.hi, rc, __fmul_rn(r.hi, rc)));
 }
 
 __device__ __forceinline__ float df_to_float(df x) { return __fadd_rn(x.hi, x.lo); }
