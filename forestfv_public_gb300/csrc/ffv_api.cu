@@ -36,7 +36,8 @@ struct ffv_ctx {
   int32_t *d_list;       // flagged cells: count, cells [n], and the face list's 12 cursors
   M5Consts m5;
   // refinement tags
-  uint32_t *d_SI;
+  void *d_SI;    // interface layers, a word of 32 or (si_wide) 64 bits per cell
+  bool si_wide;  // (from the first tags that need them on)
   int32_t *d_SItmp, *d_split;
   double *d_tagpr;  // per-cell mixture pressure and density for the criterion, FP64 and FP32 [3][n]
   // cells and subface groups the mesh buffers are allocated for (a new mesh that fits reuses
@@ -85,6 +86,7 @@ void free_mesh_buffers(ffv_ctx *c) {
   cudaFree(c->d_split);
   cudaFree(c->d_tagpr);
   c->d_SI = nullptr;
+  c->si_wide = false;
   c->d_SItmp = c->d_split = nullptr;
   c->d_tagpr = nullptr;
   c->d_info = nullptr;
@@ -829,8 +831,9 @@ int tags_device(ffv_ctx *c, const ffv_mesh *m, const ffv_tag_params *p, int32_t 
   t.si_max = 0;
   if (p->inter0 == 1 && p->inter1 == 1) t.si_max = t.lrs0 + t.lrs1;
   if (p->inter0 == 1 && p->inter1 == 0) t.si_max = t.lrs0;
-  // layers are kept in 16 bits: more than a forest of FFV_MAX_LEVEL levels is wide
-  if (t.si_max > 65536) t.si_max = 65536;
+  // every layer has a cell of its own: there are at most n.  Beyond 65535 they need wider words
+  if (t.si_max > c->n + 1) t.si_max = (int)(c->n + 1);
+  const bool wide = t.si_max > 65536;
   // inputset.c:106, m5_input.c:53
   int32_t lmax = p->lvl_uniform;
   for (int32_t l : {p->lvl_prs, p->lvl_rho, p->lvl_vel, p->lvl_inter0, p->lvl_inter1})
@@ -840,7 +843,8 @@ int tags_device(ffv_ctx *c, const ffv_mesh *m, const ffv_tag_params *p, int32_t 
   const int64_t n = c->n;
   if (!c->d_split) {  // sized for the mesh buffers' capacity, kept while meshes fit
     const int64_t cap = c->cap;
-    if (cudaMalloc(&c->d_SI, sizeof(uint32_t) * cap) != cudaSuccess ||
+    c->si_wide = wide;
+    if (cudaMalloc(&c->d_SI, (wide ? 8 : 4) * cap) != cudaSuccess ||
         cudaMalloc(&c->d_SItmp, sizeof(int32_t) * (2 * cap + 3)) != cudaSuccess ||
         cudaMalloc(&c->d_split, sizeof(int32_t) * cap) != cudaSuccess ||
         cudaMalloc(&c->d_tagpr, sizeof(double) * 3 * cap) != cudaSuccess) {
@@ -849,17 +853,25 @@ int tags_device(ffv_ctx *c, const ffv_mesh *m, const ffv_tag_params *p, int32_t 
       cudaFree(c->d_split);
       cudaFree(c->d_tagpr);
       c->d_SI = nullptr;
-  c->d_SItmp = c->d_split = nullptr;
+      c->si_wide = false;
+      c->d_SItmp = c->d_split = nullptr;
       c->d_tagpr = nullptr;
       return FFV_ERR_NOMEM;
     }
   }
+  if (wide && !c->si_wide) {
+    void *d = nullptr;
+    if (cudaMalloc(&d, 8 * c->cap) != cudaSuccess) return FFV_ERR_NOMEM;
+    cudaFree(c->d_SI);
+    c->d_SI = d;
+    c->si_wide = true;
+  }
   if (c->p.model == 5) {
-    ffv_m5_tags(c->dm, c->m5, t, c->symmetric, c->d_S, c->d_SI, c->d_SItmp, c->d_split, c->d_tagpr,
-                c->stream);
+    ffv_m5_tags(c->dm, c->m5, t, c->symmetric, c->d_S, c->d_SI, c->si_wide, c->d_SItmp, c->d_split,
+                c->d_tagpr, c->stream);
   } else {
     ffv_m0_tags(c->dm, c->p.gamma[0], c->p.pinf[0], t, c->d_S, c->d_split, c->stream);
-    CK(cudaMemsetAsync(c->d_SI, 0, sizeof(uint32_t) * n, c->stream));
+    CK(cudaMemsetAsync(c->d_SI, 0, (c->si_wide ? 8 : 4) * n, c->stream));
   }
   CK(cudaGetLastError());
   return FFV_OK;
@@ -890,7 +902,7 @@ int ffv_tags(ffv_ctx *c, const ffv_mesh *m, const ffv_tag_params *p, int32_t *sp
   CK(cudaMemcpyAsync(split, c->d_split, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, c->stream));
   if (si) {
     // the lists' space is free once the split levels are formed
-    ffv_m5_si_unpack(n, c->d_SI, c->d_SItmp, c->stream);
+    ffv_m5_si_unpack(n, c->d_SI, c->si_wide, c->d_SItmp, c->stream);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(si, c->d_SItmp, sizeof(int32_t) * 2 * n, cudaMemcpyDeviceToHost, c->stream));
   }
@@ -923,7 +935,7 @@ int ffv_tags_raw(ffv_ctx *c, const ffv_mesh *m, const ffv_tag_params *p, int32_t
                      c->stream));
   if (si) {
     // the lists' space is free once the split levels are formed
-    ffv_m5_si_unpack(n, c->d_SI, c->d_SItmp, c->stream);
+    ffv_m5_si_unpack(n, c->d_SI, c->si_wide, c->d_SItmp, c->stream);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(si, c->d_SItmp, sizeof(int32_t) * 2 * n, cudaMemcpyDeviceToHost, c->stream));
   }

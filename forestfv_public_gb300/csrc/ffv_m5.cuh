@@ -134,14 +134,14 @@ struct ffv_m5_tagc {
   int inter0, lvl0, lrs0, inter1, lvl1, lrs1, si_max;
   double thr_prs, thr_rho, thr_vel;
 };
-// SI [n]: interface layers, SI[0] | SI[1] << 16 (layers below 2^16); lists scratch [2 n + 3];
-// split [n]; symmetric: every cell's face neighbours have it as theirs
+// SI [n]: interface layers, SI[0] | SI[1] << 16, or in 64 bits SI[0] | SI[1] << 32 (wide: layers of
+// 2^16 and more); lists scratch [2 n + 3]; split [n]; symmetric: every cell's face neighbours have it as theirs
 // pr: scratch [3][n] doubles (each cell's mixture pressure and density, made once)
 void ffv_m5_tags(const ffv_dmesh &m, const M5Consts &k, const ffv_m5_tagc &t, bool symmetric,
-                 const double *S, uint32_t *SI, int32_t *lists, int32_t *split, double *pr,
+                 const double *S, void *SI, bool wide, int32_t *lists, int32_t *split, double *pr,
                  cudaStream_t st);
 // the layers as [2][n]
-void ffv_m5_si_unpack(int64_t n, const uint32_t *SI, int32_t *out, cudaStream_t st);
+void ffv_m5_si_unpack(int64_t n, const void *SI, bool wide, int32_t *out, cudaStream_t st);
 
 // exported per-leaf fields, F [nf][n] double (ffv_export_fields)
 void ffv_m5_export_fields(int64_t n, const M5Consts &k, const double *S, double *F,

@@ -1721,7 +1721,13 @@ __global__ void __launch_bounds__(128) m5_tag_cells(int64_t n, M5Consts k, bool 
   }
 }
 
-// Interface layers: one word per cell, SI[0] in its low half, SI[1] in the high one.
+// Interface layers: one word per cell, SI[0] in its low half, SI[1] in the high one; W is 32 bits wide,
+// or 64 where layers beyond 65535 can be asked for (a mesh of more cells than that and as many layers:
+// one word is half the bytes, and 16 bits are enough for all others).
+template <typename W>
+__device__ __forceinline__ int si_low(W w) { return (int)(w & ((W(1) << (4 * sizeof(W))) - 1)); }
+template <typename W>
+__device__ __forceinline__ int si_high(W w) { return (int)(w >> (4 * sizeof(W))); }
 
 // what the neighbours across a face show: hit(neighbour) of any of them, bit v for SI[v]
 template <typename Hit>
@@ -1751,8 +1757,9 @@ __device__ __forceinline__ int first_face(const ffv_dmesh &m, int64_t c, int wan
 
 // interface_location.c:17-46: SI = 1 where phi changes sign across a face (the face loop
 // stops after the first face that shows a change); those cells are listed (list nullable)
+template <typename W>
 __global__ void __launch_bounds__(128) m5_si_first(ffv_dmesh m, const uint8_t *__restrict__ phi,
-                                                   uint32_t *__restrict__ SI,
+                                                   W *__restrict__ SI,
                                                    int32_t *__restrict__ list,
                                                    int32_t *__restrict__ count) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1763,7 +1770,7 @@ __global__ void __launch_bounds__(128) m5_si_first(ffv_dmesh m, const uint8_t *_
       const uint32_t x = own ^ phi[o];
       return ((x & 3u) == 2u ? 1 : 0) | ((x >> 2) == 2u ? 2 : 0);
     });
-    SI[c] = (set & 1) | (uint32_t)(set >> 1) << 16;
+    SI[c] = (W)(set & 1) | (W)(set >> 1) << (4 * sizeof(W));
   }
   if (!list) return;
   const unsigned b = __ballot_sync(0xffffffffu, set != 0);
@@ -1779,19 +1786,22 @@ __global__ void __launch_bounds__(128) m5_si_first(ffv_dmesh m, const uint8_t *_
 // neighbours' layer lvl - 1.  The reference updates in place in leaf order, but a cell only reads
 // neighbours' lvl - 1 entries and only writes lvl into entries that were 0, so updating in place in
 // any order gives the same result (an entry that already is lvl was 0 before this layer).
-__device__ __forceinline__ int si_free(uint32_t w, int lvl) {
-  const int s0 = w & 0xffff, s1 = w >> 16;
+template <typename W>
+__device__ __forceinline__ int si_free(W w, int lvl) {
+  const int s0 = si_low(w), s1 = si_high(w);
   return (s0 == 0 || s0 == lvl ? 1 : 0) | (s1 == 0 || s1 == lvl ? 2 : 0);
 }
-__device__ __forceinline__ int si_is(uint32_t w, int lvl) {
-  return ((int)(w & 0xffff) == lvl ? 1 : 0) | ((int)(w >> 16) == lvl ? 2 : 0);
+template <typename W>
+__device__ __forceinline__ int si_is(W w, int lvl) {
+  return (si_low(w) == lvl ? 1 : 0) | (si_high(w) == lvl ? 2 : 0);
 }
-__device__ __forceinline__ int si_set(const ffv_dmesh &m, int lvl, const uint32_t *SI, int64_t c,
-                                      int free) {
+template <typename W>
+__device__ __forceinline__ int si_set(const ffv_dmesh &m, int lvl, const W *SI, int64_t c, int free) {
   return first_face(m, c, free, [&](int32_t o) { return si_is(__ldcg(SI + o), lvl - 1); });
 }
-__device__ __forceinline__ uint32_t si_word(int set, int lvl) {
-  return (set & 1 ? (uint32_t)lvl : 0u) | (set & 2 ? (uint32_t)lvl << 16 : 0u);
+template <typename W>
+__device__ __forceinline__ W si_word(int set, int lvl) {
+  return (set & 1 ? (W)lvl : W(0)) | (set & 2 ? (W)lvl << (4 * sizeof(W)) : W(0));
 }
 
 // Layer lvl from the cells that layer lvl - 1 set: only their neighbours can be next to it.  A
@@ -1799,7 +1809,8 @@ __device__ __forceinline__ uint32_t si_word(int set, int lvl) {
 // entry lists it for the next layer.  Bound by the latency of its chain of loads, so every SM is
 // filled.  The criterion's device part (cells, fourteen layers, split) took ~2.9 ms on the wall mesh
 // of 2.5 M cells with every layer over all cells and FP64 jumps and signs; now ~0.8 ms.
-__global__ void __launch_bounds__(128) m5_si_grow(ffv_dmesh m, int lvl, uint32_t *SI,
+template <typename W>
+__global__ void __launch_bounds__(128) m5_si_grow(ffv_dmesh m, int lvl, W *SI,
                                                   const int32_t *__restrict__ from,
                                                   int32_t *__restrict__ to, int32_t *count) {
   const int n_from = count[(lvl - 1) % 3];
@@ -1816,9 +1827,9 @@ __global__ void __launch_bounds__(128) m5_si_grow(ffv_dmesh m, int lvl, uint32_t
       if (!(free & mine)) return 0;
       const int set = si_set(m, lvl, SI, c, free);
       if (!set) return 0;
-      const uint32_t before = atomicOr(SI + c, si_word(set, lvl));
+      const W before = atomicOr(SI + c, si_word<W>(set, lvl));
       // the first of its visitors to set its first entry
-      if ((before & (set & 1 ? 0xffffu : 0xffff0000u)) == 0) to[atomicAdd(count + lvl % 3, 1)] = c;
+      if ((set & 1 ? si_low(before) : si_high(before)) == 0) to[atomicAdd(count + lvl % 3, 1)] = c;
       return 0;
     };
     face_shows(m, ffv_face_kind(m.info[b], face), m.nbr[(int64_t)face * m.n + b], visit);
@@ -1827,24 +1838,26 @@ __global__ void __launch_bounds__(128) m5_si_grow(ffv_dmesh m, int lvl, uint32_t
 
 // layer lvl over all cells: meshes whose neighbour relation is not symmetric (a part of a forest:
 // a fine cell sees a coarser one whose own face towards it became a boundary)
-__global__ void __launch_bounds__(128) m5_si_layer(ffv_dmesh m, int lvl, uint32_t *SI) {
+template <typename W>
+__global__ void __launch_bounds__(128) m5_si_layer(ffv_dmesh m, int lvl, W *SI) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.n) return;
-  const uint32_t w = SI[c];
+  const W w = SI[c];
   const int free = si_free(w, lvl);
   if (free == 0) return;
   const int set = si_set(m, lvl, SI, c, free);
-  if (set) SI[c] = w | si_word(set, lvl);
+  if (set) SI[c] = w | si_word<W>(set, lvl);
 }
 
 // the layers as two arrays
-__global__ void __launch_bounds__(256) m5_si_unpack(int64_t n, const uint32_t *__restrict__ SI,
+template <typename W>
+__global__ void __launch_bounds__(256) m5_si_unpack(int64_t n, const W *__restrict__ SI,
                                                     int32_t *__restrict__ out) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
-  const uint32_t w = SI[c];
-  out[c] = (int32_t)(w & 0xffff);
-  out[n + c] = (int32_t)(w >> 16);
+  const W w = SI[c];
+  out[c] = si_low(w);
+  out[n + c] = si_high(w);
 }
 
 // relative jump |x_nb - x| / max(|x_nb|, |x|) (criterionsplt.c:83-89), 0 below 1e-8
@@ -1874,8 +1887,9 @@ __device__ __forceinline__ bool jump_reaches(double thr, float thr_f, const doub
 // criterionsplt.c:3-140 per cell: the uniform level, the gradient criterion over every
 // sub-neighbour (largest jump against the threshold: any neighbour's reaches it) and the interface
 // layers
+template <typename W>
 __global__ void __launch_bounds__(128) m5_tag_split(ffv_dmesh m, ffv_m5_tagc t, TagCells x,
-                                                    const uint32_t *__restrict__ SI,
+                                                    const W *__restrict__ SI,
                                                     int32_t *__restrict__ split) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.n) return;
@@ -1905,7 +1919,7 @@ __global__ void __launch_bounds__(128) m5_tag_split(ffv_dmesh m, ffv_m5_tagc t, 
   }
   if (t.inter0 != 0) {
     for (int v = 0; v < 2; ++v) {
-      const int si = (int)(v ? SI[c] >> 16 : SI[c] & 0xffff);
+      const int si = v ? si_high(SI[c]) : si_low(SI[c]);
       if (si >= 1 && si < t.lrs0) level = level > t.lvl0 ? level : t.lvl0;
       if (si >= t.lrs0 && si < t.lrs1) level = level > t.lvl1 ? level : t.lvl1;
     }
@@ -1984,9 +1998,10 @@ void ffv_m5_export_fields(int64_t n, const M5Consts &k, const double *S, double 
   else m5_export_fields<3><<<gc, 128, 0, st>>>(n, k, S, F);
 }
 
-void ffv_m5_tags(const ffv_dmesh &m, const M5Consts &k, const ffv_m5_tagc &t, bool symmetric,
-                 const double *S, uint32_t *SI, int32_t *lists, int32_t *split, double *pr,
-                 cudaStream_t st) {
+namespace {
+template <typename W>
+void tags_impl(const ffv_dmesh &m, const M5Consts &k, const ffv_m5_tagc &t, bool symmetric, const double *S,
+               W *SI, int32_t *lists, int32_t *split, double *pr, cudaStream_t st) {
   const unsigned gc = (unsigned)((m.n + 127) / 128);
   // pr: pressure, density [n] doubles each, then both as floats; the phi codes wait in split
   float *f = reinterpret_cast<float *>(pr + 2 * m.n);
@@ -2006,13 +2021,23 @@ void ffv_m5_tags(const ffv_dmesh &m, const M5Consts &k, const ffv_m5_tagc &t, bo
       else m5_si_layer<<<gc, 128, 0, st>>>(m, lvl, SI);
     }
   } else {
-    cudaMemsetAsync(SI, 0, sizeof(uint32_t) * m.n, st);
+    cudaMemsetAsync(SI, 0, sizeof(W) * m.n, st);
   }
   m5_tag_split<<<gc, 128, 0, st>>>(m, t, x, SI, split);
 }
+}  // namespace
 
-void ffv_m5_si_unpack(int64_t n, const uint32_t *SI, int32_t *out, cudaStream_t st) {
-  m5_si_unpack<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, SI, out);
+void ffv_m5_tags(const ffv_dmesh &m, const M5Consts &k, const ffv_m5_tagc &t, bool symmetric,
+                 const double *S, void *SI, bool wide, int32_t *lists, int32_t *split, double *pr,
+                 cudaStream_t st) {
+  if (wide) tags_impl(m, k, t, symmetric, S, static_cast<unsigned long long *>(SI), lists, split, pr, st);
+  else tags_impl(m, k, t, symmetric, S, static_cast<uint32_t *>(SI), lists, split, pr, st);
+}
+
+void ffv_m5_si_unpack(int64_t n, const void *SI, bool wide, int32_t *out, cudaStream_t st) {
+  const unsigned g = (unsigned)((n + 255) / 256);
+  if (wide) m5_si_unpack<<<g, 256, 0, st>>>(n, static_cast<const unsigned long long *>(SI), out);
+  else m5_si_unpack<<<g, 256, 0, st>>>(n, static_cast<const uint32_t *>(SI), out);
 }
 
 void ffv_m5_cfl(const ffv_dmesh &m, const ffv_geom &g, const M5Consts &k, const double *S,
