@@ -27,10 +27,10 @@ struct ffv_ctx {
   // model 5 only
   double *d_Snew, *d_FF, *d_UF, *d_RHS;
   uint8_t *d_GF, *d_flag;
-  // the mesh's listed faces (ffv_face_list): n pairs' room behind GF (0.2 to 0.4 n are usual), a
-  // buffer of its own where a mesh has more
-  int32_t *d_flist, *d_flist_own;
-  int64_t cap_flist_own;
+  // the mesh's listed faces (ffv_face_list) behind GF, room for all six of every cell (0.2 to 0.4 per
+  // cell are usual; 24 bytes beside the 3 KB that a cell takes keep a regrid free of allocations on
+  // any mesh that fits)
+  int32_t *d_flist;
   ffv_face_list flist;
   bool symmetric;        // every fine face's coarse neighbour has it among its four (no part mesh)
   int32_t *d_list;       // flagged cells: count, cells [n], and the face list's 12 cursors
@@ -78,9 +78,7 @@ void free_mesh_buffers(ffv_ctx *c) {
   cudaFree(c->d_RHS);
   cudaFree(c->d_flag);
   cudaFree(c->d_list);
-  cudaFree(c->d_flist_own);
-  c->d_flist = c->d_flist_own = nullptr;
-  c->cap_flist_own = 0;
+  c->d_flist = nullptr;
   cudaFree(c->d_SI);
   cudaFree(c->d_SItmp);
   cudaFree(c->d_split);
@@ -118,7 +116,7 @@ int alloc_mesh_buffers(ffv_ctx *c) {
     if (cudaMalloc(&c->d_Snew, sizeof(double) * c->neq * n) != cudaSuccess ||
         cudaMalloc(&c->d_FF, sizeof(double) * 6 * c->neq * n) != cudaSuccess ||
         cudaMalloc(&c->d_UF, sizeof(double) * 18 * n) != cudaSuccess ||
-        cudaMalloc(&c->d_GF, (((6 * n + 3) & ~(int64_t)3) + 4 * n)) != cudaSuccess ||
+        cudaMalloc(&c->d_GF, (((6 * n + 3) & ~(int64_t)3) + 24 * n)) != cudaSuccess ||
         cudaMalloc(&c->d_RHS, sizeof(double) * c->neq * n) != cudaSuccess ||
         cudaMalloc(&c->d_flag, 10 * n) != cudaSuccess ||  // flags, and the FP32-flux form's marks
         cudaMalloc(&c->d_list, sizeof(int32_t) * (n + 13)) != cudaSuccess) {
@@ -245,27 +243,14 @@ int build_face_list(ffv_ctx *c, const int64_t *count) {
     l.off[g + 1] = l.off[g] + (int32_t)count[g];
     l.block[g + 1] = l.block[g] + (int32_t)((threads + FFV_LIST_TPB - 1) / FFV_LIST_TPB);
   }
-  const int64_t total = l.off[12];
-  int32_t *cells = c->d_flist;
-  if (total > c->cap) {
-    if (total > c->cap_flist_own) {
-      cudaFree(c->d_flist_own);
-      c->d_flist_own = nullptr;
-      c->cap_flist_own = 0;
-      if (cudaMalloc(&c->d_flist_own, sizeof(int32_t) * (total + total / 4)) != cudaSuccess)
-        return FFV_ERR_NOMEM;
-      c->cap_flist_own = total + total / 4;
-    }
-    cells = c->d_flist_own;
-  }
-  l.cells = cells;
+  l.cells = c->d_flist;
   CK(cudaMemsetAsync(c->d_GF, 0, 6 * c->n, c->stream));
   CK(cudaMemsetAsync(c->d_list, 0, sizeof(int32_t), c->stream));  // no flagged cells
   CK(whole_base(c));
-  if (total == 0) return FFV_OK;
+  if (l.off[12] == 0) return FFV_OK;
   int32_t *cursor = c->d_list + 1 + c->cap;
   CK(cudaMemcpyAsync(cursor, l.off, sizeof(int32_t) * 12, cudaMemcpyHostToDevice, c->stream));
-  list_faces<<<(unsigned)((c->n + 255) / 256), 256, 0, c->stream>>>(c->n, c->d_info, cursor, cells);
+  list_faces<<<(unsigned)((c->n + 255) / 256), 256, 0, c->stream>>>(c->n, c->d_info, cursor, c->d_flist);
   return cuda_rc(cudaGetLastError());
 }
 
