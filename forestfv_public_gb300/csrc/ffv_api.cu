@@ -33,7 +33,9 @@ struct ffv_ctx {
   int32_t *d_flist;
   ffv_face_list flist;
   bool symmetric;        // every fine face's coarse neighbour has it among its four (no part mesh)
-  int32_t *d_list;       // flagged cells: count, cells [n], and the face list's 12 cursors
+  // flagged cells: count, cells [cap], then FFV_GFM_PARTS + 1 words (list_parts; while a mesh is set,
+  // the face list's 12 cursors)
+  int32_t *d_list;
   M5Consts m5;
   // refinement tags
   void *d_SI;    // interface layers, a word of 32 or (si_wide) 64 bits per cell
@@ -119,7 +121,7 @@ int alloc_mesh_buffers(ffv_ctx *c) {
         cudaMalloc(&c->d_GF, (((6 * n + 3) & ~(int64_t)3) + 24 * n)) != cudaSuccess ||
         cudaMalloc(&c->d_RHS, sizeof(double) * c->neq * n) != cudaSuccess ||
         cudaMalloc(&c->d_flag, 10 * n) != cudaSuccess ||  // flags, and the FP32-flux form's marks
-        cudaMalloc(&c->d_list, sizeof(int32_t) * (n + 13)) != cudaSuccess) {
+        cudaMalloc(&c->d_list, sizeof(int32_t) * (n + 2 + FFV_GFM_PARTS)) != cudaSuccess) {
       free_mesh_buffers(c);
       return FFV_ERR_NOMEM;
     }
@@ -162,7 +164,7 @@ int launch_stage(ffv_ctx *c, int irk, bool follows, cudaEvent_t *ev = nullptr) {
   if (c->p.model == 5) {
     ffv_m5_bufs mb{c->d_S,   c->d_SN,   c->d_Snew, c->d_SF,     c->d_FF,    c->d_UF,
                    c->d_RHS, c->d_dt,   c->d_GF,   c->d_flag,   flat_marks(c), c->d_list,
-                   c->d_status, c->flist};
+                   c->d_list + 1 + c->cap, c->d_status, c->flist};
     ffv_m5_fp64_stage(c->dm, c->geom, c->m5, mb, irk, follows, c->stream, ev, c->knames);
     return cuda_rc(cudaGetLastError());
   }
@@ -247,11 +249,15 @@ int build_face_list(ffv_ctx *c, const int64_t *count) {
   CK(cudaMemsetAsync(c->d_GF, 0, 6 * c->n, c->stream));
   CK(cudaMemsetAsync(c->d_list, 0, sizeof(int32_t), c->stream));  // no flagged cells
   CK(whole_base(c));
-  if (l.off[12] == 0) return FFV_OK;
+  static_assert(FFV_GFM_PARTS + 1 >= 12, "the cursors' room");
   int32_t *cursor = c->d_list + 1 + c->cap;
-  CK(cudaMemcpyAsync(cursor, l.off, sizeof(int32_t) * 12, cudaMemcpyHostToDevice, c->stream));
-  list_faces<<<(unsigned)((c->n + 255) / 256), 256, 0, c->stream>>>(c->n, c->d_info, cursor, c->d_flist);
-  return cuda_rc(cudaGetLastError());
+  if (l.off[12] > 0) {
+    CK(cudaMemcpyAsync(cursor, l.off, sizeof(int32_t) * 12, cudaMemcpyHostToDevice, c->stream));
+    list_faces<<<(unsigned)((c->n + 255) / 256), 256, 0, c->stream>>>(c->n, c->d_info, cursor, c->d_flist);
+    CK(cudaGetLastError());
+  }
+  CK(cudaMemsetAsync(cursor, 0, sizeof(int32_t) * (FFV_GFM_PARTS + 1), c->stream));
+  return FFV_OK;
 }
 
 // CFL: dt = cfl * min over cells of h / max_a(|u_a| + c)  (no reference counterpart:

@@ -56,12 +56,16 @@ struct FlatMarks {
   uint8_t *face;  // [6][n]: face states
 };
 
+// blocks of a ghost-fluid pass, where many cells are flagged (m5_gfm_seq)
+#define FFV_GFM_PARTS 16
+
 struct ffv_m5_bufs {
   double *S, *SN, *Snew, *SF, *FF, *UF, *RHS, *dt;
   uint8_t *GF, *flag;  // GF [6][n]: marks of faces, as the cell that evaluates the face sees them
   FlatMarks flat;
-
-  int32_t *list;  // [1 + n]: the number of cells the last pass flagged, then the cells
+  // [1 + n]: the number of cells the last pass flagged, then the cells; list_parts [FFV_GFM_PARTS + 1]:
+  // the number of them in each block's run of cells, and the blocks that have finished (0 between passes)
+  int32_t *list, *list_parts;
   unsigned int *status;
   ffv_face_list list_faces;
 };
