@@ -1740,7 +1740,7 @@ __global__ void __launch_bounds__(128) m5_tag_cells(int64_t n, M5Consts k, bool 
   uint32_t code;
   if (N > 2) {
     const double a1 = clamp_vf(k, S[(int64_t)(C::i3 + 1) * n + c]);
-    code = phi_code(k.nsolids == 2 && k.mu[0] != 0.0 && a0 <= a1 ? a1 : a0, k.avf_lim) |
+    code = phi_code(k.nsolids == 2 && k.mu[0] != 0.0 && !f64::gt(a0, a1) ? a1 : a0, k.avf_lim) |
            phi_code(a1, k.avf_lim) << 2;
   } else {
     code = phi_code(a0, k.avf_lim) | 1u << 2;
