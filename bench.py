@@ -166,7 +166,7 @@ def _config2(name: str):
     lmin, lmax, band = BUBBLE_SIZES[name]
     mesh, S0, p = W.bubble_config2(lmin=lmin, lmax=lmax, band_cells=band)
     cfg = workload_config(name, int(mesh.n), sorted(int(x) for x in np.unique(mesh.level)))
-    alg = m5_alg_bytes(S0.shape[0], 2)
+    alg = m5_alg_bytes(S0)
     return mesh, S0, cfg["dt"], cfg, _bubble_solver_kwargs(p), alg, False
 
 
@@ -199,7 +199,7 @@ def _config3(name: str):
     cfg = workload_config(name, int(mesh.n), sorted(int(x) for x in np.unique(mesh.level)))
     cfg["amr"] = {"tags": list(wall_tags(lmax)), "every": AMR_EVERY, "horizon": AMR_HORIZON,
                   "threshold": AMR_THRESHOLD, "infer_every": AMR_INFER_EVERY}
-    return mesh, S0, cfg["dt"], cfg, _wall_solver_kwargs(p), m5_alg_bytes(21, 3), False
+    return mesh, S0, cfg["dt"], cfg, _wall_solver_kwargs(p), m5_alg_bytes(S0), False
 
 
 def wl_config3(small: bool = False, medium: bool = False):
@@ -226,21 +226,27 @@ def wall_tags(lmax: int) -> tuple:
     return (1, 4, 0, 0, 0.0, 1, lmax, 0.1, 0, 0, 0.0, 1, lmax, WALL_LRS, 0, 0, 0)
 
 
-def m5_alg_bytes(neq: int, nmat: int) -> dict:
-    """Algorithmic bytes per cell of each model-5 kernel (compulsory traffic, neighbour
-    re-reads excluded).  FP32 form: the FP32 shadow state (4 neq), the 2 N critical slots in
-    FP64, face records of neq + 2 FP32 values."""
-    d = 8 * neq
-    rec = 4 * (neq + 2)
+def m5_alg_bytes(S0) -> dict:
+    """Algorithmic bytes per cell of each model-5 kernel (compulsory traffic, neighbour re-reads
+    excluded, a face between two cells counted once) in a state like S0 [neq, n].  FP32 form: the FP32
+    copy of the state and the low parts of 2 N critical slots, face records of neq + 2 FP32 values, one
+    byte per mark; the deformation (nine variables) only for the share of cells that have one."""
+    neq = S0.shape[0]
+    nmat = (neq - 12) // 3
+    share = float(np.mean((S0[-9:] != 0.0).any(axis=0)))
+    d, face64 = 8 * neq, 8 * (neq + 3)
+    own = neq - 9 + 9 * share
+    state, rec, face = 8 * own, 4 * (own + 2), 4 * (own + 3)
     return {"m5_recon_slopes": d + 28 + 6 * d,
             "m5_relax_faces": 6 * d + 6 * 8 * (2 * nmat + 8),
-            "m5_face_flux": 6 * d + d + 28 + 6 * d + 6 * 3 * 8 + 6,
-            "m5_cell_update": d + 6 * d + 6 * 3 * 8 + d + 28 + d + d + 1,
+            "m5_face_flux": 6 * d + 28 + 3 * face64 + 6,
+            "m5_cell_update": d + 3 * face64 + d + 28 + d + d + 1,
             "m5_relax_cell": d + d + 1,
-            "m5f_recon_face": 4 * neq + 8 * 2 * nmat + 28 + 6 * rec,
-            "m5f_face_flux": 6 * rec + 8 * 2 * nmat + 28 + 6 * 4 * neq + 6 * 3 * 4 + 6,
-            "m5f_cell_update": d + 6 * 4 * neq + 6 * 3 * 4 + d + 28 + d + d + 1,
-            "m5f_relax_cell": d + d + 1}
+            "m5f_shadow": state + 4 * own + 8 * nmat + 1,
+            "m5f_recon_face": 4 * own + 8 * nmat + 28 + 1 + 6 * (rec + 1) + 1,
+            "m5f_face_flux": 6 * (rec + 1) + 28 + 3 * face + 6,
+            "m5f_cell_update": state + 3 * face + 6 + state + 28 + 8 * (nmat + 3) + state + 3,
+            "m5f_relax_cell": 2 * state + 2}
 
 
 def _config5(name: str):
@@ -254,7 +260,7 @@ def _config5(name: str):
     cfg["amr"] = {"tags": [1, lbase, 0, 0, 0.0, 1, lmax, 0.1, 0, 0, 0.0, 1, lmax, 4, 0, 0, 0],
                   "every": AMR_EVERY, "horizon": AMR_HORIZON, "threshold": AMR_THRESHOLD,
                   "infer_every": AMR_INFER_EVERY}
-    return mesh, S0, cfg["dt"], cfg, _wall_solver_kwargs(p), m5_alg_bytes(21, 3), False
+    return mesh, S0, cfg["dt"], cfg, _wall_solver_kwargs(p), m5_alg_bytes(S0), False
 
 
 def wl_config5(small: bool = False, medium: bool = False):
@@ -942,8 +948,8 @@ def measure_amr(mesh, S0, dt, kw, args, dev, amr_cfg, alg_bytes, roofline_of, ke
     err = error_report_meshes(sl.mesh, sl.download_state(), sp.mesh, sp.download_state(),
                               kw["gamma"], kw["pinf"], mu, kw["amin"], solid)
     roof32 = roofline_of(kernel_times(sl, 3), sl.mesh.n,
-                         "FP32-flux form; its face kernel mixes FP32 arithmetic with the FP64 "
-                         "pressure recovery of the critical slots")
+                         "FP32-flux form; its reconstruction is bound by instruction issue "
+                         "(bytes: the deformation for the share of cells that have one)")
     # the learned form end to end: state uploaded from and downloaded to pinned host memory
     # around every step of the same loop
     se = fresh(1)

@@ -1720,7 +1720,7 @@ __device__ __forceinline__ void update_cell(
   if (st) atomicOr(status, st);
 }
 
-// Bound by latency at 12 warps per SM (issue slots 40 %, DRAM 3.8 TB/s): three blocks of 128 threads
+// Bound by latency at 12 warps per SM (issue slots 30-37 %, 2.5-3.0 TB/s): three blocks of 128 threads
 // (at most 170 registers); at four both paths spill or wait longer.  First and later stages:
 //   bubble mesh, 2.3 M cells, all calm    301 / 322 us   (one path 442 / 510, four blocks 249 / 268)
 //   wall mesh, 10.1 M, 41 % of warps calm  2.37 / 2.86 ms (one path 2.38 / 2.79, four blocks 2.61 / 3.01)

@@ -184,7 +184,8 @@ int ffv_step_async(ffv_ctx *ctx, double dt, int32_t nsteps);
 /* Wait for queued work and return the first error the device recorded. */
 int ffv_sync(ffv_ctx *ctx);
 /* Largest stable dt for the given CFL number: cfl * min over cells of
- * h / max(|u_a| + c) (new: the reference uses a fixed DT, inputset.c:69). */
+ * h / max(|u_a| + c) (new: the reference uses a fixed DT, inputset.c:69).  Model 5: FFV_ERR_NAN
+ * where any cell has no such speed. */
 int ffv_cfl_dt(ffv_ctx *ctx, double cfl, double *dt_out);
 /* Device pointer of the conserved state (SoA), valid until the next ffv_set_mesh. */
 int ffv_state_device_ptr(ffv_ctx *ctx, double **d_S);
